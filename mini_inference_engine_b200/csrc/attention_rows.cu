@@ -35,8 +35,8 @@ __global__ void __launch_bounds__(kRowWarps * 32) attention_rows_kernel(RowsPara
   extern __shared__ float rows_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* qs = rows_smem + (size_t)warp * p.dim;
-  chain_wait();
   chain_release();
+  chain_wait();
   const long long item = (long long)blockIdx.x * kRowWarps + warp;
   if (item >= (long long)p.tokens * p.q_heads) return;
   const long long t = item / p.q_heads;

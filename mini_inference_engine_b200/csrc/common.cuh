@@ -50,11 +50,15 @@ bool chained_launch_enabled();  // false when MIE_PDL=0
 void prefer_shared_carveout(const void* kernel);
 
 #ifdef __CUDACC__
-// Programmatic dependent launch.  A kernel launched with launch_chained() may be scheduled while the kernel
-// before it on the stream is still running; it must call chain_wait() before its first access to global
-// memory (the wait returns once the previous kernel has finished and its writes are visible) and then
-// chain_release(), which lets the kernel AFTER it be scheduled early in the same way.  Both are no-ops for
-// a kernel launched the ordinary way.
+// Programmatic dependent launch.  A kernel launched with launch_chained() may be scheduled while the kernels before
+// it on the stream are still running.  It calls chain_release() once its shared memory, barriers and tensor memory are
+// set up, which lets the kernel AFTER it be scheduled in the same way, and chain_wait() before its first access to
+// global memory that another kernel of the stream writes: the wait returns once the previous kernel has finished (and
+// so, as that one waited too, all before it) and its writes are visible.  Releasing before waiting lets a GEMM two
+// launches ahead set up and request its weights while the GEMM before it is still running; a kernel is only scheduled
+// when every block of the one before it has released, so a waiting block never keeps an earlier one off the GPU.
+// Releasing after the wait is left to kernels whose successor relies on their wait (the first launch of a two-launch
+// GEMM).  Both are no-ops for a kernel launched the ordinary way.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -99,8 +99,8 @@ __global__ void __launch_bounds__(kWarps8 * 32, 1)
     tma_prefetch_desc(&kvmap);
   }
   __syncthreads();
-  chain_wait();
   chain_release();
+  chain_wait();
 
   const int g = lane >> 2, t = lane & 3;
   const int chunk = p.sc.header[0];
@@ -384,8 +384,8 @@ __global__ void __launch_bounds__(kWarps8 * 32, 1)
 template <typename T, int kMergeWarpsPerHead>
 __global__ void __launch_bounds__(kMaxGroupMerge * kMergeWarpsPerHead * 32) merge_kernel(DecodeParams p) {
   __shared__ float part[kMaxGroupMerge][kMergeWarpsPerHead][2 + kHeadDim];
-  chain_wait();
   chain_release();
+  chain_wait();
   const int b = blockIdx.x / p.kv_heads, h = blockIdx.x % p.kv_heads;
   const int first = p.sc.offsets[b], n = p.sc.offsets[b + 1] - first;
   if (n <= 1) return;

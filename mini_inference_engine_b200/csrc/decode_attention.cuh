@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(IndexView lengths, I
   __shared__ int running_s;
   __shared__ long long chunk_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  chain_wait();
   chain_release();
+  chain_wait();
 
   // With one thread per request (the usual launch) a request's length is read once and kept.
   const bool one_each = batch <= (int)blockDim.x;
@@ -301,8 +301,8 @@ __global__ void __launch_bounds__(DecodeTile<KH, VH>::kWarps * 32, 1)
     tma_prefetch_desc(&vmap);
   }
   __syncthreads();
-  chain_wait();
   chain_release();
+  chain_wait();
 
   const int g = lane >> 2, t = lane & 3;
   const int chunk = p.sc.header[0];
@@ -576,8 +576,8 @@ constexpr int kMergeWarps = 4;
 template <typename T, int VH>
 __global__ void __launch_bounds__(kMergeWarps * 32) merge_rows_kernel(DecodeParams p) {
   __shared__ float part[kMergeWarps][2 + VH * 64];
-  chain_wait();
   chain_release();
+  chain_wait();
   const int b = blockIdx.x / p.q_heads, head = blockIdx.x % p.q_heads;
   const int first = p.sc.offsets[b], n = p.sc.offsets[b + 1] - first;
   if (n <= 1) return;

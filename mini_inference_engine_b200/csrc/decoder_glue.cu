@@ -33,8 +33,8 @@ struct EmbedParams {
 
 template <typename T, int VEC>
 __global__ void embed_kernel(EmbedParams p) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const int t = blockIdx.x;
   const bool first_thread = threadIdx.x == 0;
   long long id = p.ids.at(t);
@@ -127,8 +127,8 @@ struct SumNormParams {
 template <typename T, int VEC>
 __global__ void __launch_bounds__(1024) sum_norm_kernel(SumNormParams p) {
   __shared__ float red[32];
-  chain_wait();
   chain_release();
+  chain_wait();
   const int row = blockIdx.x, tid = threadIdx.x;
   const float* x = p.x + (long long)row * p.ldx;
   const T* y = p.y == nullptr ? nullptr : reinterpret_cast<const T*>(p.y) + (long long)row * p.ldy;
@@ -203,8 +203,8 @@ struct QkvMixParams {
 
 template <typename T, int VEC, int LANES>
 __global__ void qkv_mix_kernel(QkvMixParams p) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;
   const int lane = threadIdx.x % LANES;
   const int slots = p.q_heads + 2 * p.kv_heads;
@@ -273,8 +273,8 @@ __global__ void qkv_mix_kernel(QkvMixParams p) {
 template <typename T, int VEC>
 __global__ void clamped_glu_kernel(const T* gate, const T* up, long long ld_in, T* out, long long ldo, int rows,
                                    int cols, float limit, float slope, float up_offset) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const int per_row = cols / VEC;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)rows * per_row) return;

@@ -59,7 +59,9 @@ struct GemmParams {
   // Wide kernel only: this launch covers output tiles [tile_begin, tile_end).  late_wait: the launch-chain
   // wait is taken at the end of the kernel instead of the start (second launch of a two-launch GEMM, whose
   // inputs are already known to be complete because the first launch waited for them).
-  int tile_begin, tile_end, late_wait;
+  // early_release: the next launch may start before this one's wait (not when it is the second launch of a
+  // two-launch GEMM, which takes the first one's wait for its own).
+  int tile_begin, tile_end, late_wait, early_release;
 };
 
 // Scale staging: per chunk of kChunkKb K blocks the promotion warps pull every
@@ -147,7 +149,12 @@ __global__ void __launch_bounds__((kNarrowEpiWarps + 2) * 32, (BN <= 32 ? 2 : 1)
   const int kb_first = (int)((long long)kb_total * rank / split);
   const int kb_last = (int)((long long)kb_total * (rank + 1) / split);  // exclusive
 
-  if (threadIdx.x == 0) {
+  // Everything up to the launch-chain wait overlaps the kernels queued before this one.  So does the weight half of
+  // the first stages (the caller promises that those kernels do not write the weights): the producer requests it
+  // before the TMEM allocation, which may have to wait for an earlier kernel's, and adds the activation half after
+  // the wait.
+  uint32_t prefetched = 0;
+  if (warp == E && lane == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
@@ -159,6 +166,14 @@ __global__ void __launch_bounds__((kNarrowEpiWarps + 2) * 32, (BN <= 32 ? 2 : 1)
     mbar_fence_init();
     tma_prefetch_desc(&map_w);
     tma_prefetch_desc(&map_x);
+    if (p.prefetch) {
+      const uint64_t stream_policy = l2_evict_first_policy();
+      for (int kb = kb_first; kb < kb_last && prefetched < (uint32_t)kStages; ++kb, ++prefetched) {
+        mbar_expect_tx(&full_bar[prefetched], S::kStageBytes);
+        tma_load_2d_hint(stage_base + (size_t)prefetched * S::kStageBytes, &map_w, &full_bar[prefetched], kb * kBlockK,
+                         tw * kTileR, stream_policy);
+      }
+    }
   }
   if (warp == E + 1) {
     tmem_alloc(tmem_slot, kTmemCols);
@@ -168,21 +183,8 @@ __global__ void __launch_bounds__((kNarrowEpiWarps + 2) * 32, (BN <= 32 ? 2 : 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // Barriers, tensor-map prefetch and the TMEM allocation above overlap the tail of the previous kernel.
-  // So can the weights (the caller promises that the kernel queued before this one does not write them):
-  // the producer requests the weight half of its first stages before the launch-chain wait and adds the
-  // activation half afterwards.
-  uint32_t prefetched = 0;
-  if (p.prefetch && warp == E && lane == 0) {
-    const uint64_t stream_policy = l2_evict_first_policy();
-    for (int kb = kb_first; kb < kb_last && prefetched < (uint32_t)kStages; ++kb, ++prefetched) {
-      mbar_expect_tx(&full_bar[prefetched], S::kStageBytes);
-      tma_load_2d_hint(stage_base + (size_t)prefetched * S::kStageBytes, &map_w, &full_bar[prefetched], kb * kBlockK,
-                       tw * kTileR, stream_policy);
-    }
-  }
-  chain_wait();
   chain_release();
+  chain_wait();
 
   // Promotion state that outlives the role branch (the reduction below needs it).
   constexpr int kEpiThreads = E * 32;
@@ -562,8 +564,9 @@ __global__ void __launch_bounds__(kWideThreads, 1)
       }
     }
   }
+  if (p.early_release) chain_release();
   if (!p.late_wait) chain_wait();
-  chain_release();
+  if (!p.early_release) chain_release();
 
   // K blocks this CTA will process (the promotion pipeline needs to know when the last one is reached).
   uint32_t total_blocks = 0;
@@ -990,10 +993,11 @@ WidePlan plan_wide(long long tiles, int kb, int max_split) {
 }
 
 int launch_wide_range(const CUtensorMap& mx, const CUtensorMap& mw, GemmParams p, int tile_begin, int tile_end,
-                      int split, bool late_wait, cudaStream_t stream) {
+                      int split, bool late_wait, bool tail_follows, cudaStream_t stream) {
   p.tile_begin = tile_begin;
   p.tile_end = tile_end;
   p.late_wait = late_wait ? 1 : 0;
+  p.early_release = tail_follows ? 0 : 1;
   const int count = tile_end - tile_begin;
   const int ctas = split > 1 ? count : (count < sm_count() ? count : sm_count());
   cudaLaunchConfig_t config = {};
@@ -1029,12 +1033,12 @@ int launch_wide(const CUtensorMap& mx, const CUtensorMap& mw, const GemmParams& 
   const long long tiles = (long long)((p.m + kTileR - 1) / kTileR) * ((p.n + kWideBN - 1) / kWideBN);
   MIE_CHECK_ARG(tiles <= 0x7fffffff, "too many output tiles (%lld)", tiles);
   const WidePlan plan = plan_wide(tiles, kb, max_split);
-  if (int rc = launch_wide_range(mx, mw, p, 0, plan.main_tiles, plan.main_split, false, stream)) return rc;
+  if (int rc = launch_wide_range(mx, mw, p, 0, plan.main_tiles, plan.main_split, false, plan.tail_split > 0, stream)) return rc;
   if (plan.tail_split > 0) {
     // Only with launch chaining on does the tail start before the main launch has drained; without it the
     // stream simply runs the two launches one after the other.
     return launch_wide_range(mx, mw, p, plan.main_tiles, (int)tiles, plan.tail_split, chained_launch_enabled(),
-                             stream);
+                             false, stream);
   }
   return MIE_OK;
 }
@@ -1105,7 +1109,7 @@ extern "C" int mie_fp8_gemm(const void* x8, int64_t ldx, const float* a_scale, i
     return v != nullptr && v[0] == '0' ? 0 : 1;  // MIE_GEMM_PREFETCH=0 turns it off
   }();
   p.prefetch = prefetch && !(flags & MIE_GEMM_NO_WEIGHT_PREFETCH);
-  p.tile_begin = p.tile_end = p.late_wait = 0;
+  p.tile_begin = p.tile_end = p.late_wait = p.early_release = 0;
 
   CUtensorMap mw, mx;
   if (narrow) {

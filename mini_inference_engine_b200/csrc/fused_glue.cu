@@ -31,8 +31,8 @@ struct RowNormParams {
 
 __global__ void __launch_bounds__(1024) row_norm_kernel(RowNormParams p) {
   __shared__ float red[32];
-  chain_wait();
   chain_release();
+  chain_wait();
   const int row = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int c0 = tid * 8;
@@ -104,8 +104,8 @@ __global__ void head_norm_kernel(const __nv_bfloat16* x, long long outer_stride,
 __global__ void silu_mul_kernel(const __nv_bfloat16* gate, const __nv_bfloat16* up, long long ld_in,
                                 __nv_bfloat16* out, uint8_t* q, long long ldq, float* scales, int scale_ld,
                                 int rows, int cols) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const int per_row = cols / 8;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = idx < (long long)rows * per_row;
@@ -184,8 +184,8 @@ struct QkvParams {
 };
 
 __global__ void qkv_post_kernel(QkvParams p) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int heads_total = p.q_heads + 2 * p.kv_heads;

@@ -138,8 +138,8 @@ __global__ void __launch_bounds__(kLatentThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_o = *tmem_slot;
-  chain_wait();
   chain_release();
+  chain_wait();
 
   const int chunk = p.sc.header[0], total_items = p.sc.header[2];
   const long long capacity = (long long)p.table_width * p.block_size;

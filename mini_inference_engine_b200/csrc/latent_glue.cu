@@ -66,8 +66,8 @@ struct LatentWriteParams {
 
 template <typename T, int VEC>
 __global__ void latent_write_kernel(LatentWriteParams p) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const int lane = threadIdx.x & 31, parts = p.pages == nullptr ? 1 : 2;
   const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (item >= (long long)p.tokens * parts) return;
@@ -93,8 +93,8 @@ template <typename T>
 __global__ void rotate_heads_kernel(const T* src, long long s_token, long long s_head, T* dst, long long d_token,
                                     long long d_head, IndexView positions, const float2* turns, int tokens, int heads,
                                     int rot_dim, int rotated, int lanes) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / lanes;
   const int lane = threadIdx.x % lanes;
   if (t >= tokens) return;
@@ -126,8 +126,8 @@ __global__ void rotate_heads_kernel(const T* src, long long s_token, long long s
 __global__ void latent_spans_kernel(IndexView cu_seqlens, IndexView kv_lens, int requests, long long window,
                                     int table_width, long long row_capacity, long long token_capacity, int* spans,
                                     int* lens_out, int* table_out, int* status) {
-  chain_wait();
   chain_release();
+  chain_wait();
   __shared__ int base_s;
   if (threadIdx.x == 0) base_s = 0;
   __syncthreads();
@@ -174,8 +174,8 @@ struct GatherParams {
 
 template <typename Unit>
 __global__ void latent_gather_kernel(GatherParams p) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const int lane = threadIdx.x & 31;
   const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (row >= p.rows || row >= p.spans[2 * p.requests]) return;

@@ -101,8 +101,8 @@ constexpr int kOuterWarps = 8;
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kOuterWarps * 32) outer_decode_kernel(OuterParams p) {
   extern __shared__ float outer_smem[];
-  chain_wait();
   chain_release();
+  chain_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x / p.heads, h = blockIdx.x % p.heads;
   const int col = (blockIdx.y * 32 + lane) * VEC;
@@ -164,8 +164,8 @@ __global__ void __launch_bounds__(kOuterWarps * 32) outer_decode_kernel(OuterPar
 template <typename T>
 __global__ void __launch_bounds__(kOuterWarps * 32) outer_rows_kernel(OuterParams p) {
   extern __shared__ float outer_smem[];
-  chain_wait();
   chain_release();
+  chain_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r = blockIdx.x / p.heads, h = blockIdx.x % p.heads, col = blockIdx.y * 32 + lane;
   const long long begin = p.seg.cu_seqlens.at(r), end = p.seg.cu_seqlens.at(r + 1);
@@ -258,8 +258,8 @@ __global__ void __launch_bounds__(256 * VD, KD + VD == 2 ? 2 : 1) outer_chunk_ke
   const uint32_t base = smem_u32(chunk_smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
   const int h = blockIdx.y, col0 = blockIdx.z * VD * 64;
-  chain_wait();
   chain_release();
+  chain_wait();
   Segment seg;
   if (!p.seg.find(blockIdx.x, &seg)) return;
   if (!kEmit && seg.last) return;  // nobody needs what the last segment adds
@@ -538,8 +538,8 @@ constexpr int kCarryBatch = 8;  // segments whose loads are in flight together
 
 // carry[segment] <- state before the segment, from what the segments before it added.
 __global__ void outer_carry_kernel(OuterParams p) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const int r = blockIdx.x / p.heads, h = blockIdx.x % p.heads;
   const int e = blockIdx.y * blockDim.x + threadIdx.x, size = p.dim * p.vdim;
   if (e >= size) return;
@@ -655,8 +655,8 @@ __device__ __forceinline__ void average_emit(const float (&g)[VEC], T* out, cons
 
 template <typename T, int VEC>
 __global__ void average_decode_kernel(AverageParams p) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC, row = blockIdx.x;
   if (c >= p.width) return;
   float* slot = p.slots.at(row);
@@ -683,8 +683,8 @@ __global__ void average_decode_kernel(AverageParams p) {
 // What a segment does to a state before it: S -> product S + sum.
 template <typename T, int VEC>
 __global__ void __launch_bounds__(128, 8) average_summary_kernel(AverageParams p) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
   Segment seg;
   if (c >= p.width || !p.seg.find(blockIdx.x, &seg) || seg.last) return;
@@ -734,8 +734,8 @@ __global__ void __launch_bounds__(128, 8) average_summary_kernel(AverageParams p
 
 // carry[segment][0] <- state before the segment.
 __global__ void average_carry_kernel(AverageParams p) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const int r = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= p.width) return;
   int first = 0;
@@ -769,8 +769,8 @@ __global__ void average_carry_kernel(AverageParams p) {
 
 template <typename T, int VEC>
 __global__ void __launch_bounds__(128, 8) average_segment_kernel(AverageParams p) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
   Segment seg;
   if (c >= p.width || !p.seg.find(blockIdx.x, &seg)) return;

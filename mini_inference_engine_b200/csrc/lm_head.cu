@@ -95,8 +95,8 @@ __global__ void __launch_bounds__(kLmThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  chain_wait();
   chain_release();
+  chain_wait();
 
   if (warp == 4) {
     // ---------------- TMA producer ----------------
@@ -221,8 +221,8 @@ __global__ void __launch_bounds__(kLmThreads, 1)
 // embedding gather, for one) stays inside its table.
 __global__ void lm_head_finish_kernel(unsigned long long* keys, long long* tokens, int* values, int batch,
                                       long long vocab_offset, long long vocab, int* status) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= batch) return;
   const unsigned long long key = keys[b];

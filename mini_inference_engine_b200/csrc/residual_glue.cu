@@ -32,8 +32,8 @@ constexpr int kKept = 2;
 template <typename T, int VEC>
 __global__ void __launch_bounds__(512) residual_norm_kernel(ResidualParams p) {
   __shared__ float red[2][32];
-  chain_wait();
   chain_release();
+  chain_wait();
   const int tid = threadIdx.x, step = blockDim.x * VEC;
   float* x = p.x + (long long)blockIdx.x * p.ldx;
   const T* y = reinterpret_cast<const T*>(p.y) + (long long)blockIdx.x * p.ldy;
@@ -133,8 +133,8 @@ __device__ __forceinline__ float gelu_tanh(float z) {
 
 template <typename T, int VEC>
 __global__ void gelu_kernel(GeluParams p) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const int per_row = p.cols / VEC;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)p.rows * per_row) return;
@@ -176,8 +176,8 @@ struct GatedNormParams {
 template <typename T, int VEC>
 __global__ void __launch_bounds__(512) gated_norm_kernel(GatedNormParams p) {
   __shared__ float red[32];
-  chain_wait();
   chain_release();
+  chain_wait();
   const int tid = threadIdx.x, step = blockDim.x * VEC;
   const T* x = reinterpret_cast<const T*>(p.x) + (long long)blockIdx.x * p.ldx;
   const T* gate = reinterpret_cast<const T*>(p.gate) + (long long)blockIdx.x * p.ldg;
@@ -227,8 +227,8 @@ __global__ void __launch_bounds__(512) gated_norm_kernel(GatedNormParams p) {
 
 // logits <- cap * tanh(logits / cap), in place.
 __global__ void softcap_kernel(float* logits, long long count, float cap) {
-  chain_wait();
   chain_release();
+  chain_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) logits[i] = cap * tanhf(logits[i] / cap);
 }
