@@ -417,6 +417,17 @@ int mie_lm_head_argmax(const void* x, int64_t ldx, const void* w, int64_t ldw, i
                        int32_t k, int64_t vocab_offset, uint64_t* keys, int64_t* tokens, int32_t* values,
                        int32_t* status, void* stream);
 
+/*
+ * Projection of up to MIE_LINEAR_MAX_ROWS bf16 rows: y[m, n] = x[m, k] w[n, k]^T (+ bias[n]), fp32 sums rounded once
+ * to bf16 (the decode-sized products of the bf16 designs; larger ones are library products).  k must be a multiple of
+ * 8, operand rows 16-byte aligned; strides in elements.  Part of the launch chain: the weights may be requested before
+ * the kernels queued earlier on the stream have finished, so those must not be kernels of this library that write
+ * them.  kernel: 0 picks by the number of rows, 1 the register kernel (at most 32 rows), 2 the tensor-memory kernel.
+ */
+#define MIE_LINEAR_MAX_ROWS 128
+int mie_linear(const void* x, int64_t ldx, const void* w, int64_t ldw, const void* bias, void* y, int64_t ldy,
+               int32_t m, int32_t n, int32_t k, int32_t kernel, int32_t* status, void* stream);
+
 /* ---------------------------------------------------------------------------
  * Tensor-parallel exchange (no counterpart in the reference, which runs on one
  * GPU; these serve the head-sharded TP = 2/4/8 decode step).

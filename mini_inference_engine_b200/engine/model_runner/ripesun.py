@@ -41,6 +41,7 @@ from ..kernels.decoder_glue import (
     softcap_,
     sum_rms_norm,
 )
+from ..kernels.linear import linear
 from ..kernels.recurrence import StateBuffer, gated_average, outer_recurrence
 from ..kv_cache.latent_attention import (
     VisibleSpans,
@@ -350,9 +351,8 @@ class RipesunRunner(PagedStepRunner):
 
     # -- projections ----------------------------------------------------------------------------
 
-    @staticmethod
-    def _linear(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-        return torch.nn.functional.linear(x, weight)
+    def _linear(self, x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+        return linear(x, weight, status=self.status)
 
     def _finish(self, x32: torch.Tensor, return_logits: bool):
         """Final norm, then greedy tokens (and the logits when asked for) of residual rows.  The soft cap is monotonic:

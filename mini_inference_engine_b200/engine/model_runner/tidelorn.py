@@ -24,6 +24,7 @@ from dataclasses import dataclass
 
 import torch
 
+from ..kernels.linear import linear
 from ..kernels.decoder_glue import clamped_glu, embed_tokens, qkv_norm_mix_write, sinusoid_turns, sum_rms_norm
 from ..kv_cache.sink_attention import (
     attention_rows,
@@ -267,9 +268,8 @@ class TidelornRunner(PagedStepRunner):
 
     # -- projections ----------------------------------------------------------------------------
 
-    @staticmethod
-    def _linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
-        return torch.nn.functional.linear(x, weight, bias)
+    def _linear(self, x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
+        return linear(x, weight, bias, status=self.status)
 
     def _logits(self, final: torch.Tensor) -> torch.Tensor:
         """fp32 logits of normed rows."""

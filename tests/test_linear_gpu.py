@@ -1,0 +1,56 @@
+"""bf16 projections of decode-sized batches against the product in 64 bits."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from mini_inference_engine_b200.engine.kernels.linear import linear, linear_supported
+
+pytestmark = pytest.mark.gpu
+
+# Weight rows and columns around the tiles of both kernels (16 and 128 rows, units of 64 columns, K cut in up to 8).
+SHAPES = [(1, 8), (16, 64), (17, 72), (127, 520), (129, 256), (2048, 2048), (8200, 512), (2112, 4096), (300, 6152)]
+
+
+@pytest.mark.parametrize("n,k", SHAPES)
+@pytest.mark.parametrize("m", [1, 8, 9, 16, 17, 32, 33, 64, 65, 128])
+@pytest.mark.parametrize("kernel", [1, 2])
+def test_product_against_64_bits(n, k, m, kernel, device):
+    if kernel == 1 and m > 32:
+        pytest.skip("the register kernel takes up to 32 rows")
+    torch.manual_seed(n * 31 + k + m)
+    # Rows of a wider buffer and a nonsense tail past k: the kernels must honour the strides.
+    x = torch.full((m, k + 24), float("nan"), dtype=torch.bfloat16, device=device)[:, :k]
+    w = torch.full((n, k + 8), float("nan"), dtype=torch.bfloat16, device=device)[:, :k]
+    x.copy_(torch.randn(m, k, device=device))
+    w.copy_(torch.randn(n, k, device=device) / k ** 0.5)
+    bias = torch.randn(n, device=device).to(torch.bfloat16) if m % 2 else None
+    status = torch.zeros(1, dtype=torch.int32, device=device)
+    assert linear_supported(x, w, bias)
+    out = linear(x, w, bias, status=status, kernel=kernel)
+    exact = x.double() @ w.double().t() + (0.0 if bias is None else bias.double())
+    # One rounding to bf16 (2^-9 of the value) of sums whose fp32 error is below k 2^-24 of the terms' magnitude.
+    bound = exact.abs() * 2.0 ** -8 + k * 2.0 ** -23 * (x.double().abs() @ w.double().abs().t()) + 1e-30
+    assert bool(((out.double() - exact).abs() <= bound).all())
+    assert int(status.item()) == 0
+
+
+def test_infinities_and_nans_stay_where_they_belong(device):
+    for kernel, m in ((1, 5), (2, 40)):
+        x = torch.ones(m, 128, dtype=torch.bfloat16, device=device)
+        w = torch.ones(64, 128, dtype=torch.bfloat16, device=device)
+        x[1, 3], w[7, 70] = float("inf"), float("nan")
+        status = torch.zeros(1, dtype=torch.int32, device=device)
+        out = linear(x, w, status=status, kernel=kernel).float()
+        assert bool(out[:, 7].isnan().all())
+        rest = torch.cat([out[:, :7], out[:, 8:]], dim=1)
+        assert bool((rest[1] == float("inf")).all()) and bool((rest[0] == 128).all())
+
+
+def test_what_the_kernels_do_not_take_goes_to_the_library(device):
+    x, w = torch.randn(4, 12, device=device), torch.randn(6, 12, device=device)
+    status = torch.zeros(1, dtype=torch.int32, device=device)
+    for a, b in ((x, w), (x.bfloat16(), w.bfloat16()), (x[:0].bfloat16(), w.bfloat16())):
+        assert not linear_supported(a, b)
+        torch.testing.assert_close(linear(a, b, status=status), torch.nn.functional.linear(a, b))
