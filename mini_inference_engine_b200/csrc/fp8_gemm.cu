@@ -15,7 +15,7 @@
 //     128 UMMA rows are weight rows and the BN = 16..128 columns are tokens, so
 //     a handful of tokens still fills the tensor core's M and the kernel is a
 //     pure weight-streaming (HBM-bound) loop; E = 4 promotion warps, one TMA
-//     producer warp, one MMA-issuer warp that also owns the TMEM allocation.
+//     producer warp, two MMA-issuer warps.
 //     More than 128 tokens: fp8_gemm_wide_kernel (described at its definition).
 //   * A shape with fewer output tiles than SMs cuts the K range of every tile
 //     into parts that run as one thread-block cluster and are reduced through
@@ -74,6 +74,7 @@ struct ScaleStage {
 };
 
 constexpr int kNarrowEpiWarps = 4;  // promotion warps of fp8_gemm_kernel (one per TMEM lane quadrant)
+constexpr int kNarrowThreads = (kNarrowEpiWarps + 3) * 32;
 
 template <int BN>
 struct GemmSmem {
@@ -84,7 +85,11 @@ struct GemmSmem {
   static constexpr int kCtasPerSm = BN <= 32 ? 2 : 1;
   static constexpr int kBudget = (kCtasPerSm == 2 ? 100 : 200) * 1024 - kScaleBytes;
   static constexpr int kStages = (kBudget / kStageBytes) > 12 ? 12 : (kBudget / kStageBytes);
-  static constexpr int kBarBytes = (2 * kStages + 16) * 8;
+  // Accumulator ring in TMEM: up to 8 BN-column buffers, so the MMA issuers can run several K blocks ahead of the
+  // promotion, but not more buffers than stages (see done_bar).
+  static constexpr int kAccMax = (512 / kCtasPerSm) / BN < kStages ? (512 / kCtasPerSm) / BN : kStages;
+  static constexpr int kAcc = kAccMax >= 8 ? 8 : kAccMax >= 4 ? 4 : 2;
+  static constexpr int kBarBytes = (2 * kStages + 8) * 8;
   static constexpr int kTotal = kStages * kStageBytes + kBarBytes + kScaleBytes + 64 + 1024;
 };
 
@@ -110,19 +115,20 @@ __device__ __forceinline__ void store_out(const GemmParams& p, long long token, 
 }
 
 // Up to 128 tokens.  The 128 UMMA rows are weight rows (one 128-row scale block per tile), the BN columns
-// are tokens.  Warps 0..3 promote, warp 4 is the TMA producer, warp 5 issues the MMAs and owns TMEM.
+// are tokens.  Warps 0..3 promote, warp 4 is the TMA producer, warps 5 and 6 issue the MMAs of alternate K blocks (one
+// thread's wait, four MMAs and commit take about 770 cycles whatever BN is, and with a second commit per block 900:
+// longer than the block's weights take from HBM) and warp 5 owns TMEM.  A K block has one commit, on the barrier that
+// both frees its stage and hands its accumulator to the promotion.
 // grid = (tiles, split), cluster = (1, split, 1): CTA `rank` of a cluster takes the rank-th part of K.
 template <int BN>
-__global__ void __launch_bounds__((kNarrowEpiWarps + 2) * 32, (BN <= 32 ? 2 : 1))
+__global__ void __launch_bounds__(kNarrowThreads, (BN <= 32 ? 2 : 1))
     fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                     const GemmParams p) {
   using S = GemmSmem<BN>;
   using SS = ScaleStage<BN>;
   constexpr int E = kNarrowEpiWarps;
   constexpr int kStages = S::kStages;
-  // Accumulator ring in TMEM: as many BN-column buffers as fit (at most 8), so the MMA issuer can run
-  // several K blocks ahead of the promotion.
-  constexpr int kAcc = (512 / S::kCtasPerSm) / BN > 8 ? 8 : (512 / S::kCtasPerSm) / BN;
+  constexpr int kAcc = S::kAcc;
   constexpr uint32_t kTmemCols = kAcc * BN < 32 ? 32 : kAcc * BN;
   static_assert((kTmemCols & (kTmemCols - 1)) == 0 && kTmemCols <= 512, "TMEM columns must be a power of two <= 512");
   static_assert(BN % 16 == 0, "token tile must be a multiple of 16");
@@ -135,9 +141,10 @@ __global__ void __launch_bounds__((kNarrowEpiWarps + 2) * 32, (BN <= 32 ? 2 : 1)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* stage_base = smem;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kStages * S::kStageBytes);
-  uint64_t* empty_bar = full_bar + kStages;
-  uint64_t* tmem_full = empty_bar + kStages;
-  uint64_t* tmem_empty = tmem_full + 8;
+  // The MMAs of the stage's K block have completed: waited for by the producer and, before the block after next of the
+  // same stage can complete (kAcc <= kStages), by the promotion.
+  uint64_t* done_bar = full_bar + kStages;
+  uint64_t* tmem_empty = done_bar + kStages;
   float* sscale = reinterpret_cast<float*>(tmem_empty + 8);  // staged scale products of the current K chunk
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sscale + SS::kFloats);
 
@@ -157,12 +164,9 @@ __global__ void __launch_bounds__((kNarrowEpiWarps + 2) * 32, (BN <= 32 ? 2 : 1)
   if (warp == E && lane == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+      mbar_init(&done_bar[s], 1);
     }
-    for (int b = 0; b < kAcc; ++b) {
-      mbar_init(&tmem_full[b], 1);
-      mbar_init(&tmem_empty[b], E);
-    }
+    for (int b = 0; b < kAcc; ++b) mbar_init(&tmem_empty[b], E);
     mbar_fence_init();
     tma_prefetch_desc(&map_w);
     tma_prefetch_desc(&map_x);
@@ -203,7 +207,7 @@ __global__ void __launch_bounds__((kNarrowEpiWarps + 2) * 32, (BN <= 32 ? 2 : 1)
           tma_load_2d(dst + kTileR * kBlockK, &map_x, &full_bar[s], kb * kBlockK, tt * BN);
           continue;
         }
-        if (!mbar_wait_bounded(&empty_bar[s], ((n / kStages) & 1u) ^ 1u)) {
+        if (!mbar_wait_bounded(&done_bar[s], ((n / kStages) & 1u) ^ 1u)) {
           raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
           break;
         }
@@ -212,12 +216,12 @@ __global__ void __launch_bounds__((kNarrowEpiWarps + 2) * 32, (BN <= 32 ? 2 : 1)
         tma_load_2d(dst + kTileR * kBlockK, &map_x, &full_bar[s], kb * kBlockK, tt * BN);
       }
     }
-  } else if (warp == E + 1) {
-    // ---------------- MMA issuer ----------------
+  } else if (warp > E) {
+    // ---------------- MMA issuers ----------------
     if (lane == 0) {
       constexpr uint32_t idesc = instr_desc_f8(BN);
-      uint32_t n = 0;
-      for (int kb = kb_first; kb < kb_last; ++kb, ++n) {
+      const uint32_t blocks = (uint32_t)(kb_last - kb_first);
+      for (uint32_t n = (uint32_t)(warp - (E + 1)); n < blocks; n += 2) {
         const int s = n % kStages, b = n % kAcc;
         if (!mbar_wait_bounded(&full_bar[s], (n / kStages) & 1u) ||
             !mbar_wait_bounded(&tmem_empty[b], ((n / kAcc) & 1u) ^ 1u)) {
@@ -233,8 +237,7 @@ __global__ void __launch_bounds__((kNarrowEpiWarps + 2) * 32, (BN <= 32 ? 2 : 1)
           umma_f8(tmem_base + b * BN, da + (uint64_t)(k * kUmmaK / 16), db + (uint64_t)(k * kUmmaK / 16), idesc,
                   k > 0 ? 1u : 0u);
         }
-        umma_commit(&empty_bar[s]);  // frees the smem stage once these MMAs have read it
-        umma_commit(&tmem_full[b]);  // hands the K block's accumulator to the promotion warps
+        umma_commit(&done_bar[s]);  // frees the smem stage and hands the accumulator to the promotion warps
       }
     }
   } else {
@@ -258,7 +261,7 @@ __global__ void __launch_bounds__((kNarrowEpiWarps + 2) * 32, (BN <= 32 ? 2 : 1)
       for (int kk = 0; kk < kc; ++kk, ++n) {
         const int b = n % kAcc;
         const float* s_col = sscale + kk * BN;
-        if (!mbar_wait_bounded(&tmem_full[b], (n / kAcc) & 1u)) {
+        if (!mbar_wait_bounded(&done_bar[n % kStages], (n / kStages) & 1u)) {
           raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
           ok = false;
           break;
@@ -372,25 +375,29 @@ __global__ void __launch_bounds__((kNarrowEpiWarps + 2) * 32, (BN <= 32 ? 2 : 1)
 //     idle) stage ring in a swizzled [row][4-column group] layout, and after a cluster barrier reads the
 //     column slice it owns from every peer with 16-byte distributed-shared-memory loads, adds the partials
 //     in rank order (a fixed order: results do not depend on timing) and stores bf16.  No global scratch.
-//   * 12 warps: 8 promotion warps (two warpgroups), one TMA producer, one MMA issuer, two idle.  The
-//     producer warpgroup hands most of its registers to the promotion warps (setmaxnreg), which keep the
-//     128 x 256 fp32 result in registers (128 per thread) next to two 32-column landing buffers.
-//   * Two 256-column accumulators ping-pong in TMEM.  Promotion of one K block: two rounds of two TMEM loads
-//     in flight; the multiply-adds (packed fp32x2) of one landing buffer run while the other is being
-//     refilled, and the first loads of the next K block are issued before the last columns of the current
-//     one are consumed.  The accumulator goes back to the MMA issuer as soon as its last load has landed.
+//   * Two 256-column accumulators ping-pong in TMEM, each with its own MMA issuer thread, and a K block has one
+//     commit, on the barrier that both frees its stage and hands its accumulator over: one thread's wait, four MMAs
+//     and commit take about 770 cycles, the MMAs 512 (two issuers measured 512 with nothing to promote).
+//   * 20 warps: 16 promotion warps, one TMA producer, two MMA issuers, one idle.  A promotion warp keeps 32 rows x 64
+//     columns of the fp32 result in registers and adds a K block in two loads of 32 columns (packed fp32x2
+//     multiply-adds); four warps per scheduler hide the loads' latency (eight warps with 128 columns each and the
+//     loads pipelined by hand: 4736 x 19456 x 2560 307 us, sixteen 264).  The accumulator goes back to its issuer
+//     as soon as the second load has landed.  A thread requests its row's scale one K block ahead.
+//   * A pair of CTAs on one 256 x 256 tile (cta_group::2, a third less operand traffic) measured 3 % faster at 12032
+//     tokens and up to 20 % slower at a few hundred, where its tiles leave more rows empty.
 // --------------------------------------------------------------------------
 constexpr int kWideBN = 256;
-constexpr int kWideEpiWarps = 8;
-constexpr int kWideThreads = 384;
-constexpr int kWideStages = 4;
-constexpr int kWideStageBytes = kTileR * kBlockK + kWideBN * kBlockK;  // 48 KiB
-constexpr int kWideChunkKb = 16;                                        // K blocks of scales staged at a time
-constexpr int kWideScaleFloats = kWideChunkKb * (kTileR + 2);
+constexpr int kWideEpiWarps = 16;
+constexpr int kWideThreads = 640;
 constexpr int kWideStoreBytes = kWideEpiWarps * 2048;  // per promotion warp: 32 rows x 32 columns of 16-bit output
-constexpr int kWideSmemBytes = kWideStages * kWideStageBytes + kWideStoreBytes + (2 * kWideStages + 4) * 8 +
-                               kWideScaleFloats * 4 + 64 + 1024;
+
+constexpr int kWideStages = 4;
+constexpr int kWideAcc = 2;
+constexpr int kWideStageBytes = kTileR * kBlockK + kWideBN * kBlockK;  // 48 KiB
+constexpr int kWideSmemBytes =
+    kWideStages * kWideStageBytes + kWideStoreBytes + (2 * kWideStages + kWideAcc) * 8 + 64 + 1024;
 static_assert(kWideStages * kWideStageBytes >= kTileR * kWideBN * 4, "stage ring too small for the fp32 partial tile");
+static_assert(kWideAcc <= kWideStages, "a done barrier must not run a phase ahead of the promotion");
 
 struct WideItem {
   int tm, tn, k0, k1;
@@ -401,7 +408,7 @@ struct WideItem {
 // rank-th part of its K range.
 __device__ __forceinline__ bool wide_item(int first, int tiles, int tiles_m, int kb_total, int split, int rank,
                                           int idx, WideItem& it) {
-  const int tile = first + blockIdx.x + idx * gridDim.x;
+  const int tile = first + (int)blockIdx.x + idx * (int)gridDim.x;
   if (tile >= tiles || (split > 1 && idx > 0)) return false;
   it.tm = tile % tiles_m;
   it.tn = tile / tiles_m;
@@ -421,21 +428,16 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_addr, uint32_t ra
   return v;
 }
 
-__device__ __forceinline__ void tmem_ld_wait_pin(float (&a)[32], float (&b)[32]) {
+__device__ __forceinline__ void tmem_ld_wait_pin(float (&a)[32]) {
   // The wait is what makes the registers of the earlier tcgen05.ld valid; naming them as in/out operands
-  // keeps every later use of a and b behind it.
+  // keeps every later use of a behind it.
   uint32_t* r = reinterpret_cast<uint32_t*>(a);
-  uint32_t* q = reinterpret_cast<uint32_t*>(b);
   asm volatile("tcgen05.wait::ld.sync.aligned;"
                : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
                  "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
                  "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]),
                  "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]),
-                 "+r"(r[29]), "+r"(r[30]), "+r"(r[31]), "+r"(q[0]), "+r"(q[1]), "+r"(q[2]), "+r"(q[3]), "+r"(q[4]),
-                 "+r"(q[5]), "+r"(q[6]), "+r"(q[7]), "+r"(q[8]), "+r"(q[9]), "+r"(q[10]), "+r"(q[11]),
-                 "+r"(q[12]), "+r"(q[13]), "+r"(q[14]), "+r"(q[15]), "+r"(q[16]), "+r"(q[17]), "+r"(q[18]),
-                 "+r"(q[19]), "+r"(q[20]), "+r"(q[21]), "+r"(q[22]), "+r"(q[23]), "+r"(q[24]), "+r"(q[25]),
-                 "+r"(q[26]), "+r"(q[27]), "+r"(q[28]), "+r"(q[29]), "+r"(q[30]), "+r"(q[31])
+                 "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
                :
                : "memory");
 }
@@ -508,20 +510,19 @@ __device__ __forceinline__ void wide_cluster_reduce(const GemmParams& p, uint32_
 __global__ void __launch_bounds__(kWideThreads, 1)
     fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                          const GemmParams p) {
-  constexpr int BN = kWideBN, E = kWideEpiWarps, kStages = kWideStages, kAcc = 2;
-  constexpr int kCols = BN / 2;  // columns owned by one promotion warp
+  constexpr int BN = kWideBN, E = kWideEpiWarps, kStages = kWideStages, kStageBytes = kWideStageBytes;
+  constexpr int kAcc = kWideAcc;
+  constexpr int kCols = BN * 4 / E;  // columns owned by one promotion warp
   constexpr uint32_t kTmemCols = 512;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* stage_base = smem;
-  uint8_t* store_base = smem + kStages * kWideStageBytes;
+  uint8_t* store_base = smem + kStages * kStageBytes;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(store_base + kWideStoreBytes);
-  uint64_t* empty_bar = full_bar + kStages;
-  uint64_t* tmem_full = empty_bar + kStages;
-  uint64_t* tmem_empty = tmem_full + kAcc;
-  float* sscale = reinterpret_cast<float*>(tmem_empty + kAcc);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sscale + kWideScaleFloats);
+  uint64_t* done_bar = full_bar + kStages;  // the MMAs of the stage's K block have completed
+  uint64_t* tmem_empty = done_bar + kStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + kAcc);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kb_total = (p.k + kBlockK - 1) / kBlockK;
@@ -532,12 +533,9 @@ __global__ void __launch_bounds__(kWideThreads, 1)
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+      mbar_init(&done_bar[s], 1);
     }
-    for (int b = 0; b < kAcc; ++b) {
-      mbar_init(&tmem_full[b], 1);
-      mbar_init(&tmem_empty[b], E);
-    }
+    for (int b = 0; b < kAcc; ++b) mbar_init(&tmem_empty[b], E);
     mbar_fence_init();
     tma_prefetch_desc(&map_x);
     tma_prefetch_desc(&map_w);
@@ -550,6 +548,13 @@ __global__ void __launch_bounds__(kWideThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  auto load_x = [&](uint32_t s, int kb, const WideItem& it) {
+    tma_load_2d(stage_base + (size_t)s * kStageBytes, &map_x, &full_bar[s], kb * kBlockK, it.tm * kTileR);
+  };
+  auto load_w = [&](uint32_t s, int kb, const WideItem& it) {
+    tma_load_2d(stage_base + (size_t)s * kStageBytes + kTileR * kBlockK, &map_w, &full_bar[s], kb * kBlockK,
+                it.tn * BN);
+  };
   // Barriers, tensor-map prefetch and the TMEM allocation above overlap the tail of the previous kernel.
   // So can the weights (nothing on the stream writes them): the producer requests the weight half of its
   // first stages before the launch-chain wait and adds the activation half afterwards.
@@ -558,9 +563,8 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     WideItem first;
     if (wide_item(p.tile_begin, tiles, tiles_m, kb_total, split, rank, 0, first)) {
       for (int kb = first.k0; kb < first.k1 && prefetched < (uint32_t)kStages; ++kb, ++prefetched) {
-        mbar_expect_tx(&full_bar[prefetched], kWideStageBytes);
-        tma_load_2d(stage_base + (size_t)prefetched * kWideStageBytes + kTileR * kBlockK, &map_w,
-                    &full_bar[prefetched], kb * kBlockK, first.tn * BN);
+        mbar_expect_tx(&full_bar[prefetched], kStageBytes);
+        load_w(prefetched, kb, first);
       }
     }
   }
@@ -572,11 +576,12 @@ __global__ void __launch_bounds__(kWideThreads, 1)
   uint32_t total_blocks = 0;
   {
     WideItem it;
-    for (int idx = 0; wide_item(p.tile_begin, tiles, tiles_m, kb_total, split, rank, idx, it); ++idx) total_blocks += (uint32_t)(it.k1 - it.k0);
+    for (int idx = 0; wide_item(p.tile_begin, tiles, tiles_m, kb_total, split, rank, idx, it); ++idx)
+      total_blocks += (uint32_t)(it.k1 - it.k0);
   }
 
   if (warp >= E) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
     if (warp == E && lane == 0) {
       // ---------------- TMA producer ----------------
       uint32_t n = 0;
@@ -584,42 +589,41 @@ __global__ void __launch_bounds__(kWideThreads, 1)
       WideItem it;
       for (int idx = 0; ok && wide_item(p.tile_begin, tiles, tiles_m, kb_total, split, rank, idx, it); ++idx) {
         for (int kb = it.k0; kb < it.k1; ++kb, ++n) {
-          const int s = n % kStages;
-          uint8_t* dst = stage_base + (size_t)s * kWideStageBytes;
+          const uint32_t s = n % kStages;
           if (n < prefetched) {  // the weight half is already on its way
-            tma_load_2d(dst, &map_x, &full_bar[s], kb * kBlockK, it.tm * kTileR);
+            load_x(s, kb, it);
             continue;
           }
-          if (!mbar_wait_bounded(&empty_bar[s], ((n / kStages) & 1u) ^ 1u)) {
+          if (!mbar_wait_bounded(&done_bar[s], ((n / kStages) & 1u) ^ 1u)) {
             raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
             ok = false;
             break;
           }
-          mbar_expect_tx(&full_bar[s], kWideStageBytes);
-          tma_load_2d(dst, &map_x, &full_bar[s], kb * kBlockK, it.tm * kTileR);
-          tma_load_2d(dst + kTileR * kBlockK, &map_w, &full_bar[s], kb * kBlockK, it.tn * BN);
+          mbar_expect_tx(&full_bar[s], kStageBytes);
+          load_x(s, kb, it);
+          load_w(s, kb, it);
         }
       }
-    } else if (warp == E + 1 && lane == 0) {
-      // ---------------- MMA issuer ----------------
+    } else if ((warp == E + 1 || warp == E + 2) && lane == 0) {
+      // ---------------- MMA issuers, one per accumulator ----------------
       constexpr uint32_t idesc = instr_desc_f8(BN);
-      for (uint32_t n = 0; n < total_blocks; ++n) {
-        const int s = n % kStages, b = n % kAcc;
+      const int b = warp - (E + 1);
+      for (uint32_t n = b; n < total_blocks; n += kAcc) {
+        const int s = n % kStages;
         if (!mbar_wait_bounded(&full_bar[s], (n / kStages) & 1u) ||
             !mbar_wait_bounded(&tmem_empty[b], ((n / kAcc) & 1u) ^ 1u)) {
           raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
           break;
         }
         tc_fence_after();
-        const uint32_t a_addr = smem_u32(stage_base + (size_t)s * kWideStageBytes);
+        const uint32_t a_addr = smem_u32(stage_base + (size_t)s * kStageBytes);
         const uint64_t da = smem_desc_k128(a_addr), db = smem_desc_k128(a_addr + kTileR * kBlockK);
 #pragma unroll
         for (int k = 0; k < kBlockK / kUmmaK; ++k) {
           umma_f8(tmem_base + b * BN, da + (uint64_t)(k * kUmmaK / 16), db + (uint64_t)(k * kUmmaK / 16), idesc,
                   k > 0 ? 1u : 0u);
         }
-        umma_commit(&empty_bar[s]);  // frees the smem stage once these MMAs have read it
-        umma_commit(&tmem_full[b]);  // hands the K block's accumulator to the promotion warps
+        umma_commit(&done_bar[s]);  // frees the smem stage and hands the accumulator to the promotion warps
       }
     }
     __syncwarp();
@@ -628,75 +632,52 @@ __global__ void __launch_bounds__(kWideThreads, 1)
       cluster_sync_all();  // peers have read this CTA's partial
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
     // ---------------- Promotion warps ----------------
-    constexpr int kEpiThreads = E * 32;
-    const int quad = warp & 3, half = warp >> 2;
+    const int quad = warp & 3;
     const int row_in_tile = quad * 32 + lane;
-    const int col0 = half * kCols;
+    const int col0 = (warp >> 2) * kCols;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)col0;
     const int epi_tid = threadIdx.x;
     float acc[kCols];
-    float buf_a[32], buf_b[32];
 #pragma unroll
     for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
     uint32_t n = 0;
     bool ok = true;
-    // First accumulator: its first 64 columns start the pipeline.
-    if (total_blocks > 0) {
-      ok = mbar_wait_bounded(&tmem_full[0], 0);
-      if (!ok) raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
-      tc_fence_after();
-      if (ok) {
-        tmem_ld32(lane_addr, buf_a);
-        tmem_ld32(lane_addr + 32, buf_b);
-      }
-    }
     WideItem it;
     for (int idx = 0; ok && wide_item(p.tile_begin, tiles, tiles_m, kb_total, split, rank, idx, it); ++idx) {
       const int tok0 = it.tm * kTileR;
-      for (int kb0 = it.k0; kb0 < it.k1 && ok; kb0 += kWideChunkKb) {
-        const int kc = it.k1 - kb0 < kWideChunkKb ? it.k1 - kb0 : kWideChunkKb;
-        // Stage this chunk's scales (all loads in flight together).
-        epi_bar_sync(kEpiThreads);  // the previous chunk's readers are done
-        float* s_w = sscale + kWideChunkKb * kTileR;
-        for (int i = epi_tid; i < kc * kTileR; i += kEpiThreads) {
-          const int kk = i / kTileR, tok = tok0 + i % kTileR;
-          sscale[i] = tok < p.m ? p.a_scale[(long long)(kb0 + kk) * p.a_scale_ld + tok] : 0.f;
+      // The scales of this thread's row and of its columns' weight block, requested a K block ahead.
+      const int blk = it.tn * 2 + col0 / 128;
+      const bool row_live = tok0 + row_in_tile < p.m, col_live = blk * 128 < p.n;
+      const float* a_at = p.a_scale + (long long)it.k0 * p.a_scale_ld + (row_live ? tok0 + row_in_tile : 0);
+      const float* w_at = p.w_scale + (col_live ? (long long)blk * p.w_scale_ld : 0) + it.k0;
+      float a_next = row_live ? *a_at : 0.f, w_next = col_live ? *w_at : 0.f;
+      for (int kb = it.k0; kb < it.k1; ++kb, ++n) {
+        const uint32_t taddr = lane_addr + (n & 1) * BN;
+        if (!mbar_wait_bounded(&done_bar[n % kStages], (n / kStages) & 1u)) {
+          raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
+          ok = false;
+          break;
         }
-        for (int i = epi_tid; i < kc * 2; i += kEpiThreads) {
-          const int kk = i >> 1, blk = it.tn * 2 + (i & 1);
-          s_w[i] = blk * 128 < p.n ? p.w_scale[(long long)blk * p.w_scale_ld + kb0 + kk] : 0.f;
+        tc_fence_after();
+        const float s = a_next * w_next;
+        if (kb + 1 < it.k1) {
+          a_at += p.a_scale_ld;
+          if (row_live) a_next = *a_at;
+          if (col_live) w_next = *++w_at;
         }
-        epi_bar_sync(kEpiThreads);
-        for (int kk = 0; kk < kc; ++kk, ++n) {
-          const int b = n & 1;
-          const float s = sscale[kk * kTileR + row_in_tile] * s_w[kk * 2 + half];
-          const uint32_t taddr = lane_addr + (uint32_t)(b * BN);
-          tmem_ld_wait_pin(buf_a, buf_b);  // columns 0..63 have landed
-          promote32(acc, buf_a, s);
-          tmem_ld32(taddr + 64, buf_a);
-          promote32(acc + 32, buf_b, s);
-          tmem_ld32(taddr + 96, buf_b);
-          tmem_ld_wait_pin(buf_a, buf_b);  // columns 64..127 have landed
-          // Every load of this accumulator has landed: hand the buffer back to the MMA issuer.
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&tmem_empty[b]);
-          promote32(acc + 64, buf_a, s);
-          const bool more = n + 1 < total_blocks;
-          if (more) {
-            if (!mbar_wait_bounded(&tmem_full[b ^ 1], ((n + 1) >> 1) & 1u)) {
-              raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
-              ok = false;
-            }
-            tc_fence_after();
-            if (ok) tmem_ld32(lane_addr + (uint32_t)((b ^ 1) * BN), buf_a);
-          }
-          promote32(acc + 96, buf_b, s);
-          if (more && ok) tmem_ld32(lane_addr + (uint32_t)((b ^ 1) * BN) + 32, buf_b);
-          if (!ok) break;
-        }
+        float buf[32];
+        tmem_ld32(taddr, buf);
+        tmem_ld_wait_pin(buf);
+        promote32(acc, buf, s);
+        tmem_ld32(taddr + 32, buf);
+        tmem_ld_wait_pin(buf);
+        // Every load of this accumulator has landed: hand the buffer back to the MMA issuer.
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tmem_empty[n & 1]);
+        promote32(acc + 32, buf, s);
       }
       if (!ok) break;
 
@@ -915,7 +896,6 @@ template <int BN>
 int launch_gemm(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p, long long tiles, int split,
                 cudaStream_t stream) {
   using S = GemmSmem<BN>;
-  constexpr int E = kNarrowEpiWarps;
   static bool configured[64] = {false};
   int dev = 0;
   MIE_CUDA(cudaGetDevice(&dev));
@@ -926,7 +906,7 @@ int launch_gemm(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& 
   }
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3((unsigned)tiles, (unsigned)split, 1);
-  config.blockDim = dim3((E + 2) * 32, 1, 1);
+  config.blockDim = dim3(kNarrowThreads, 1, 1);
   config.dynamicSmemBytes = S::kTotal;
   config.stream = stream;
   cudaLaunchAttribute attr[2];
