@@ -13,6 +13,8 @@ quantiser.  2,112 bytes per token and layer at 8 KV heads instead of 4,096.
 
 from __future__ import annotations
 
+import math
+
 import torch
 
 from ... import _lib
@@ -26,7 +28,10 @@ class Fp8KvPool:
 
     def __init__(self, layers: int, num_pages: int, kv_heads: int, device: torch.device) -> None:
         self.layers, self.num_pages, self.kv_heads = layers, num_pages, kv_heads
-        self.data = torch.zeros(layers, num_pages, kv_heads, 2, PAGE, HEAD_DIM, dtype=torch.uint8, device=device)
+        shape = (layers, num_pages, kv_heads, 2, PAGE, HEAD_DIM)
+        flat = torch.zeros(math.prod(shape) + 1024, dtype=torch.uint8, device=device)
+        start = -flat.data_ptr() % 1024  # small tensors are only 512-byte aligned
+        self.data = flat[start:start + math.prod(shape)].view(shape)
         self.scales = torch.zeros(layers, num_pages, kv_heads, 2, PAGE, dtype=torch.float32, device=device)
         if self.data.data_ptr() % 1024 or self.scales.data_ptr() % 128:
             raise RuntimeError("the allocator returned an unaligned FP8 KV pool")
