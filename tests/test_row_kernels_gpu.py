@@ -1,0 +1,85 @@
+"""Row kernels at the sizes where their lanes, alignments and quotients can go wrong."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from mini_inference_engine_b200 import _lib
+from mini_inference_engine_b200.engine.kernels import sm89_fp8
+from oracle import hot_path
+
+pytestmark = pytest.mark.gpu
+
+
+def test_quotients_of_the_quantiser_are_ieee_quotients(device):
+    """Zeros of both signs, tiny and huge groups, infinities and NaN: the bytes of an IEEE division."""
+
+    torch.manual_seed(0)
+    x = torch.randn(64, 256).to(torch.bfloat16)
+    x[0], x[1], x[2, ::2], x[3] = 0.0, -0.0, -0.0, x[3] * 1e-37
+    x[4] *= 3e37
+    x[5, 7], x[6, 9], x[7, 11] = float("inf"), float("-inf"), float("nan")
+    x[8:24] *= torch.exp(torch.linspace(-30, 30, 16))[:, None].to(torch.bfloat16)
+    got, scales = sm89_fp8.quantize_sm89_fp8_activation(x.to(device))
+    groups = x.float().view(64, 2, 128)
+    want_scale = torch.nan_to_num(groups.abs(), nan=0.0, posinf=float("inf")).amax(-1) / 448.0
+    want = (groups / want_scale.clamp_min(1e-12)[..., None]).view(64, 256)
+    # the conversion saturates where torch's overflows to NaN; both keep NaN
+    want = torch.where(want.isnan(), want, want.clamp(-448, 448)).to(torch.float8_e4m3fn)
+    assert torch.equal(scales.cpu(), want_scale)
+    nan = want.float().isnan()
+    assert torch.equal(got.cpu().float().isnan(), nan)
+    assert torch.equal(got.cpu().view(torch.uint8)[~nan], want.view(torch.uint8)[~nan])
+
+
+@pytest.mark.parametrize("heads", [(1, 1), (3, 1), (16, 8), (32, 8), (40, 20)])
+@pytest.mark.parametrize("offset", [0, 4])  # rows aligned to 16 bytes, and to 8 only
+def test_qkv_rows_of_odd_head_counts_and_alignments(heads, offset, device, status_clean):
+    """Half-warps of different head kinds share a warp; the e4m3 pool holds the quantised bf16 rows."""
+
+    from mini_inference_engine_b200.engine.model_runner.qwen3_decode import Qwen3Shape, rope_table
+
+    torch.manual_seed(1)
+    q_heads, kv_heads = heads
+    tokens, pages, width = 5, 4, (q_heads + 2 * kv_heads) * 128
+    rows = torch.randn(tokens, width + 8).to(torch.bfloat16)
+    qkv = rows[:, offset:offset + width]
+    weights = [(1 + 0.1 * torch.randn(128)).to(torch.bfloat16) for _ in range(2)]
+    positions = torch.tensor([0, 17, 18, 31, 40], dtype=torch.int32)
+    owners = torch.zeros(tokens, dtype=torch.int32)
+    tables = torch.tensor([[2, 0, 3]], dtype=torch.int32)
+    q, k, v = (part.reshape(1, tokens, -1, 128) for part in qkv.split([q_heads * 128, kv_heads * 128, kv_heads * 128], 1))
+    cos, sin = hot_path.rope_cos_sin(positions.view(1, tokens), 128, 5_000_000.0)
+    q_want, k_want = hot_path.apply_rotary_pos_emb(hot_path.rms_norm(q, weights[0], 1e-6).transpose(1, 2),
+                                                   hot_path.rms_norm(k, weights[1], 1e-6).transpose(1, 2), cos, sin)
+    keys_want = torch.zeros(pages, kv_heads, 16, 128, dtype=torch.bfloat16)
+    values_want = torch.zeros_like(keys_want)
+    hot_path.write_packed_kv(k_want, v.transpose(1, 2), owners, positions, tables, keys_want, values_want)
+
+    d_rows = rows.to(device)
+    d_qkv, d_w = d_rows[:, offset:offset + width], [w.to(device) for w in weights]
+    rope, status = rope_table(Qwen3Shape(), 64, device), _lib.status_word(device)
+    keys = torch.zeros(pages, kv_heads, 16, 128, dtype=torch.bfloat16, device=device)
+    values, queries = torch.zeros_like(keys), torch.empty(tokens, q_heads, 128, dtype=torch.bfloat16, device=device)
+    meta = [t.to(device) for t in (positions, owners, tables)]
+    common = (_lib.ptr(d_qkv), d_qkv.stride(0), _lib.ptr(d_w[0]), _lib.ptr(d_w[1]), _lib.ptr(rope), 64,
+              *(_lib.index_arg(t) for t in meta), _lib.ptr(queries))
+    tail = (tokens, q_heads, kv_heads)
+    _lib.check(_lib.load().mie_qkv_norm_rope_write(*common, _lib.view4_arg(keys), _lib.view4_arg(values), *tail, 16, pages,
+                                                   1, 3, 1e-6, _lib.ptr(status), _lib.stream_arg(device)))
+    raw = torch.zeros(pages * kv_heads * 4096 + offset, dtype=torch.uint8, device=device)
+    data, scales = raw[offset:], torch.zeros(pages, kv_heads, 2, 16, device=device)
+    _lib.check(_lib.load().mie_qkv_norm_rope_write_kv8(*common, _lib.ptr(data), kv_heads * 4096, _lib.ptr(scales), *tail,
+                                                       pages, 1, 3, 1e-6, _lib.ptr(status), _lib.stream_arg(device)))
+    torch.cuda.synchronize()
+    assert torch.equal(values.cpu(), values_want)
+    # Rounding points are the oracle's; a sum in another order can move the norm by one bf16 step of an entry (2^-8).
+    for got, want in ((queries.cpu(), q_want[0].transpose(0, 1)), (keys.cpu(), keys_want)):
+        assert (got.float() - want.float()).abs().max() <= 2 ** -7 * want.float().abs().max()
+        assert (got != want).float().mean() < 0.05
+    pool = data.view(pages, kv_heads, 2, 16, 128).cpu()
+    for which, dense in enumerate((keys, values)):
+        want_q, want_s = hot_path.quantize_kv_rows(dense.cpu())
+        assert torch.equal(pool[:, :, which], want_q)
+        assert torch.equal(scales[:, :, which].cpu(), want_s)
