@@ -332,6 +332,34 @@ int mie_fp8_gemm(const void* x8, int64_t ldx, const float* a_scale, int32_t a_sc
                  int64_t ldw, const float* w_scale, int32_t w_scale_ld, void* y, int64_t ldy, int32_t out_dtype,
                  int32_t m, int32_t n, int32_t k, int32_t max_split, int32_t flags, int32_t* status, void* stream);
 
+/*
+ * The same product with its rows finished in place of stored, for the token
+ * counts at which mie_fp8_gemm_finishes(m, n) is 1 (decode batches; n = weight
+ * rows): one launch where the unfused chain has two, with that chain's rounding
+ * points.
+ *
+ * mie_fp8_gemm_silu: w8 holds [gate | up], each `cols` rows (a multiple of
+ * 128); q / scales receive bf16(bf16(silu(gate)) * up) quantised for the next
+ * product as mie_silu_mul does it.
+ *
+ * mie_fp8_gemm_qkv: w8 holds [q | k | v] heads of 128 rows; what follows the
+ * product is mie_qkv_norm_rope_write, or with kv_pool (then block_size is 16
+ * and the page views are not read) mie_qkv_norm_rope_write_kv8.
+ */
+int mie_fp8_gemm_finishes(int32_t m, int32_t n);
+int mie_fp8_gemm_silu(const void* x8, int64_t ldx, const float* a_scale, int32_t a_scale_ld, const void* w8,
+                      int64_t ldw, const float* w_scale, int32_t w_scale_ld, void* q, int64_t ldq, float* scales,
+                      int32_t scale_ld, int32_t m, int32_t cols, int32_t k, int32_t max_split, int32_t flags,
+                      int32_t* status, void* stream);
+int mie_fp8_gemm_qkv(const void* x8, int64_t ldx, const float* a_scale, int32_t a_scale_ld, const void* w8,
+                     int64_t ldw, const float* w_scale, int32_t w_scale_ld, const void* q_weight,
+                     const void* k_weight, const void* cos_sin, int32_t max_pos, mie_index_t positions,
+                     mie_index_t token_to_sequence, mie_index_t block_tables, void* q_out, mie_view4_t key_blocks,
+                     mie_view4_t value_blocks, void* kv_pool, int64_t page_stride_bytes, float* kv_scales, int32_t m,
+                     int32_t k, int32_t q_heads, int32_t kv_heads, int32_t block_size, int32_t num_blocks,
+                     int32_t table_rows, int32_t table_width, float eps, int32_t max_split, int32_t flags,
+                     int32_t* status, void* stream);
+
 /* ------------------------------------------------------------------------
  * Fused memory-bound glue (bf16 activations)
  * ---------------------------------------------------------------------- */

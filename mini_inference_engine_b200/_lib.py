@@ -107,6 +107,15 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
                                                    c_void_p, c_void_p]),
     "mie_fp8_quantize": (ctypes.c_int, [c_void_p, c_int64, c_int32, c_void_p, c_int64, c_void_p, c_int32, c_int32,
                                         c_int32, c_void_p]),
+    "mie_fp8_gemm_finishes": (ctypes.c_int, [c_int32, c_int32]),
+    "mie_fp8_gemm_silu": (ctypes.c_int, [c_void_p, c_int64, c_void_p, c_int32, c_void_p, c_int64, c_void_p, c_int32,
+                                         c_void_p, c_int64, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32,
+                                         c_int32, c_void_p, c_void_p]),
+    "mie_fp8_gemm_qkv": (ctypes.c_int, [c_void_p, c_int64, c_void_p, c_int32, c_void_p, c_int64, c_void_p, c_int32,
+                                        c_void_p, c_void_p, c_void_p, c_int32, IndexT, IndexT, IndexT, c_void_p,
+                                        View4T, View4T, c_void_p, c_int64, c_void_p, c_int32, c_int32, c_int32,
+                                        c_int32, c_int32, c_int32, c_int32, c_int32, c_float, c_int32, c_int32,
+                                        c_void_p, c_void_p]),
     "mie_fp8_gemm": (ctypes.c_int, [c_void_p, c_int64, c_void_p, c_int32, c_void_p, c_int64, c_void_p, c_int32,
                                     c_void_p, c_int64, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32,
                                     c_void_p, c_void_p]),
@@ -254,7 +263,9 @@ def index_arg(tensor: torch.Tensor | None) -> IndexT:
                   strides[1] if len(strides) > 1 else 0)
 
 
-def view4_arg(tensor: torch.Tensor) -> View4T:
+def view4_arg(tensor: torch.Tensor | None) -> View4T:
+    if tensor is None:
+        return View4T(None, (c_int64 * 4)(0, 0, 0, 0))
     if tensor.ndim != 4:
         raise ValueError("expected a 4-D tensor")
     return View4T(tensor.data_ptr(), (c_int64 * 4)(*tensor.stride()))

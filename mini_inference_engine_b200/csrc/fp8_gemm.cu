@@ -14,8 +14,10 @@
 //   * Two kernels.  Up to 128 tokens (decode): fp8_gemm_kernel, "swapped" - the
 //     128 UMMA rows are weight rows and the BN = 16..128 columns are tokens, so
 //     a handful of tokens still fills the tensor core's M and the kernel is a
-//     pure weight-streaming (HBM-bound) loop; E = 4 promotion warps, one TMA
-//     producer warp, two MMA-issuer warps.
+//     pure weight-streaming (HBM-bound) loop; 4 or 8 promotion warps, one TMA
+//     producer warp, two MMA-issuer warps.  Its rows can be finished in place of
+//     stored: SiLU(gate) * up with the next GEMM's quantisation, or the q/k norm,
+//     RoPE and cache write of a merged qkv projection (Finish).
 //     More than 128 tokens: fp8_gemm_wide_kernel (described at its definition).
 //   * A shape with fewer output tiles than SMs cuts the K range of every tile
 //     into parts that run as one thread-block cluster and are reduced through
@@ -30,6 +32,7 @@
 
 #include "common.cuh"
 #include "glue.cuh"
+#include "qkv_rows.cuh"
 #include "umma.cuh"
 
 namespace mie {
@@ -63,6 +66,18 @@ struct GemmParams {
   // early_release: the next launch may start before this one's wait (not when it is the second launch of a
   // two-launch GEMM, which takes the first one's wait for its own).
   int tile_begin, tile_end, late_wait, early_release;
+  // Finish::kSilu: the quantised result (y is not written).
+  uint8_t* q;
+  long long ldq;
+  float* q_scales;
+  int q_scale_ld;
+};
+
+// What the narrow kernel does with a finished row of 128 outputs of one token.
+enum class Finish {
+  kStore,  // bf16 / fp16 to y
+  kSilu,   // weights [gate | up]: SiLU(gate) * up as e4m3 with one scale per token and 128 columns
+  kQkv     // weights [q | k | v], heads of 128: q/k norm, RoPE, queries to q_out, keys and values to the cache
 };
 
 // Scale staging: per chunk of kChunkKb K blocks the promotion warps pull every
@@ -70,74 +85,161 @@ struct GemmParams {
 // global-memory latency sits between two K blocks.
 template <int BN>
 struct ScaleStage {
-  static constexpr int kChunkKb = 4096 / BN > 32 ? 32 : 4096 / BN;
+  static constexpr int kChunkKb = 32;
   static constexpr int kFloats = kChunkKb * BN;  // one a_scale * w_scale product per (K block, token)
 };
 
-constexpr int kNarrowEpiWarps = 4;  // promotion warps of fp8_gemm_kernel (one per TMEM lane quadrant)
-constexpr int kNarrowThreads = (kNarrowEpiWarps + 3) * 32;
+// Promotion warps of fp8_gemm_kernel: one per TMEM lane quadrant, and from 64 tokens two, which share the columns.
+template <int BN>
+constexpr int kNarrowEpiWarps = BN >= 64 ? 8 : 4;
+template <int BN>
+constexpr int kNarrowThreads = (kNarrowEpiWarps<BN> + 3) * 32;
 
 template <int BN>
 struct GemmSmem {
   static constexpr int kStageBytes = kTileR * kBlockK + BN * kBlockK;
   static constexpr int kScaleBytes = ScaleStage<BN>::kFloats * 4;
   // Narrow column tiles (few tokens) use few registers: two CTAs share an SM, which halves the cost of a
-  // partial last wave and doubles the TMA requests in flight per SM.
+  // partial last wave and doubles the TMA requests in flight per SM.  (At 64 columns two CTAs of four stages each
+  // measured 6144 x 2560 10.3 us against 9.3 and 19456 x 2560 20.7 against the wide kernel's 18.2.)
   static constexpr int kCtasPerSm = BN <= 32 ? 2 : 1;
-  static constexpr int kBudget = (kCtasPerSm == 2 ? 100 : 200) * 1024 - kScaleBytes;
+  static constexpr int kBudget = (kCtasPerSm == 2 ? 108 : 200) * 1024 - kScaleBytes;
   static constexpr int kStages = (kBudget / kStageBytes) > 12 ? 12 : (kBudget / kStageBytes);
   // Accumulator ring in TMEM: up to 8 BN-column buffers, so the MMA issuers can run several K blocks ahead of the
   // promotion, but not more buffers than stages (see done_bar).
   static constexpr int kAccMax = (512 / kCtasPerSm) / BN < kStages ? (512 / kCtasPerSm) / BN : kStages;
   static constexpr int kAcc = kAccMax >= 8 ? 8 : kAccMax >= 4 ? 4 : 2;
   static constexpr int kBarBytes = (2 * kStages + 8) * 8;
-  static constexpr int kTotal = kStages * kStageBytes + kBarBytes + kScaleBytes + 64 + 1024;
+  static constexpr int kPlaceBytes = BN * 16;  // Finish::kQkv: position and page of the tokens
+  static constexpr int kTotal = kStages * kStageBytes + kBarBytes + kScaleBytes + kPlaceBytes + 64 + 1024;
+  static_assert(kTotal <= (kCtasPerSm == 2 ? 113 : 226) * 1024, "shared memory of an SM");
+  static_assert(kStages * kStageBytes >= BN * kTileR * 4, "the stage ring also parks the fp32 rows");
 };
 
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Largest split * ceil(chunks / split) over the allowed split factors (1..8).
-constexpr int max_reduction_chunks(int chunks) {
-  int worst = chunks;
-  for (int split = 2; split <= 8; ++split) {
-    const int used = split * ((chunks + split - 1) / split);
-    if (used > worst) worst = used;
-  }
-  return worst;
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_addr, uint32_t rank) {
+  uint32_t remote;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(remote)
+               : "memory");
+  return v;
 }
 
-__device__ __forceinline__ void store_out(const GemmParams& p, long long token, int col, float v) {
-  if (p.out_f16)
-    reinterpret_cast<__half*>(p.y)[token * p.ldy + col] = __float2half_rn(v);
-  else
-    reinterpret_cast<__nv_bfloat16*>(p.y)[token * p.ldy + col] = __float2bfloat16_rn(v);
+// Four outputs of a token from weight row n0 of the narrow kernel.
+__device__ __forceinline__ void store_row4(const GemmParams& p, int tok, int n0, const float (&v)[4], bool vec) {
+  uint16_t* dst = reinterpret_cast<uint16_t*>(p.y) + (long long)tok * p.ldy + n0;
+  if (vec && n0 + 4 <= p.n) {
+    uint2 w;
+    w.x = p.out_f16 ? Mma16816<__half>::pack(v[0], v[1]) : Mma16816<__nv_bfloat16>::pack(v[0], v[1]);
+    w.y = p.out_f16 ? Mma16816<__half>::pack(v[2], v[3]) : Mma16816<__nv_bfloat16>::pack(v[2], v[3]);
+    *reinterpret_cast<uint2*>(dst) = w;
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (n0 + j >= p.n) break;
+    if (p.out_f16)
+      reinterpret_cast<__half*>(dst)[j] = __float2half_rn(v[j]);
+    else
+      reinterpret_cast<__nv_bfloat16*>(dst)[j] = __float2bfloat16_rn(v[j]);
+  }
+}
+
+// The end of the narrow kernel.  Every CTA of the cluster has parked its fp32 sums as [token][128 weight rows]; CTA
+// `rank` finishes its share of the live tokens.  A warp takes a token, a lane four weight rows (16-byte
+// distributed-shared-memory loads, the rows of several tokens from all CTAs in flight together) and adds the kSplit
+// parts of K in part order, so that results do not depend on timing.
+template <int BN, Finish kFinish, int kSplit>
+__device__ __forceinline__ void finish_rows(const GemmParams& p, const QkvParams& qkv, const longlong2* place,
+                                            uint32_t park, int rank, int tile, int tok0, int warp, int lane) {
+  constexpr int kPeers = kFinish == Finish::kSilu ? 2 * kSplit : kSplit;  // gate parts have even ranks, up parts odd ones
+  constexpr int kBatch = kPeers >= 8 ? 1 : kPeers >= 4 ? 2 : 4;
+  constexpr int kWarps = kNarrowEpiWarps<BN>;
+  const int live = p.m - tok0 < BN ? p.m - tok0 : BN;
+  const int slice = (live + kPeers - 1) / kPeers;
+  const int lo = rank * slice, hi = lo + slice < live ? lo + slice : live;
+  const bool vec = p.ldy % 4 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
+  for (int j0 = lo + warp; j0 < hi; j0 += kWarps * kBatch) {
+    float4 part[kBatch][kPeers];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int j = j0 + u * kWarps < hi ? j0 + u * kWarps : j0;
+#pragma unroll
+      for (int peer = 0; peer < kPeers; ++peer)
+        part[u][peer] = ld_cluster_f4(park + (uint32_t)((j * kTileR + lane * 4) * 4), (uint32_t)peer);
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int j = j0 + u * kWarps, tok = tok0 + j;
+      if (j >= hi) break;
+      auto total = [&](int first, int step, float (&v)[4]) {
+        v[0] = v[1] = v[2] = v[3] = 0.f;
+#pragma unroll
+        for (int peer = first; peer < kPeers; peer += step) {
+          v[0] += part[u][peer].x;
+          v[1] += part[u][peer].y;
+          v[2] += part[u][peer].z;
+          v[3] += part[u][peer].w;
+        }
+      };
+      float v[4];
+      if constexpr (kFinish == Finish::kStore) {
+        total(0, 1, v);
+        store_row4(p, tok, tile * kTileR + lane * 4, v, vec);
+      } else if constexpr (kFinish == Finish::kQkv) {
+        total(0, 1, v);
+        qkv_row_warp(qkv, tok, tile, lane, pack4(v), place[j].x, place[j].y);
+      } else {
+        // The rounding points of the unfused chain: gate and up to bf16, SiLU to bf16, their product to bf16.
+        float up[4];
+        total(0, 2, v);
+        total(1, 2, up);
+        uint2 raw;
+        const uint2 up2 = pack4(up);
+        __nv_bfloat162* r2 = reinterpret_cast<__nv_bfloat162*>(&raw);
+        const __nv_bfloat162* u2 = reinterpret_cast<const __nv_bfloat162*>(&up2);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          r2[i] = __hmul2(__floats2bfloat162_rn(gate_sigmoid(round_bf16(v[2 * i])),
+                                                gate_sigmoid(round_bf16(v[2 * i + 1]))),
+                          u2[i]);
+        unpack4(raw, v);
+        const float amax = warp_max(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
+        const float scale = __fdiv_rn(amax, 448.0f);
+        uint32_t packed[1];
+        quantize_values(v, fmaxf(scale, 1e-12f), packed);
+        *reinterpret_cast<uint32_t*>(p.q + (long long)tok * p.ldq + tile * kTileR + lane * 4) = packed[0];
+        if (lane == 0) p.q_scales[(long long)tile * p.q_scale_ld + tok] = scale;
+      }
+    }
+  }
 }
 
 // Up to 128 tokens.  The 128 UMMA rows are weight rows (one 128-row scale block per tile), the BN columns
-// are tokens.  Warps 0..3 promote, warp 4 is the TMA producer, warps 5 and 6 issue the MMAs of alternate K blocks (one
+// are tokens.  Warps 0..E-1 promote, warp E is the TMA producer, warps E + 1 and E + 2 issue the MMAs of alternate K blocks (one
 // thread's wait, four MMAs and commit take about 770 cycles whatever BN is, and with a second commit per block 900:
-// longer than the block's weights take from HBM) and warp 5 owns TMEM.  A K block has one commit, on the barrier that
+// longer than the block's weights take from HBM) and the first of them owns TMEM.  A K block has one commit, on the barrier that
 // both frees its stage and hands its accumulator to the promotion.
-// grid = (tiles, split), cluster = (1, split, 1): CTA `rank` of a cluster takes the rank-th part of K.
-template <int BN>
-__global__ void __launch_bounds__(kNarrowThreads, (BN <= 32 ? 2 : 1))
+// grid = (tiles, split), cluster = (1, split, 1): CTA `rank` of a cluster takes the rank-th part of K.  Finish::kSilu: a
+// cluster has a CTA for the gate rows and one for the up rows of every part of K (ranks 2 part and 2 part + 1).
+template <int BN, Finish kFinish>
+__global__ void __launch_bounds__(kNarrowThreads<BN>, GemmSmem<BN>::kCtasPerSm)
     fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                    const GemmParams p) {
+                    const __grid_constant__ GemmParams p, const __grid_constant__ QkvParams qkv) {
   using S = GemmSmem<BN>;
   using SS = ScaleStage<BN>;
-  constexpr int E = kNarrowEpiWarps;
+  constexpr int E = kNarrowEpiWarps<BN>, kCols = BN * 4 / E;  // columns of a promotion warp
   constexpr int kStages = S::kStages;
   constexpr int kAcc = S::kAcc;
   constexpr uint32_t kTmemCols = kAcc * BN < 32 ? 32 : kAcc * BN;
   static_assert((kTmemCols & (kTmemCols - 1)) == 0 && kTmemCols <= 512, "TMEM columns must be a power of two <= 512");
   static_assert(BN % 16 == 0, "token tile must be a multiple of 16");
-  // The stage ring doubles as the landing zone of the cluster reduction: split slots of ceil(BN/8/split)
-  // 8-column chunks each, at most (BN/8 + 7) chunks in total.
-  static_assert(kStages * S::kStageBytes >= max_reduction_chunks(BN / 8) * 8 * kTileR * 4,
-                "stage ring too small for the reduction");
-
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* stage_base = smem;
@@ -147,15 +249,18 @@ __global__ void __launch_bounds__(kNarrowThreads, (BN <= 32 ? 2 : 1))
   uint64_t* done_bar = full_bar + kStages;
   uint64_t* tmem_empty = done_bar + kStages;
   float* sscale = reinterpret_cast<float*>(tmem_empty + 8);  // staged scale products of the current K chunk
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sscale + SS::kFloats);
+  longlong2* place = reinterpret_cast<longlong2*>(sscale + SS::kFloats);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(place + BN);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kb_total = (p.k + kBlockK - 1) / kBlockK;
-  const int tiles_w = (p.n + kTileR - 1) / kTileR;
-  const int split = gridDim.y, rank = blockIdx.y, tile = blockIdx.x;
-  const int tw = tile % tiles_w, tt = tile / tiles_w;  // weight-row tile, token tile
-  const int kb_first = (int)((long long)kb_total * rank / split);
-  const int kb_last = (int)((long long)kb_total * (rank + 1) / split);  // exclusive
+  constexpr bool kPairs = kFinish == Finish::kSilu;
+  const int tiles_n = (p.n + kTileR - 1) / kTileR / (kPairs ? 2 : 1);  // output tiles over the weight rows
+  const int split = gridDim.y / (kPairs ? 2 : 1), rank = blockIdx.y, part = rank / (kPairs ? 2 : 1);
+  const int tn = (int)blockIdx.x % tiles_n, tt = (int)blockIdx.x / tiles_n;  // output tile, token tile
+  const int tw = kPairs && (rank & 1) ? tiles_n + tn : tn;                   // weight-row tile
+  const int kb_first = (int)((long long)kb_total * part / split);
+  const int kb_last = (int)((long long)kb_total * (part + 1) / split);  // exclusive
 
   // Everything up to the launch-chain wait overlaps the kernels queued before this one.  So does the weight half of
   // the first stages (the caller promises that those kernels do not write the weights): the producer requests it
@@ -191,10 +296,10 @@ __global__ void __launch_bounds__(kNarrowThreads, (BN <= 32 ? 2 : 1))
   chain_release();
   chain_wait();
 
-  // Promotion state that outlives the role branch (the reduction below needs it).
+  // Promotion state that outlives the role branch (the parked rows below need it).
   constexpr int kEpiThreads = E * 32;
-  const int row_in_tile = (warp & 3) * 32 + lane;
-  float acc[BN];
+  const int row_in_tile = (warp & 3) * 32 + lane, col0 = E == 4 ? 0 : (warp >> 2) * kCols;
+  float acc[kCols];
 
   if (warp == E) {
     // ---------------- TMA producer ----------------
@@ -243,12 +348,20 @@ __global__ void __launch_bounds__(kNarrowThreads, (BN <= 32 ? 2 : 1))
     }
   } else {
     // ---------------- Promotion warps: add every K block with its scales ----------------
-    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col0;
     const int epi_tid = threadIdx.x;  // promotion warps are warps 0..E-1
+    if constexpr (kFinish == Finish::kQkv) {
+      // The tokens' positions and pages, while the operands are on their way; the first output tile's CTA reports.
+      if (epi_tid < BN && tt * BN + epi_tid < p.m) {
+        long long pos, page;
+        qkv_place(qkv, tt * BN + epi_tid, tn == 0 && rank == 0, pos, page);
+        place[epi_tid] = make_longlong2(pos, page);
+      }
+    }
     uint32_t n = 0;
     bool ok = true;
 #pragma unroll
-    for (int j = 0; j < BN; ++j) acc[j] = 0.f;
+    for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
     for (int kb0 = kb_first; kb0 < kb_last && ok; kb0 += SS::kChunkKb) {
       const int kc = kb_last - kb0 < SS::kChunkKb ? kb_last - kb0 : SS::kChunkKb;
       // Stage this chunk's scale products a_scale[token] * w_scale (all loads in flight together).
@@ -261,7 +374,7 @@ __global__ void __launch_bounds__(kNarrowThreads, (BN <= 32 ? 2 : 1))
       epi_bar_sync(kEpiThreads);
       for (int kk = 0; kk < kc; ++kk, ++n) {
         const int b = n % kAcc;
-        const float* s_col = sscale + kk * BN;
+        const float* s_col = sscale + kk * BN + col0;
         if (!mbar_wait_bounded(&done_bar[n % kStages], (n / kStages) & 1u)) {
           raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
           ok = false;
@@ -269,10 +382,10 @@ __global__ void __launch_bounds__(kNarrowThreads, (BN <= 32 ? 2 : 1))
         }
         tc_fence_after();
         const uint32_t taddr = lane_addr + (uint32_t)(b * BN);
-        if constexpr (BN % 64 == 0) {
-          // Two loads in flight per wait: halves the TMEM round trips per K block.
+        if constexpr (kCols % 64 == 0) {
+          // Two loads in flight per wait.
 #pragma unroll
-          for (int c = 0; c < BN; c += 64) {
+          for (int c = 0; c < kCols; c += 64) {
             float d0[32], d1[32];
             tmem_ld32(taddr + c, d0);
             tmem_ld32(taddr + c + 32, d1);
@@ -282,7 +395,7 @@ __global__ void __launch_bounds__(kNarrowThreads, (BN <= 32 ? 2 : 1))
 #pragma unroll
             for (int j = 0; j < 32; ++j) acc[c + 32 + j] = fmaf(d1[j], s_col[c + 32 + j], acc[c + 32 + j]);
           }
-        } else if constexpr (BN % 32 == 0) {
+        } else if constexpr (kCols % 32 == 0) {
           float d[32];
           tmem_ld32(taddr, d);
           tmem_ld_wait();
@@ -302,61 +415,31 @@ __global__ void __launch_bounds__(kNarrowThreads, (BN <= 32 ? 2 : 1))
     }
   }
 
-  // ---------------- output: direct (split == 1) or reduced across the cluster ----------------
-  const int w_row = tw * kTileR + row_in_tile;  // weight row = output column
-  if (split == 1) {
-    if (warp < E && w_row < p.n) {
+  // ---------------- output ----------------
+  // Every MMA of this CTA has completed (the promotion consumed the last accumulator), so the stage ring is free and
+  // parks the rows.
+  const uint32_t park = smem_u32(stage_base);
+  if (warp < E) {
 #pragma unroll
-      for (int j = 0; j < BN; ++j) {
-        const int tok = tt * BN + j;
-        if (tok < p.m) store_out(p, tok, w_row, acc[j]);
-      }
-    }
-  } else {
-    // Every MMA of this CTA has completed (the promotion consumed the last accumulator), so the stage ring
-    // is free.  Rank d owns the 8-token chunks [d * slice, (d + 1) * slice) of the tile: every CTA pushes
-    // its partial of those tokens into slot [its own rank] of the owner's ring (remote shared-memory
-    // stores), the cluster barrier publishes them, and the owner adds the slots in rank order.
-    constexpr int kChunks = BN / 8;
-    const int slice = (kChunks + split - 1) / split;            // chunks per owner
-    const int slice_floats = slice * 8 * kTileR;                 // one slot
-    const uint32_t red_addr = smem_u32(stage_base);
-    cluster_sync_all();  // every CTA of the cluster is done with its own stage ring
-    if (warp < E) {
-#pragma unroll
-      for (int j = 0; j < BN; ++j) {
-        const int owner = (j >> 3) / slice;
-        const int local_col = j - owner * slice * 8;
-        const uint32_t local = red_addr + (uint32_t)((rank * slice_floats + local_col * kTileR + row_in_tile) * 4);
-        uint32_t remote;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"((uint32_t)owner));
-        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(acc[j]) : "memory");
-      }
-    }
-    cluster_sync_all();
-    if (warp < E) {
-      const float* red = reinterpret_cast<const float*>(stage_base);
-      const int chunk_lo = rank * slice, chunk_hi = (rank + 1) * slice < kChunks ? (rank + 1) * slice : kChunks;
-      for (int ch = chunk_lo; ch < chunk_hi; ++ch) {
-        float sum[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) sum[j] = 0.f;
-        for (int peer = 0; peer < split; ++peer) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            sum[j] += red[peer * slice_floats + ((ch - chunk_lo) * 8 + j) * kTileR + row_in_tile];
-        }
-        if (w_row < p.n) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int tok = tt * BN + ch * 8 + j;
-            if (tok < p.m) store_out(p, tok, w_row, sum[j]);
-          }
-        }
-      }
-    }
-    // No CTA reads a peer after the barrier above, so nothing more is needed before exit.
+    for (int j = 0; j < kCols; ++j)
+      asm volatile("st.shared.f32 [%0], %1;" ::"r"(park + (uint32_t)(((col0 + j) * kTileR + row_in_tile) * 4)),
+                   "f"(acc[j])
+                   : "memory");
   }
+  __syncwarp();
+  cluster_sync_all();
+  if (warp < E) {
+    if (split == 1)
+      finish_rows<BN, kFinish, 1>(p, qkv, place, park, rank, tn, tt * BN, warp, lane);
+    else if (split == 2)
+      finish_rows<BN, kFinish, 2>(p, qkv, place, park, rank, tn, tt * BN, warp, lane);
+    else if (split == 4)
+      finish_rows<BN, kFinish, 4>(p, qkv, place, park, rank, tn, tt * BN, warp, lane);
+    else if constexpr (!kPairs)
+      finish_rows<BN, kFinish, 8>(p, qkv, place, park, rank, tn, tt * BN, warp, lane);
+  }
+  __syncwarp();
+  if (gridDim.y > 1) cluster_sync_all();  // no CTA leaves while a peer may still read its rows
 
   tc_fence_before();
   __syncthreads();
@@ -416,17 +499,6 @@ __device__ __forceinline__ bool wide_item(int first, int tiles, int tiles_m, int
   it.k0 = (int)((long long)kb_total * rank / split);
   it.k1 = (int)((long long)kb_total * (rank + 1) / split);
   return true;
-}
-
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_addr, uint32_t rank) {
-  uint32_t remote;
-  float4 v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(remote)
-               : "memory");
-  return v;
 }
 
 __device__ __forceinline__ void tmem_ld_wait_pin(float (&a)[32]) {
@@ -882,11 +954,10 @@ int operand_map(const void* ptr, long long rows, long long k, long long ld, int 
 // (which grows with the tile width).  Cluster sizes 1, 2 and 4 are used, and 8 for the narrow tiles that
 // run two 100 KB CTAs per SM (o / down at up to 32 tokens: 160 CTAs instead of 80); 3 and 8 co-schedule
 // badly with one 200 KB CTA per SM (measured), and larger splits leave too little work per CTA.
-int choose_split(long long tiles, int kb_total, int bn, int ctas_per_sm, int max_split) {
+int choose_split(long long tiles, int kb_total, int bn, int ctas_per_sm, int max_split, int limit) {
   const int slots = sm_count() * ctas_per_sm;
   int best = 1;
   double best_cost = 1e30;
-  const int limit = ctas_per_sm == 2 ? 8 : 4;
   for (int s = 1; s <= limit; s *= 2) {
     if (s > kb_total || (max_split > 0 && s > max_split)) break;
     const long long ctas = tiles * s;
@@ -900,21 +971,26 @@ int choose_split(long long tiles, int kb_total, int bn, int ctas_per_sm, int max
   return best;
 }
 
-template <int BN>
-int launch_gemm(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p, long long tiles, int split,
-                cudaStream_t stream) {
+template <int BN, Finish kFinish>
+int launch_narrow_tiles(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p, const QkvParams& qkv,
+                        int max_split, cudaStream_t stream) {
   using S = GemmSmem<BN>;
   static bool configured[64] = {false};
   int dev = 0;
   MIE_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    MIE_CUDA(cudaFuncSetAttribute(fp8_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    MIE_CUDA(cudaFuncSetAttribute(fp8_gemm_kernel<BN, kFinish>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   S::kTotal));
     configured[dev] = true;
   }
+  constexpr int kPair = kFinish == Finish::kSilu ? 2 : 1;
+  const long long tiles = (long long)((p.n + kTileR - 1) / kTileR) * ((p.m + BN - 1) / BN);
+  MIE_CHECK_ARG(tiles <= 0x7fffffff, "too many output tiles (%lld)", tiles);
+  const int kb = (p.k + kBlockK - 1) / kBlockK;
+  const int split = choose_split(tiles, kb, BN, S::kCtasPerSm, max_split, (S::kCtasPerSm == 2 ? 8 : 4) / kPair);
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3((unsigned)tiles, (unsigned)split, 1);
-  config.blockDim = dim3(kNarrowThreads, 1, 1);
+  config.gridDim = dim3((unsigned)(tiles / kPair), (unsigned)(split * kPair), 1);
+  config.blockDim = dim3(kNarrowThreads<BN>, 1, 1);
   config.dynamicSmemBytes = S::kTotal;
   config.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -922,17 +998,39 @@ int launch_gemm(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = (unsigned)split;
+  attr[0].val.clusterDim.y = (unsigned)(split * kPair);
   attr[0].val.clusterDim.z = 1;
   config.attrs = attr;
   config.numAttrs = chained_launch_enabled() ? 2 : 1;
-  MIE_CUDA(cudaLaunchKernelEx(&config, fp8_gemm_kernel<BN>, mw, mx, p));
+  MIE_CUDA(cudaLaunchKernelEx(&config, fp8_gemm_kernel<BN, kFinish>, mw, mx, p, qkv));
   MIE_LAUNCH_CHECK("fp8_gemm_kernel");
   return MIE_OK;
 }
 
 // Column-tile width for the swapped orientation: smallest of 16/32/64/128 covering m.
 int swap_bn(int m) { return m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128; }
+
+template <Finish kFinish>
+int launch_narrow(const void* x8, long long ldx, const void* w8, long long ldw, const GemmParams& p,
+                  const QkvParams& qkv, int max_split, cudaStream_t stream) {
+  const int bn = swap_bn(p.m);
+  CUtensorMap mw, mx;
+  if (int rc = operand_map(w8, p.n, p.k, ldw, kTileR, &mw)) return rc;
+  if (int rc = operand_map(x8, p.m, p.k, ldx, bn, &mx)) return rc;
+  switch (bn) {
+    case 16: return launch_narrow_tiles<16, kFinish>(mw, mx, p, qkv, max_split, stream);
+    case 32: return launch_narrow_tiles<32, kFinish>(mw, mx, p, qkv, max_split, stream);
+    case 64: return launch_narrow_tiles<64, kFinish>(mw, mx, p, qkv, max_split, stream);
+    default: return launch_narrow_tiles<128, kFinish>(mw, mx, p, qkv, max_split, stream);
+  }
+}
+
+// Whether m tokens of an n-row weight take the narrow kernel: up to 128 tokens, unless that needs a second wave (more
+// 128-row weight tiles than SMs at more than 32 tokens, where only one of its CTAs fits an SM: gate_up): the wide
+// kernel's 256-row tiles then finish in one round.
+bool narrow_fits(int m, int n) {
+  return m <= 32 || (m <= 128 && (n + kTileR - 1) / kTileR <= sm_count());
+}
 
 // Schedule of the wide kernel.  `tiles` output tiles of `kb` K blocks on P SMs (one 200 KB CTA each):
 //   tiles <= P      one launch; whole tiles, or one tile per 2-/4-CTA cluster with the K range cut when all
@@ -1047,32 +1145,21 @@ extern "C" int mie_fp8_quantize(const void* x, int64_t ldx, int32_t dtype, void*
   return launch_quantize<__half>(x, ldx, q, ldq, scales, scale_ld, m, k, (cudaStream_t)stream);
 }
 
-extern "C" int mie_fp8_gemm(const void* x8, int64_t ldx, const float* a_scale, int32_t a_scale_ld, const void* w8,
-                            int64_t ldw, const float* w_scale, int32_t w_scale_ld, void* y, int64_t ldy,
-                            int32_t out_dtype, int32_t m, int32_t n, int32_t k, int32_t max_split, int32_t flags,
-                            int32_t* status, void* stream_) {
-  cudaStream_t stream = (cudaStream_t)stream_;
-  MIE_CHECK_ARG(x8 && a_scale && w8 && w_scale && y, "null pointer");
+namespace mie {
+namespace {
+
+// Argument checks and parameters that the GEMM entry points share.
+int gemm_params(GemmParams& p, const void* x8, int64_t ldx, const float* a_scale, int32_t a_scale_ld, const void* w8,
+                int64_t ldw, const float* w_scale, int32_t w_scale_ld, int32_t m, int32_t n, int32_t k, int32_t flags,
+                int32_t* status) {
+  MIE_CHECK_ARG(x8 && a_scale && w8 && w_scale, "null pointer");
   MIE_CHECK_ARG(m >= 0 && n >= 1 && k >= 1, "invalid GEMM shape %d x %d x %d", m, n, k);
-  MIE_CHECK_ARG(out_dtype == MIE_DTYPE_BF16 || out_dtype == MIE_DTYPE_F16, "output must be bf16 or fp16");
   MIE_CHECK_ARG(ldx % 16 == 0 && ldw % 16 == 0, "operand row strides must be multiples of 16 bytes");
   MIE_CHECK_ARG(((reinterpret_cast<uintptr_t>(x8) | reinterpret_cast<uintptr_t>(w8)) & 15) == 0,
                 "operands must be 16-byte aligned");
-  MIE_CHECK_ARG(ldy >= n && a_scale_ld >= m && w_scale_ld >= (k + 127) / 128, "invalid leading dimension");
+  MIE_CHECK_ARG(a_scale_ld >= m && w_scale_ld >= (k + 127) / 128, "invalid leading dimension");
   MIE_CHECK_ARG((flags & ~(MIE_GEMM_NO_WEIGHT_PREFETCH)) == 0, "unknown flag bits %d", flags);
-  if (m == 0) return MIE_OK;
-
-  // Up to 128 tokens stream the weights through the narrow kernel, unless that needs a second wave of
-  // full-K tiles (more 128-row weight tiles than SMs at more than 32 tokens, where only one of its CTAs
-  // fits an SM: gate_up): the wide kernel's 256-row tiles then finish in one round.  Between 129 and 256
-  // tokens a weight of at most 12 row tiles (N <= 1536: the merged qkv of a 4- or 8-way head shard) is
-  // still faster there, as two token tiles (measured 9.7 vs 12.6 us at N = 768, 10.8 vs 13.1 at N = 1536;
-  // at N = 2560 the wide kernel wins).
-  const int tiles_w = (n + kTileR - 1) / kTileR;
-  const bool narrow = (m <= 128 && !(m > 32 && tiles_w > sm_count())) || (m <= 256 && tiles_w <= 12);
-  const int kb = (k + kBlockK - 1) / kBlockK;
-
-  GemmParams p;
+  p = GemmParams{};
   p.m = m;
   p.n = n;
   p.k = k;
@@ -1080,33 +1167,91 @@ extern "C" int mie_fp8_gemm(const void* x8, int64_t ldx, const float* a_scale, i
   p.a_scale_ld = a_scale_ld;
   p.w_scale = w_scale;
   p.w_scale_ld = w_scale_ld;
-  p.y = y;
-  p.ldy = ldy;
-  p.out_f16 = out_dtype == MIE_DTYPE_F16;
   p.status = status;
   static const int prefetch = [] {
     const char* v = getenv("MIE_GEMM_PREFETCH");
     return v != nullptr && v[0] == '0' ? 0 : 1;  // MIE_GEMM_PREFETCH=0 turns it off
   }();
   p.prefetch = prefetch && !(flags & MIE_GEMM_NO_WEIGHT_PREFETCH);
-  p.tile_begin = p.tile_end = p.late_wait = p.early_release = 0;
+  return MIE_OK;
+}
 
+}  // namespace
+}  // namespace mie
+
+extern "C" int mie_fp8_gemm(const void* x8, int64_t ldx, const float* a_scale, int32_t a_scale_ld, const void* w8,
+                            int64_t ldw, const float* w_scale, int32_t w_scale_ld, void* y, int64_t ldy,
+                            int32_t out_dtype, int32_t m, int32_t n, int32_t k, int32_t max_split, int32_t flags,
+                            int32_t* status, void* stream_) {
+  cudaStream_t stream = (cudaStream_t)stream_;
+  GemmParams p;
+  if (int rc = gemm_params(p, x8, ldx, a_scale, a_scale_ld, w8, ldw, w_scale, w_scale_ld, m, n, k, flags, status))
+    return rc;
+  MIE_CHECK_ARG(y, "null pointer");
+  MIE_CHECK_ARG(out_dtype == MIE_DTYPE_BF16 || out_dtype == MIE_DTYPE_F16, "output must be bf16 or fp16");
+  MIE_CHECK_ARG(ldy >= n, "invalid leading dimension");
+  if (m == 0) return MIE_OK;
+  p.y = y;
+  p.ldy = ldy;
+  p.out_f16 = out_dtype == MIE_DTYPE_F16;
+
+  // Between 129 and 256 tokens a weight of at most 12 row tiles (N <= 1536: the merged qkv of a 4- or 8-way head shard)
+  // is still faster in the narrow kernel, as two token tiles (measured 9.7 vs 12.6 us at N = 768, 10.8 vs 13.1 at
+  // N = 1536; at N = 2560 the wide kernel wins).
+  if (narrow_fits(m, n) || (m <= 256 && (n + kTileR - 1) / kTileR <= 12))
+    return launch_narrow<Finish::kStore>(x8, ldx, w8, ldw, p, QkvParams{}, max_split, stream);
   CUtensorMap mw, mx;
-  if (narrow) {
-    const int bn = swap_bn(m);
-    const long long tiles = (long long)((n + kTileR - 1) / kTileR) * ((m + bn - 1) / bn);
-    MIE_CHECK_ARG(tiles <= 0x7fffffff, "too many output tiles (%lld)", tiles);
-    const int split = choose_split(tiles, kb, bn, bn <= 32 ? 2 : 1, max_split);
-    if (int rc = operand_map(w8, n, k, ldw, kTileR, &mw)) return rc;
-    if (int rc = operand_map(x8, m, k, ldx, bn, &mx)) return rc;
-    switch (bn) {
-      case 16: return launch_gemm<16>(mw, mx, p, tiles, split, stream);
-      case 32: return launch_gemm<32>(mw, mx, p, tiles, split, stream);
-      case 64: return launch_gemm<64>(mw, mx, p, tiles, split, stream);
-      default: return launch_gemm<128>(mw, mx, p, tiles, split, stream);
-    }
-  }
   if (int rc = operand_map(x8, m, k, ldx, kTileR, &mx)) return rc;
   if (int rc = operand_map(w8, n, k, ldw, kWideBN, &mw)) return rc;
   return launch_wide(mx, mw, p, max_split, stream);
+}
+
+extern "C" int mie_fp8_gemm_finishes(int32_t m, int32_t n) { return m >= 1 && n >= 1 && narrow_fits(m, n) ? 1 : 0; }
+
+extern "C" int mie_fp8_gemm_silu(const void* x8, int64_t ldx, const float* a_scale, int32_t a_scale_ld, const void* w8,
+                                 int64_t ldw, const float* w_scale, int32_t w_scale_ld, void* q, int64_t ldq,
+                                 float* scales, int32_t scale_ld, int32_t m, int32_t cols, int32_t k,
+                                 int32_t max_split, int32_t flags, int32_t* status, void* stream) {
+  MIE_CHECK_ARG(q && scales, "null pointer");
+  MIE_CHECK_ARG(cols >= 128 && cols % 128 == 0 && cols <= 0x3fffffff, "cols must be a multiple of 128");
+  GemmParams p;
+  if (int rc = gemm_params(p, x8, ldx, a_scale, a_scale_ld, w8, ldw, w_scale, w_scale_ld, m, 2 * cols, k, flags, status))
+    return rc;
+  MIE_CHECK_ARG(scale_ld >= m && ldq >= cols && ldq % 4 == 0 && (reinterpret_cast<uintptr_t>(q) & 3) == 0,
+                "the quantised rows must be 4-byte aligned and have scale storage");
+  if (m == 0) return MIE_OK;
+  MIE_CHECK_ARG(narrow_fits(m, 2 * cols), "%d tokens of %d columns are not finished in the projection", m, cols);
+  p.q = (uint8_t*)q;
+  p.ldq = ldq;
+  p.q_scales = scales;
+  p.q_scale_ld = scale_ld;
+  return launch_narrow<Finish::kSilu>(x8, ldx, w8, ldw, p, QkvParams{}, max_split, (cudaStream_t)stream);
+}
+
+extern "C" int mie_fp8_gemm_qkv(const void* x8, int64_t ldx, const float* a_scale, int32_t a_scale_ld, const void* w8,
+                                int64_t ldw, const float* w_scale, int32_t w_scale_ld, const void* q_weight,
+                                const void* k_weight, const void* cos_sin, int32_t max_pos, mie_index_t positions,
+                                mie_index_t token_to_sequence, mie_index_t block_tables, void* q_out,
+                                mie_view4_t key_blocks, mie_view4_t value_blocks, void* kv_pool,
+                                int64_t page_stride_bytes, float* kv_scales, int32_t m, int32_t k, int32_t q_heads,
+                                int32_t kv_heads, int32_t block_size, int32_t num_blocks, int32_t table_rows,
+                                int32_t table_width, float eps, int32_t max_split, int32_t flags, int32_t* status,
+                                void* stream) {
+  QkvParams qkv;
+  if (int rc = kv_pool != nullptr ? qkv_e4m3_pool(qkv, kv_pool, page_stride_bytes, kv_scales, kv_heads)
+                                  : qkv_bf16_pages(qkv, key_blocks, value_blocks))
+    return rc;
+  MIE_CHECK_ARG(kv_pool == nullptr || block_size == 16, "the e4m3 pool has pages of 16 tokens");
+  if (int rc = qkv_common(qkv, q_weight, k_weight, cos_sin, max_pos, positions, token_to_sequence, block_tables, q_out,
+                          m, q_heads, kv_heads, block_size, num_blocks, table_rows, table_width, eps, status))
+    return rc;
+  const long long heads = (long long)q_heads + 2ll * kv_heads;
+  MIE_CHECK_ARG(heads <= 0xffffff, "too many heads");
+  GemmParams p;
+  if (int rc = gemm_params(p, x8, ldx, a_scale, a_scale_ld, w8, ldw, w_scale, w_scale_ld, m, (int)heads * kTileR, k, flags,
+                           status))
+    return rc;
+  if (m == 0) return MIE_OK;
+  MIE_CHECK_ARG(narrow_fits(m, p.n), "%d tokens of %lld heads are not finished in the projection", m, heads);
+  return launch_narrow<Finish::kQkv>(x8, ldx, w8, ldw, p, qkv, max_split, (cudaStream_t)stream);
 }

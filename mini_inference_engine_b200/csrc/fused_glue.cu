@@ -7,6 +7,7 @@
 // GEMM consumes, which removes the separate quantiser pass.
 #include "common.cuh"
 #include "glue.cuh"
+#include "qkv_rows.cuh"
 
 namespace mie {
 namespace {
@@ -169,30 +170,6 @@ __global__ void rope_kernel(const __nv_bfloat16* x, long long sb, long long sh, 
 // all the heads of its half-warp, whose rows are in flight together.  A warp per (token, head) with 8-byte accesses
 // looked all of that up per head: 12032 tokens of 48 heads 185 us, now 129 us (147 MB in, 147 MB out).
 // ---------------------------------------------------------------------------
-struct QkvParams {
-  const __nv_bfloat16* qkv;  // [tokens][ld]: q heads | k heads | v heads
-  long long ld;
-  const __nv_bfloat16* q_weight;
-  const __nv_bfloat16* k_weight;
-  const __nv_bfloat16* cos_sin;  // [max_pos][2][128]: cos row then sin row
-  int max_pos;
-  IndexView positions;           // [tokens]
-  IndexView token_to_sequence;   // [tokens] or null (token t belongs to sequence t)
-  IndexView tables;              // [sequences][width]
-  __nv_bfloat16* q_out;          // [tokens][q_heads][128]
-  char* key_blocks;
-  char* value_blocks;
-  long long kb_s[3], vb_s[3];    // page, head, token strides (elements)
-  int tokens, q_heads, kv_heads, block_size, num_blocks, table_rows, table_width;
-  float eps;
-  int* status;
-  // e4m3 K/V pool [pages][kv_heads][2][16][128] with scales [pages][kv_heads][2][16] (block_size 16), or null.
-  uint8_t* kv8_pool;
-  long long kv8_page_stride;  // bytes
-  float* kv8_scales;
-  bool wide;  // every row of every tensor is 16-byte aligned, of the e4m3 pool 8-byte (otherwise 8- and 4-byte)
-};
-
 // Eight bf16 values, 16-byte aligned when `wide`, else 8-byte.
 __device__ __forceinline__ uint4 load8(const __nv_bfloat16* p, bool wide) {
   if (wide) return *reinterpret_cast<const uint4*>(p);
@@ -229,23 +206,8 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvParams p) {
     }
   };
   load_batch(h_first);
-  const long long pos = p.positions.at(t);
-  const long long seq = p.token_to_sequence.valid() ? p.token_to_sequence.at(t) : t;
-  const bool reports = threadIdx.x == 0 && blockIdx.y == 0;
-  // Where the token's K / V rows go; -1: nowhere.
-  long long page = -1;
-  if (seq < 0 || seq >= p.table_rows) {
-    if (reports) raise_status(p.status, MIE_STATUS_BAD_SEQUENCE);
-  } else if (pos < 0 || pos >= (long long)p.table_width * p.block_size) {
-    if (reports) raise_status(p.status, MIE_STATUS_BAD_POSITION);
-  } else {
-    page = p.tables.at(seq, pos / p.block_size);
-    if (page < 0 || page >= p.num_blocks) {
-      if (reports) raise_status(p.status, MIE_STATUS_BAD_PAGE);
-      page = -1;
-    }
-  }
-  if (reports && (pos < 0 || pos >= p.max_pos)) raise_status(p.status, MIE_STATUS_BAD_POSITION);
+  long long pos, page;
+  qkv_place(p, t, threadIdx.x == 0 && blockIdx.y == 0, pos, page);
   const long long cpos = pos < 0 ? 0 : (pos >= p.max_pos ? p.max_pos - 1 : pos);
   const __nv_bfloat16* cs = p.cos_sin + cpos * 256 + l16 * 8;
   float c[8], s[8];
@@ -310,8 +272,6 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvParams p) {
     }
   }
 }
-
-bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace
 }  // namespace mie
@@ -389,42 +349,20 @@ extern "C" int mie_rope(mie_view4_t x, const void* cos, const void* sin, int64_t
 
 namespace {
 
-int launch_qkv_post(mie::QkvParams& p, const void* qkv, int64_t ld, const void* q_weight, const void* k_weight,
-                    const void* cos_sin, int32_t max_pos, const mie_index_t& positions,
-                    const mie_index_t& token_to_sequence, const mie_index_t& block_tables, void* q_out, int32_t tokens,
-                    int32_t q_heads, int32_t kv_heads, int32_t block_size, int32_t num_blocks, int32_t table_rows,
-                    int32_t table_width, float eps, int32_t* status, void* stream) {
-  MIE_CHECK_ARG(qkv && q_weight && k_weight && cos_sin && positions.ptr && block_tables.ptr && q_out, "null pointer");
-  MIE_CHECK_ARG(ld % 4 == 0 && (reinterpret_cast<uintptr_t>(qkv) & 7) == 0, "qkv rows must be 8-byte aligned");
-  MIE_CHECK_ARG(tokens >= 0 && q_heads >= 1 && kv_heads >= 1 && max_pos >= 1, "invalid shape");
+int launch_qkv_post(mie::QkvParams& p, const void* qkv, int64_t ld, int32_t tokens, void* stream) {
+  MIE_CHECK_ARG(qkv != nullptr && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(qkv) & 7) == 0,
+                "qkv rows must be 8-byte aligned");
   if (tokens == 0) return MIE_OK;
   p.qkv = (const __nv_bfloat16*)qkv;
   p.ld = ld;
-  p.q_weight = (const __nv_bfloat16*)q_weight;
-  p.k_weight = (const __nv_bfloat16*)k_weight;
-  p.cos_sin = (const __nv_bfloat16*)cos_sin;
-  p.max_pos = max_pos;
-  p.positions = IndexView(positions);
-  p.token_to_sequence = IndexView(token_to_sequence);
-  p.tables = IndexView(block_tables);
-  p.q_out = (__nv_bfloat16*)q_out;
-  p.tokens = tokens;
-  p.q_heads = q_heads;
-  p.kv_heads = kv_heads;
-  p.block_size = block_size;
-  p.num_blocks = num_blocks;
-  p.table_rows = table_rows;
-  p.table_width = table_width;
-  p.eps = eps;
-  p.status = status;
   auto rows16 = [](const void* ptr, const long long* strides) {
     return aligned16(ptr) && strides[0] % 8 == 0 && strides[1] % 8 == 0 && strides[2] % 8 == 0;
   };
-  p.wide = ld % 8 == 0 && aligned16(qkv) && aligned16(q_weight) && aligned16(k_weight) && aligned16(cos_sin) &&
-           aligned16(q_out) &&
+  p.wide = ld % 8 == 0 && aligned16(qkv) && aligned16(p.q_weight) && aligned16(p.k_weight) && aligned16(p.cos_sin) &&
+           aligned16(p.q_out) &&
            (p.kv8_pool != nullptr ? (reinterpret_cast<uintptr_t>(p.kv8_pool) & 7) == 0 && p.kv8_page_stride % 8 == 0
                                   : rows16(p.key_blocks, p.kb_s) && rows16(p.value_blocks, p.vb_s));
-  const int lanes = ((q_heads + 2 * kv_heads) * 16 + 31) / 32 * 32;
+  const int lanes = ((p.q_heads + 2 * p.kv_heads) * 16 + 31) / 32 * 32;
   const int threads = lanes < 256 ? lanes : 256;
   // Few tokens: several blocks each, so that a half-warp has one head (one token of 48 heads 3 us less).
   const int blocks = tokens <= sm_count() ? (lanes + threads - 1) / threads : 1;
@@ -443,24 +381,12 @@ extern "C" int mie_qkv_norm_rope_write(const void* qkv, int64_t ld, const void* 
                                        int32_t q_heads, int32_t kv_heads, int32_t block_size, int32_t num_blocks,
                                        int32_t table_rows, int32_t table_width, float eps, int32_t* status,
                                        void* stream) {
-  MIE_CHECK_ARG(key_blocks.ptr && value_blocks.ptr, "null pointer");
-  MIE_CHECK_ARG(key_blocks.stride[3] == 1 && value_blocks.stride[3] == 1, "pages must be contiguous in head_dim");
-  for (int i = 0; i < 3; ++i) {
-    MIE_CHECK_ARG(key_blocks.stride[i] % 4 == 0 && value_blocks.stride[i] % 4 == 0, "page strides must be multiples of 4");
-  }
   QkvParams p;
-  p.key_blocks = (char*)key_blocks.ptr;
-  p.value_blocks = (char*)value_blocks.ptr;
-  for (int i = 0; i < 3; ++i) {
-    p.kb_s[i] = key_blocks.stride[i];
-    p.vb_s[i] = value_blocks.stride[i];
-  }
-  p.kv8_pool = nullptr;
-  p.kv8_page_stride = 0;
-  p.kv8_scales = nullptr;
-  return launch_qkv_post(p, qkv, ld, q_weight, k_weight, cos_sin, max_pos, positions, token_to_sequence, block_tables,
-                         q_out, tokens, q_heads, kv_heads, block_size, num_blocks, table_rows, table_width, eps,
-                         status, stream);
+  if (int rc = qkv_bf16_pages(p, key_blocks, value_blocks)) return rc;
+  if (int rc = qkv_common(p, q_weight, k_weight, cos_sin, max_pos, positions, token_to_sequence, block_tables, q_out,
+                          tokens, q_heads, kv_heads, block_size, num_blocks, table_rows, table_width, eps, status))
+    return rc;
+  return launch_qkv_post(p, qkv, ld, tokens, stream);
 }
 
 extern "C" int mie_qkv_norm_rope_write_kv8(const void* qkv, int64_t ld, const void* q_weight, const void* k_weight,
@@ -470,17 +396,10 @@ extern "C" int mie_qkv_norm_rope_write_kv8(const void* qkv, int64_t ld, const vo
                                            int32_t tokens, int32_t q_heads, int32_t kv_heads, int32_t num_blocks,
                                            int32_t table_rows, int32_t table_width, float eps, int32_t* status,
                                            void* stream) {
-  MIE_CHECK_ARG(kv_pool && kv_scales, "null pointer");
-  MIE_CHECK_ARG(page_stride_bytes >= (long long)kv_heads * 4096 && page_stride_bytes % 4 == 0 &&
-                    (reinterpret_cast<uintptr_t>(kv_pool) & 3) == 0,
-                "the e4m3 pool needs a page stride of at least kv_heads * 4096 bytes");
   QkvParams p;
-  p.key_blocks = p.value_blocks = nullptr;
-  for (int i = 0; i < 3; ++i) p.kb_s[i] = p.vb_s[i] = 0;
-  p.kv8_pool = (uint8_t*)kv_pool;
-  p.kv8_page_stride = page_stride_bytes;
-  p.kv8_scales = kv_scales;
-  return launch_qkv_post(p, qkv, ld, q_weight, k_weight, cos_sin, max_pos, positions, token_to_sequence, block_tables,
-                         q_out, tokens, q_heads, kv_heads, /*block_size=*/16, num_blocks, table_rows, table_width, eps,
-                         status, stream);
+  if (int rc = qkv_e4m3_pool(p, kv_pool, page_stride_bytes, kv_scales, kv_heads)) return rc;
+  if (int rc = qkv_common(p, q_weight, k_weight, cos_sin, max_pos, positions, token_to_sequence, block_tables, q_out,
+                          tokens, q_heads, kv_heads, /*block_size=*/16, num_blocks, table_rows, table_width, eps, status))
+    return rc;
+  return launch_qkv_post(p, qkv, ld, tokens, stream);
 }

@@ -22,6 +22,19 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
   return raw;
 }
 
+__device__ __forceinline__ void unpack4(const uint2& raw, float (&v)[4]) {
+  const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  const float2 lo = __bfloat1622float2(p[0]), hi = __bfloat1622float2(p[1]);
+  v[0] = lo.x, v[1] = lo.y, v[2] = hi.x, v[3] = hi.y;
+}
+__device__ __forceinline__ uint2 pack4(const float (&v)[4]) {
+  uint2 raw;
+  __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&raw);
+  p[0] = __floats2bfloat162_rn(v[0], v[1]);
+  p[1] = __floats2bfloat162_rn(v[2], v[3]);
+  return raw;
+}
+
 // a / b from y, an approximation of 1 / b: quotient, its exact remainder, correction.  Correctly rounded when y is the
 // correctly rounded reciprocal (Markstein's theorem), else within a little more than half a unit in the last place.
 // Three instructions where an IEEE division takes about ten.  b and y must be finite.

@@ -384,6 +384,21 @@ class Qwen3DecodeRunner(PagedStepRunner):
                                             inter, _lib.stream_arg(self.device)))
         return q, scales
 
+    def _gated_quantized(self, quantized, layer, rows: int):
+        """The merged gate_up projection and SiLU(gate) * up, quantised for down_proj: one launch for a decode batch."""
+
+        weight, inter = layer.gate_up, self.local_inter
+        if not sm89_fp8.finishes_rows(weight, rows):
+            return self._silu_mul_quantized(self._gemm(quantized, weight, layer.gate_up_scale, rows, self.shape.hidden),
+                                            rows)
+        q, scales = self._quant_buffers(rows, inter)
+        _lib.check(_lib.load().mie_fp8_gemm_silu(
+            _lib.ptr(quantized[0]), quantized[0].stride(0), _lib.ptr(quantized[1]), quantized[1].stride(0),
+            _lib.ptr(weight), weight.stride(0), _lib.ptr(layer.gate_up_scale), layer.gate_up_scale.stride(0), _lib.ptr(q),
+            q.stride(0), _lib.ptr(scales), scales.stride(0), rows, inter, self.shape.hidden,
+            sm89_fp8.default_max_split(), 0, _lib.ptr(self.status), _lib.stream_arg(self.device)))
+        return q, scales
+
     def _row_parallel_then_norm(self, quantized, weight, weight_scale, rows: int, k: int, residual, norm_weight,
                                 *, quantize: bool):
         """Row-parallel projection, sum over the ranks, residual add and RMSNorm of the sum.  Returns
@@ -423,6 +438,32 @@ class Qwen3DecodeRunner(PagedStepRunner):
             shape.page, self.total_pages, table_rows, int(block_tables.shape[1]), shape.rms_eps,
             _lib.ptr(self.status), _lib.stream_arg(self.device)))
 
+    def _project_qkv(self, layer_index: int, layer, quantized, queries, positions, token_to_sequence, block_tables,
+                     tokens: int, table_rows: int) -> None:
+        """The merged q/k/v projection and ``_qkv_post``: one launch for a decode batch."""
+
+        shape, weight = self.shape, layer.qkv
+        if not sm89_fp8.finishes_rows(weight, tokens):
+            qkv = self._gemm(quantized, weight, layer.qkv_scale, tokens, shape.hidden)
+            self._qkv_post(layer_index, layer, qkv, queries, positions, token_to_sequence, block_tables, tokens,
+                           table_rows)
+            return
+        if self.kv8 is not None:
+            none = _lib.view4_arg(None)
+            cache = (none, none, _lib.ptr(self.kv8.data[layer_index]), self.kv8.page_stride_bytes,
+                     _lib.ptr(self.kv8.scales[layer_index]))
+        else:
+            cache = (_lib.view4_arg(self.key_blocks[layer_index]), _lib.view4_arg(self.value_blocks[layer_index]), None,
+                     0, None)
+        _lib.check(_lib.load().mie_fp8_gemm_qkv(
+            _lib.ptr(quantized[0]), quantized[0].stride(0), _lib.ptr(quantized[1]), quantized[1].stride(0),
+            _lib.ptr(weight), weight.stride(0), _lib.ptr(layer.qkv_scale), layer.qkv_scale.stride(0),
+            _lib.ptr(layer.q_norm), _lib.ptr(layer.k_norm), _lib.ptr(self.rope), int(self.rope.shape[0]),
+            _lib.index_arg(positions), _lib.index_arg(token_to_sequence), _lib.index_arg(block_tables),
+            _lib.ptr(queries), *cache, tokens, shape.hidden, self.local_q_heads, self.local_kv_heads, shape.page,
+            self.total_pages, table_rows, int(block_tables.shape[1]), shape.rms_eps, sm89_fp8.default_max_split(), 0,
+            _lib.ptr(self.status), _lib.stream_arg(self.device)))
+
     # -- the decode forward -------------------------------------------------------------------
 
     def decode_forward(self, input_ids: torch.Tensor, sequence_lengths: torch.Tensor,
@@ -441,9 +482,8 @@ class Qwen3DecodeRunner(PagedStepRunner):
         _, _, quantized = self._norm(hidden, layers[0].input_norm, quantize=True)
         residual, final = hidden, None
         for index, layer in enumerate(layers):
-            qkv = self._gemm(quantized, layer.qkv, layer.qkv_scale, batch, shape.hidden)
             queries = torch.empty(batch, lq, 1, hd, dtype=torch.bfloat16, device=self.device)
-            self._qkv_post(index, layer, qkv, queries, positions, None, block_tables, batch, batch)
+            self._project_qkv(index, layer, quantized, queries, positions, None, block_tables, batch, batch)
             attended = torch.empty_like(queries)
             attn_q = self._quant_buffers(batch, lq * hd)
             if self.kv8 is not None:
@@ -460,8 +500,7 @@ class Qwen3DecodeRunner(PagedStepRunner):
                                         quantized_out=attn_q)
             _, residual, quantized = self._row_parallel_then_norm(attn_q, layer.o, layer.o_scale, batch, lq * hd,
                                                                   residual, layer.post_norm, quantize=True)
-            gate_up = self._gemm(quantized, layer.gate_up, layer.gate_up_scale, batch, shape.hidden)
-            act_q = self._silu_mul_quantized(gate_up, batch)
+            act_q = self._gated_quantized(quantized, layer, batch)
             last = index + 1 == len(layers)
             next_norm = self.weights.final_norm if last else layers[index + 1].input_norm
             final, residual, quantized = self._row_parallel_then_norm(act_q, layer.down, layer.down_scale, batch,
@@ -530,10 +569,9 @@ class Qwen3DecodeRunner(PagedStepRunner):
             chunk_tables = torch.where(chunk_tables >= 0, numbering.view_as(chunk_tables),
                                        torch.full_like(chunk_tables, -1))
         for index, layer in enumerate(layers):
-            qkv = self._gemm(quantized, layer.qkv, layer.qkv_scale, tokens, shape.hidden)
             queries = torch.empty(tokens, lq, hd, dtype=torch.bfloat16, device=self.device)
-            self._qkv_post(index, layer, qkv, queries, token_positions, token_to_sequence, block_tables, tokens,
-                           table_rows)
+            self._project_qkv(index, layer, quantized, queries, token_positions, token_to_sequence, block_tables, tokens,
+                              table_rows)
             attended = torch.empty_like(queries)
             if decode_rows and self.kv8 is not None:
                 launch_decode_attention_kv8(queries[:decode_rows].unsqueeze(2), attended[:decode_rows].unsqueeze(2),
@@ -559,8 +597,7 @@ class Qwen3DecodeRunner(PagedStepRunner):
             attn_q = self._quantize(attended.view(tokens, lq * hd))
             _, residual, quantized = self._row_parallel_then_norm(attn_q, layer.o, layer.o_scale, tokens, lq * hd,
                                                                   residual, layer.post_norm, quantize=True)
-            gate_up = self._gemm(quantized, layer.gate_up, layer.gate_up_scale, tokens, shape.hidden)
-            act_q = self._silu_mul_quantized(gate_up, tokens)
+            act_q = self._gated_quantized(quantized, layer, tokens)
             last = index + 1 == len(layers)
             next_norm = self.weights.final_norm if last else layers[index + 1].input_norm
             normed, residual, quantized = self._row_parallel_then_norm(act_q, layer.down, layer.down_scale, tokens,

@@ -1,0 +1,121 @@
+"""Projections that finish their own rows: equal to the projection followed by the row kernel."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from mini_inference_engine_b200 import _lib
+from mini_inference_engine_b200.engine.kernels import sm89_fp8
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(m, n, k, device):
+    generator = torch.Generator(device=device).manual_seed(n + k + m)
+    w8 = (torch.randn(n, k, generator=generator, device=device) * 32).clamp(-448, 448).to(torch.float8_e4m3fn)
+    w_scale = torch.rand(n // 128, -(-k // 128), generator=generator, device=device) * 2e-3 + 1e-4
+    x = torch.randn(m, k, generator=generator, device=device).to(torch.bfloat16)
+    x[0] *= 0.0 if m > 1 else 1.0
+    q, scales = sm89_fp8.quantize_activation_kmajor(x)
+    return q, scales, w8, w_scale
+
+
+def _product(q, scales, w8, w_scale, m, k, max_split):
+    out = torch.empty(m, w8.shape[0], dtype=torch.bfloat16, device=q.device)
+    sm89_fp8.launch_fp8_gemm(q, scales, w8, w_scale, out, m, k, max_split=max_split)
+    return out
+
+
+# Tokens at the edges of the column tiles; a K that is cut in parts, one of a single block, one with a tail.
+SIZES = [(m, k) for m in (1, 15, 16, 17, 32, 33, 64, 65, 128) for k in (128, 1024, 2560)] + [(5, 2032), (40, 9728)]
+
+
+@pytest.mark.parametrize("m,k", SIZES)
+@pytest.mark.parametrize("max_split", [0, 1])
+def test_gated_rows(m, k, max_split, device, status_clean):
+    cols = 384
+    q, scales, w8, w_scale = _operands(m, 2 * cols, k, device)
+    lib, stream = _lib.load(), _lib.stream_arg(device)
+    assert lib.mie_fp8_gemm_finishes(m, 2 * cols)
+    got, got_s = torch.zeros(m, cols, dtype=torch.uint8, device=device), torch.zeros(3, m + 2, device=device)
+    _lib.check(lib.mie_fp8_gemm_silu(
+        _lib.ptr(q), q.stride(0), _lib.ptr(scales), scales.stride(0), _lib.ptr(w8), k, _lib.ptr(w_scale), w_scale.stride(0),
+        _lib.ptr(got), cols, _lib.ptr(got_s), m + 2, m, cols, k, max_split, 0, _lib.ptr(_lib.status_word(device)), stream))
+    both = _product(q, scales, w8, w_scale, m, k, max_split)
+    want, want_s = torch.zeros_like(got), torch.zeros_like(got_s)
+    _lib.check(lib.mie_silu_mul(_lib.ptr(both), _lib.ptr(both[:, cols:]), 2 * cols, None, _lib.ptr(want), cols,
+                                _lib.ptr(want_s), m + 2, m, cols, stream))
+    torch.cuda.synchronize()
+    if max_split == 1:  # the same sums in the same order
+        assert torch.equal(got, want) and torch.equal(got_s, want_s)
+        return
+    # K may be cut elsewhere: fp32 sums in another order, which can move a bf16 rounding (2^-8) and through it an e4m3
+    # one (2^-3 of a value, at most one step).
+    full = got.view(torch.float8_e4m3fn).float() * got_s[:, :m].t().repeat_interleave(128, 1)
+    ref = want.view(torch.float8_e4m3fn).float() * want_s[:, :m].t().repeat_interleave(128, 1)
+    top = want_s[:, :m].t().repeat_interleave(128, 1) * 448
+    assert ((full - ref).abs() <= 0.13 * ref.abs() + 2 ** -8 * top).all()
+    assert ((full - ref).norm() <= 1e-2 * ref.norm()).all()
+
+
+@pytest.mark.parametrize("m,k", SIZES)
+@pytest.mark.parametrize("heads", [(4, 2), (3, 1)])
+@pytest.mark.parametrize("kv8", [False, True])
+def test_cache_rows(m, k, heads, kv8, device, status_clean):
+    from mini_inference_engine_b200.engine.model_runner.qwen3_decode import Qwen3Shape, rope_table
+
+    q_heads, kv_heads = heads
+    n, pages, width = (q_heads + 2 * kv_heads) * 128, m + 3, 2
+    q, scales, w8, w_scale = _operands(m, n, k, device)
+    lib, stream, status = _lib.load(), _lib.stream_arg(device), _lib.status_word(device)
+    norms = [(1 + 0.1 * torch.randn(128, device=device)).to(torch.bfloat16) for _ in range(2)]
+    rope = rope_table(Qwen3Shape(), 64, device)
+    positions = torch.arange(m, dtype=torch.int32, device=device) % 32
+    tables = torch.randperm(pages, device=device)[:m].to(torch.int32)[:, None].repeat(1, width).contiguous()
+    meta = (_lib.ptr(norms[0]), _lib.ptr(norms[1]), _lib.ptr(rope), 64, _lib.index_arg(positions), _lib.index_arg(None),
+            _lib.index_arg(tables))
+    results = []
+    for fused in (True, False):
+        queries = torch.zeros(m, q_heads, 128, dtype=torch.bfloat16, device=device)
+        keys = torch.zeros(pages, kv_heads, 16, 128, dtype=torch.bfloat16, device=device)
+        values, pool = torch.zeros_like(keys), torch.zeros(pages, kv_heads, 2, 16, 128, dtype=torch.uint8, device=device)
+        pool_s = torch.zeros(pages, kv_heads, 2, 16, device=device)
+        views = (_lib.view4_arg(keys), _lib.view4_arg(values))
+        if fused:
+            _lib.check(lib.mie_fp8_gemm_qkv(
+                _lib.ptr(q), q.stride(0), _lib.ptr(scales), scales.stride(0), _lib.ptr(w8), k, _lib.ptr(w_scale),
+                w_scale.stride(0), *meta, _lib.ptr(queries), *views, _lib.ptr(pool) if kv8 else None, kv_heads * 4096,
+                _lib.ptr(pool_s), m, k, q_heads, kv_heads, 16, pages, m, width, 1e-6, 1, 0, _lib.ptr(status), stream))
+        else:
+            rows = _product(q, scales, w8, w_scale, m, k, 1)
+            tail = (m, q_heads, kv_heads)
+            if kv8:
+                _lib.check(lib.mie_qkv_norm_rope_write_kv8(_lib.ptr(rows), n, *meta, _lib.ptr(queries), _lib.ptr(pool),
+                                                           kv_heads * 4096, _lib.ptr(pool_s), *tail, pages, m, width, 1e-6,
+                                                           _lib.ptr(status), stream))
+            else:
+                _lib.check(lib.mie_qkv_norm_rope_write(_lib.ptr(rows), n, *meta, _lib.ptr(queries), *views, *tail, 16,
+                                                       pages, m, width, 1e-6, _lib.ptr(status), stream))
+        results.append((queries, keys, values, pool.view(torch.float8_e4m3fn).float() * pool_s[..., None]))
+    torch.cuda.synchronize()
+    # The projected rows are the same; the sum of squares of a row is added in another order, which can move a bf16
+    # rounding of the norm (2^-8, through the rotation twice that) and of an e4m3 value (2^-3).
+    for index, (got, want) in enumerate(zip(*results)):
+        got, want = got.float(), want.float()
+        limit = 2 ** -6 * want.abs().amax(-1, keepdim=True) + (0.13 * want.abs() if index == 3 else 0.0)
+        assert ((got - want).abs() <= limit).all()
+        assert (got != want).float().mean() < 0.05
+    assert torch.equal(results[0][2], results[1][2])  # values are copied
+
+
+def test_sizes_that_are_not_finished_are_refused(device):
+    q, scales, w8, w_scale = _operands(130, 768, 256, device)
+    out, out_s = torch.zeros(130, 384, dtype=torch.uint8, device=device), torch.zeros(3, 130, device=device)
+    lib = _lib.load()
+    assert not lib.mie_fp8_gemm_finishes(130, 768) and not lib.mie_fp8_gemm_finishes(33, 128 * 400)
+    with pytest.raises(Exception, match="not finished in the projection"):
+        _lib.check(lib.mie_fp8_gemm_silu(
+            _lib.ptr(q), q.stride(0), _lib.ptr(scales), scales.stride(0), _lib.ptr(w8), 256, _lib.ptr(w_scale), 2,
+            _lib.ptr(out), 384, _lib.ptr(out_s), 130, 130, 384, 256, 0, 0, _lib.ptr(_lib.status_word(device)),
+            _lib.stream_arg(device)))
