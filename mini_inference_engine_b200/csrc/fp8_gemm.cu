@@ -329,8 +329,10 @@ __global__ void __launch_bounds__(kNarrowThreads<BN>, GemmSmem<BN>::kCtasPerSm)
       const uint32_t blocks = (uint32_t)(kb_last - kb_first);
       for (uint32_t n = (uint32_t)(warp - (E + 1)); n < blocks; n += 2) {
         const int s = n % kStages, b = n % kAcc;
-        if (!mbar_wait_bounded(&full_bar[s], (n / kStages) & 1u) ||
-            !mbar_wait_bounded(&tmem_empty[b], ((n / kAcc) & 1u) ^ 1u)) {
+        // In this order: the stage's previous block may be the other issuer's, and a released accumulator (of a block no
+        // older, kAcc <= kStages) tells that its barrier phase is over.
+        if (!mbar_wait_bounded(&tmem_empty[b], ((n / kAcc) & 1u) ^ 1u) ||
+            !mbar_wait_bounded(&full_bar[s], (n / kStages) & 1u)) {
           raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
           break;
         }
@@ -683,8 +685,10 @@ __global__ void __launch_bounds__(kWideThreads, 1)
       const int b = warp - (E + 1);
       for (uint32_t n = b; n < total_blocks; n += kAcc) {
         const int s = n % kStages;
-        if (!mbar_wait_bounded(&full_bar[s], (n / kStages) & 1u) ||
-            !mbar_wait_bounded(&tmem_empty[b], ((n / kAcc) & 1u) ^ 1u)) {
+        // In this order: the stage's previous block may be the other issuer's, and a released accumulator (of a block no
+        // older, kAcc <= kStages) tells that its barrier phase is over.
+        if (!mbar_wait_bounded(&tmem_empty[b], ((n / kAcc) & 1u) ^ 1u) ||
+            !mbar_wait_bounded(&full_bar[s], (n / kStages) & 1u)) {
           raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
           break;
         }

@@ -119,3 +119,18 @@ def test_sizes_that_are_not_finished_are_refused(device):
             _lib.ptr(q), q.stride(0), _lib.ptr(scales), scales.stride(0), _lib.ptr(w8), 256, _lib.ptr(w_scale), 2,
             _lib.ptr(out), 384, _lib.ptr(out_s), 130, 130, 384, 256, 0, 0, _lib.ptr(_lib.status_word(device)),
             _lib.stream_arg(device)))
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 2560, 9728), (24, 2560, 9728), (300, 1024, 2560)])
+def test_repeated_products_are_identical(m, n, k, device, status_clean):
+    """Two threads issue alternate K blocks over an odd number of stages: none may take a stage before its block landed,
+    however late the operands come (L2 is flushed in between)."""
+
+    q, scales, w8, w_scale = _operands(m, n, k, device)
+    first = _product(q, scales, w8, w_scale, m, k, 0)
+    flush = torch.empty(160 << 20, dtype=torch.uint8, device=device)
+    different = torch.zeros((), dtype=torch.int64, device=device)
+    for _ in range(200):
+        flush.zero_()
+        different += (_product(q, scales, w8, w_scale, m, k, 0) != first).any()
+    assert int(different.item()) == 0
