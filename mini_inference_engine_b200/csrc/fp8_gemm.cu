@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kNarrowThreads<BN>, GemmSmem<BN>::kCtasPerSm)
   longlong2* place = reinterpret_cast<longlong2*>(sscale + SS::kFloats);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(place + BN);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   const int kb_total = (p.k + kBlockK - 1) / kBlockK;
   constexpr bool kPairs = kFinish == Finish::kSilu;
   const int tiles_n = (p.n + kTileR - 1) / kTileR / (kPairs ? 2 : 1);  // output tiles over the weight rows
@@ -324,19 +324,20 @@ __global__ void __launch_bounds__(kNarrowThreads<BN>, GemmSmem<BN>::kCtasPerSm)
     }
   } else if (warp > E) {
     // ---------------- MMA issuers ----------------
-    if (lane == 0) {
+    {
       constexpr uint32_t idesc = instr_desc_f8(BN);
       const uint32_t blocks = (uint32_t)(kb_last - kb_first);
       for (uint32_t n = (uint32_t)(warp - (E + 1)); n < blocks; n += 2) {
         const int s = n % kStages, b = n % kAcc;
         // In this order: the stage's previous block may be the other issuer's, and a released accumulator (of a block no
         // older, kAcc <= kStages) tells that its barrier phase is over.
-        if (!mbar_wait_bounded(&tmem_empty[b], ((n / kAcc) & 1u) ^ 1u) ||
-            !mbar_wait_bounded(&full_bar[s], (n / kStages) & 1u)) {
+        if (!warp_wait_bounded(&tmem_empty[b], ((n / kAcc) & 1u) ^ 1u) ||
+            !warp_wait_bounded(&full_bar[s], (n / kStages) & 1u)) {
           raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
           break;
         }
         tc_fence_after();
+        if (!elect_one()) continue;
         const uint32_t a_addr = smem_u32(stage_base + (size_t)s * S::kStageBytes);
         const uint32_t b_addr = a_addr + kTileR * kBlockK;
         const uint64_t da = smem_desc_k128(a_addr), db = smem_desc_k128(b_addr);
@@ -599,7 +600,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
   uint64_t* tmem_empty = done_bar + kStages;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + kAcc);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   const int kb_total = (p.k + kBlockK - 1) / kBlockK;
   const int tiles_m = (p.m + kTileR - 1) / kTileR;
   const int tiles = p.tile_end;
@@ -679,7 +680,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
           load_w(s, kb, it);
         }
       }
-    } else if ((warp == E + 1 || warp == E + 2) && lane == 0) {
+    } else if (warp == E + 1 || warp == E + 2) {
       // ---------------- MMA issuers, one per accumulator ----------------
       constexpr uint32_t idesc = instr_desc_f8(BN);
       const int b = warp - (E + 1);
@@ -687,12 +688,13 @@ __global__ void __launch_bounds__(kWideThreads, 1)
         const int s = n % kStages;
         // In this order: the stage's previous block may be the other issuer's, and a released accumulator (of a block no
         // older, kAcc <= kStages) tells that its barrier phase is over.
-        if (!mbar_wait_bounded(&tmem_empty[b], ((n / kAcc) & 1u) ^ 1u) ||
-            !mbar_wait_bounded(&full_bar[s], (n / kStages) & 1u)) {
+        if (!warp_wait_bounded(&tmem_empty[b], ((n / kAcc) & 1u) ^ 1u) ||
+            !warp_wait_bounded(&full_bar[s], (n / kStages) & 1u)) {
           raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
           break;
         }
         tc_fence_after();
+        if (!elect_one()) continue;
         const uint32_t a_addr = smem_u32(stage_base + (size_t)s * kStageBytes);
         const uint64_t da = smem_desc_k128(a_addr), db = smem_desc_k128(a_addr + kTileR * kBlockK);
 #pragma unroll

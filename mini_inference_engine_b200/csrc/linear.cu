@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kTileThreads, TileSmem<BN>::kCtasPerSm)
   uint64_t* empty_bar = full_bar + kStages;
   uint64_t* done_bar = empty_bar + kStages;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   const int split = gridDim.y, rank = blockIdx.y, tile = blockIdx.x;
   const int kb_total = (p.k + kTileK - 1) / kTileK;
   const int kb_first = (int)((long long)kb_total * rank / split);
@@ -341,15 +341,16 @@ __global__ void __launch_bounds__(kTileThreads, TileSmem<BN>::kCtasPerSm)
     }
     __syncwarp();
   } else if (warp == 5) {
-    if (lane == 0) {
+    {
       constexpr uint32_t idesc = instr_desc_bf16(kTileRows, BN, 0, 0);
       for (int i = 0; i < kb_count; ++i) {
         const int s = i % kStages;
-        if (!mbar_wait_bounded(&full_bar[s], (i / kStages) & 1u)) {
+        if (!warp_wait_bounded(&full_bar[s], (i / kStages) & 1u)) {
           raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
           break;
         }
         tc_fence_after();
+        if (!elect_one()) continue;
         const uint32_t a = smem_u32(ring + (size_t)s * S::kStageBytes);
         const uint64_t da = smem_desc_k128(a), db = smem_desc_k128(a + kTileRows * 128);
 #pragma unroll
@@ -357,7 +358,8 @@ __global__ void __launch_bounds__(kTileThreads, TileSmem<BN>::kCtasPerSm)
           umma_f16(tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, i > 0 || k > 0 ? 1u : 0u);
         umma_commit(&empty_bar[s]);
       }
-      umma_commit(done_bar);  // the accumulator is complete, the ring idle
+      __syncwarp();
+      if (elect_one()) umma_commit(done_bar);  // the accumulator is complete, the ring idle
     }
     __syncwarp();
   } else {
