@@ -35,13 +35,19 @@ class StateBuffer:
         self.rows[target].copy_(self.rows[source])
 
 
-def segment_tokens(max_query_len: int, lanes: int, sm_count: int = 148) -> int:
+def segment_tokens(max_query_len: int, lanes: int, sm_count: int = 148, per_sm: float = 0.0) -> int:
     """Tokens per parallel segment of a packed chunk, 0 for one segment per request.  ``lanes`` is how many CTAs run
     without cutting; requests are cut until the GPU has about one CTA per SM to run, in pieces of at least 256 (the
-    pieces but the last are gone over twice)."""
+    pieces but the last are gone over twice).  With ``per_sm``, the tokens an SM would go over if the work were spread
+    evenly, requests that nearly fill the GPU are cut too when the longest is much longer than that: cutting costs about
+    1.9 times an even spread (10000 tokens of 16 heads in five prompts, longest 2869: 343 us uncut, 261 cut; all 2000: 250
+    uncut, 262 cut)."""
 
-    if max_query_len <= 256 or 2 * lanes > sm_count:
+    if max_query_len <= 256:
         return 0
+    if 2 * lanes > sm_count:
+        length = max(256, -(-int(per_sm / 3) // TILE) * TILE)
+        return length if per_sm > 0 and max_query_len > 1.9 * per_sm + 200 else 0
     pieces = sm_count // max(lanes, 1)
     length = -(-max_query_len // pieces)
     return max(256, -(-length // TILE) * TILE)
@@ -54,7 +60,8 @@ def outer_recurrence(rows, out, decay, state, slots, positions, *, heads: int, d
     tokens, requests = int(rows.shape[0]), 0 if cu_seqlens is None else int(cu_seqlens.shape[0]) - 1
     length, carry = 0, None
     if cu_seqlens is not None and _lib.load().mie_outer_recurrence_chunked(dim, value_dim, _lib.DTYPE_CODES[rows.dtype]):
-        length = segment_tokens(max_query_len, requests * heads * -(-value_dim // 128))
+        lanes = heads * -(-value_dim // 128)
+        length = segment_tokens(max_query_len, requests * lanes, per_sm=tokens * lanes / 148)
         if length and max_query_len > length:
             carry = torch.empty((tokens // length + requests) * heads * dim * value_dim, dtype=torch.float32,
                                 device=rows.device)
