@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kOffBar);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kNumBars);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
 
   const int r = blockIdx.y;
   const int kvh = kExt ? (int)blockIdx.z / p.v_passes : (int)blockIdx.z;
@@ -251,17 +251,18 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == kSoftmaxWarps + 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    {
       constexpr int kFmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
       constexpr uint32_t idesc_s = instr_desc_f16(kKv, kFmt, 0);   // S = Q K^T : A = Q in TMEM, B = K, K-major
       constexpr uint32_t idesc_o = instr_desc_f16(VH * 64, kFmt, 1);  // O += P V : A = P in TMEM, B = V, MN-major
-      bool ok = mbar_wait_bounded(&bars[kQFull], 0);
+      bool ok = warp_wait_bounded(&bars[kQFull], 0);
       // S(j) overwrites the TMEM buffer that held S(j-2) / P(j-2); P(j-2) V(j-2) was issued earlier by this
       // thread and tcgen05.mma executes in issue order, so no barrier is needed for the reuse.
       auto issue_s = [&](int j) {
         const int s = j % kKvStages, b = j & 1;
-        if (!mbar_wait_bounded(&bars[kKFull + s], (j / kKvStages) & 1u)) return false;
+        if (!warp_wait_bounded(&bars[kKFull + s], (j / kKvStages) & 1u)) return false;
         tc_fence_after();
+        if (!elect_one()) return true;
         const uint32_t k_addr = smem_u32(smem + kOffK + s * kKTile);
 #pragma unroll
         for (int ks = 0; ks < KH * 4; ++ks) {  // 16 dims each
@@ -275,17 +276,20 @@ __global__ void __launch_bounds__(kThreads, 1)
         return true;
       };
       if (ok) ok = issue_s(0);
+      __syncwarp();
       for (int j = 0; j < n_tiles && ok; ++j) {
         const int s = j % kKvStages, b = j & 1;
         if (j + 1 < n_tiles) ok = issue_s(j + 1);
+        __syncwarp();
         if (!ok) break;
-        if (!mbar_wait_bounded(&bars[kPFull + b], (j >> 1) & 1u) ||
-            !mbar_wait_bounded(&bars[kVFull + s], (j / kKvStages) & 1u) ||
-            (j == n_tiles - 1 && !mbar_wait_bounded(&bars[kVClean], 0))) {
+        if (!warp_wait_bounded(&bars[kPFull + b], (j >> 1) & 1u) ||
+            !warp_wait_bounded(&bars[kVFull + s], (j / kKvStages) & 1u) ||
+            (j == n_tiles - 1 && !warp_wait_bounded(&bars[kVClean], 0))) {
           ok = false;
           break;
         }
         tc_fence_after();
+        if (!elect_one()) continue;
         const uint32_t v_addr = smem_u32(smem + kOffV + s * kVTile);
 #pragma unroll
         for (int kt = 0; kt < 8; ++kt) {  // 8 x 16 tokens = 8 TMEM columns of packed P each
