@@ -648,6 +648,14 @@ int mie_gated_norm(const void* x, int64_t ldx, const void* gate, int64_t ldg, co
 int mie_softcap(float* logits, int64_t count, float cap, void* stream);
 
 /*
+ * Greedy tokens of logit rows (bf16 or fp32 by `dtype`, row stride ld): out[r] is
+ * the index of row r's largest value, the first one among equals; a NaN counts
+ * as larger than any number.
+ */
+int mie_argmax_rows(const void* logits, int64_t ld, int32_t dtype, int32_t rows, int32_t cols, int64_t* out,
+                    void* stream);
+
+/*
  * One merged projection row [q_rank | rank | rot_dim] (row stride ld) ->
  * rms_norm(first part) * q_weight to q_out, and, with pages, the cached row
  * [rms_norm(second part) * weight | third part rotated] to the token's slot of

@@ -171,6 +171,7 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
                                 c_int32, c_int32, c_void_p, c_void_p]),
     "mie_gated_norm": (ctypes.c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int32,
                                       c_int32, c_int32, c_float, c_void_p]),
+    "mie_argmax_rows": (ctypes.c_int, [c_void_p, c_int64, c_int32, c_int32, c_int32, c_void_p, c_void_p]),
     "mie_softcap": (ctypes.c_int, [c_void_p, c_int64, c_float, c_void_p]),
     "mie_latent_norm_write": (ctypes.c_int, [c_void_p, c_int64, c_int32, c_int32, c_int32, c_int32, c_void_p,
                                              c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_int64,

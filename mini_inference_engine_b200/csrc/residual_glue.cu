@@ -225,12 +225,86 @@ __global__ void __launch_bounds__(512) gated_norm_kernel(GatedNormParams p) {
   }
 }
 
-// logits <- cap * tanh(logits / cap), in place.
-__global__ void softcap_kernel(float* logits, long long count, float cap) {
+// logits <- cap * tanh(logits / cap), in place, 16 bytes a thread from the first aligned element on (one element a thread:
+// 64 x 151936 41 us, now 13.7).
+__global__ void softcap_kernel(float* logits, long long count, float cap, int head) {
   chain_release();
   chain_wait();
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < count) logits[i] = cap * tanhf(logits[i] / cap);
+  auto capped = [&](float x) { return cap * tanhf(x / cap); };
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, i = head + t * 4;
+  if (t < head) logits[t] = capped(logits[t]);
+  if (i + 4 <= count) {
+    float4 v = *reinterpret_cast<const float4*>(logits + i);
+    *reinterpret_cast<float4*>(logits + i) = make_float4(capped(v.x), capped(v.y), capped(v.z), capped(v.w));
+  } else {
+    for (long long j = i; j < count; ++j) logits[j] = capped(logits[j]);
+  }
+}
+
+// Greedy token of a row: index of its largest value, the first one among equals; a NaN counts as larger than any number.
+// A cluster of CTAs reads a row in 16-byte pieces, each thread keeping its best, and the first CTA compares the others'.
+constexpr int kArgmaxCtas = 8, kArgmaxThreads = 256;
+
+__device__ __forceinline__ unsigned long long argmax_key(float v, int index) {
+  const uint32_t bits = __float_as_uint(v);
+  const uint32_t order = v != v ? 0xffffffffu : bits >> 31 ? ~bits : bits | 0x80000000u;
+  return (unsigned long long)(v == 0.f ? 0x80000000u : order) << 32 | (uint32_t)~index;
+}
+
+template <typename T>
+__global__ void __cluster_dims__(kArgmaxCtas, 1, 1) __launch_bounds__(kArgmaxThreads)
+    argmax_rows_kernel(const T* logits, long long ld, int cols, int vec, long long* out) {
+  __shared__ unsigned long long best_of[kArgmaxThreads / 32];
+  chain_release();
+  chain_wait();
+  constexpr int kVec = 16 / (int)sizeof(T), kBatch = 4;
+  const int row = blockIdx.x / kArgmaxCtas, rank = blockIdx.x % kArgmaxCtas, step = kArgmaxCtas * kArgmaxThreads;
+  const T* src = logits + (long long)row * ld;
+  const int first = rank * kArgmaxThreads + threadIdx.x, units = vec ? cols / kVec : 0;
+  unsigned long long best = 0;
+  auto take = [&](float v, int index) {
+    const unsigned long long key = argmax_key(v, index);
+    best = key > best ? key : best;
+  };
+  for (int u0 = first; u0 < units; u0 += kBatch * step) {
+    uint4 raw[kBatch];
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b)
+      raw[b] = *reinterpret_cast<const uint4*>(src + (long long)(u0 + b * step < units ? u0 + b * step : u0) * kVec);
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      const int u = u0 + b * step < units ? u0 + b * step : u0;
+      const T* v = reinterpret_cast<const T*>(&raw[b]);
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) take(to_float<T>(v[i]), u * kVec + i);
+    }
+  }
+  for (int c = units * kVec + first; c < cols; c += step) take(to_float<T>(src[c]), c);
+  auto reduce = [](unsigned long long v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long other = __shfl_xor_sync(0xffffffffu, v, o);
+      v = other > v ? other : v;
+    }
+    return v;
+  };
+  best = reduce(best);
+  if ((threadIdx.x & 31) == 0) best_of[threadIdx.x >> 5] = best;
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (rank == 0 && threadIdx.x < 32) {
+    constexpr int kWarps = kArgmaxThreads / 32;
+    best = 0;
+    for (int i = threadIdx.x; i < kArgmaxCtas * kWarps; i += 32) {
+      uint32_t remote;
+      unsigned long long v;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(&best_of[i % kWarps])), "r"(i / kWarps));
+      asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(remote) : "memory");
+      best = v > best ? v : best;
+    }
+    best = reduce(best);
+    if (threadIdx.x == 0) out[row] = (long long)(uint32_t)~(uint32_t)best;
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 int row_threads(int cols, bool vec) {
@@ -311,8 +385,29 @@ extern "C" int mie_gated_norm(const void* x, int64_t ldx, const void* gate, int6
 extern "C" int mie_softcap(float* logits, int64_t count, float cap, void* stream) {
   MIE_CHECK_ARG(logits && count >= 0 && cap > 0.f, "soft cap needs logits and a positive cap");
   if (count == 0) return MIE_OK;
-  MIE_CUDA(launch_chained(softcap_kernel, dim3((unsigned)((count + 255) / 256)), dim3(256), 0, (cudaStream_t)stream,
-                          logits, (long long)count, cap));
+  const int head = (int)(((16 - (reinterpret_cast<uintptr_t>(logits) & 15)) & 15) / 4);  // up to the first aligned one
+  const long long threads = count / 4 + 4;  // also covers a row shorter than the head
+  MIE_CUDA(launch_chained(softcap_kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, (cudaStream_t)stream,
+                          logits, (long long)count, cap, head < count ? head : (int)count));
   MIE_LAUNCH_CHECK("softcap_kernel");
+  return MIE_OK;
+}
+
+extern "C" int mie_argmax_rows(const void* logits, int64_t ld, int32_t dtype, int32_t rows, int32_t cols, int64_t* out,
+                               void* stream) {
+  MIE_CHECK_ACT_DTYPE(dtype);
+  MIE_CHECK_ARG(logits && out && rows >= 0 && cols >= 1 && ld >= cols, "invalid sizes");
+  MIE_CHECK_ARG(rows <= 0x7fffffff / kArgmaxCtas, "too many rows");
+  if (rows == 0) return MIE_OK;
+  const int act = dtype == MIE_DTYPE_BF16 ? 8 : 4;
+  const int vec = ld % act == 0 && aligned(logits, 16) ? 1 : 0;
+  const dim3 grid((unsigned)(rows * kArgmaxCtas)), block(kArgmaxThreads);
+  if (dtype == MIE_DTYPE_BF16)
+    MIE_CUDA(launch_chained(argmax_rows_kernel<__nv_bfloat16>, grid, block, 0, (cudaStream_t)stream,
+                            (const __nv_bfloat16*)logits, (long long)ld, cols, vec, (long long*)out));
+  else
+    MIE_CUDA(launch_chained(argmax_rows_kernel<float>, grid, block, 0, (cudaStream_t)stream, (const float*)logits,
+                            (long long)ld, cols, vec, (long long*)out));
+  MIE_LAUNCH_CHECK("argmax_rows_kernel");
   return MIE_OK;
 }

@@ -136,6 +136,20 @@ def gated_rms_norm(x, gate, weight, *, eps: float) -> torch.Tensor:
     return out
 
 
+def argmax_rows(logits: torch.Tensor) -> torch.Tensor:
+    """``logits.argmax(dim=-1)`` of ``[rows, vocabulary]`` logits in one pass (256 x 151936 in bf16: 52 us the
+    library's, 44 here; 64 rows in fp32 23 and 15)."""
+
+    if not (logits.is_cuda and logits.ndim == 2 and logits.dtype in (torch.bfloat16, torch.float32)
+            and logits.shape[1] > 0 and logits.stride(1) == 1 and logits.stride(0) >= logits.shape[1]):
+        return logits.argmax(dim=-1)
+    rows, cols = logits.shape
+    out = torch.empty(rows, dtype=torch.int64, device=logits.device)
+    _lib.check(_lib.load().mie_argmax_rows(_lib.ptr(logits), logits.stride(0), _lib.DTYPE_CODES[logits.dtype], rows, cols,
+                                           _lib.ptr(out), _lib.stream_arg(logits.device)))
+    return out
+
+
 def softcap_(logits, cap: float) -> torch.Tensor:
     """cap * tanh(logits / cap) in place on contiguous fp32 logits."""
 
@@ -143,5 +157,5 @@ def softcap_(logits, cap: float) -> torch.Tensor:
     return logits
 
 
-__all__ = ["clamped_glu", "embed_tokens", "gated_rms_norm", "gelu", "qkv_norm_mix_write", "residual_norm_",
+__all__ = ["argmax_rows", "clamped_glu", "embed_tokens", "gated_rms_norm", "gelu", "qkv_norm_mix_write", "residual_norm_",
            "sinusoid_turns", "softcap_", "sum_rms_norm"]

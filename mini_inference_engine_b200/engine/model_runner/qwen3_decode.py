@@ -35,6 +35,7 @@ import torch
 
 from ... import _lib
 from ..kernels import sm89_fp8
+from ..kernels.decoder_glue import argmax_rows
 from .peer_exchange import PeerExchange
 from .step_runner import (
     DEFAULT_DECODE_BUCKETS,
@@ -513,7 +514,7 @@ class Qwen3DecodeRunner(PagedStepRunner):
         logits = torch.matmul(final, self.weights.lm_head.t())
         self.launches_per_step = int(lib.mie_launch_count() - launches_before)
         if self.tp == 1:
-            tokens = logits.argmax(dim=-1)
+            tokens = argmax_rows(logits)
             return (tokens, logits) if return_logits else tokens
         return sharded_greedy_tokens(logits, self.weights.vocab_start, self.tp, self.group)
 
@@ -610,7 +611,10 @@ class Qwen3DecodeRunner(PagedStepRunner):
             return picked
         logits = torch.matmul(final, self.weights.lm_head.t())
         self.launches_per_step = int(lib.mie_launch_count() - launches_before)
-        picked = sharded_greedy_tokens(logits, self.weights.vocab_start, self.tp, self.group)
+        if self.tp == 1:
+            picked = argmax_rows(logits)
+        else:
+            picked = sharded_greedy_tokens(logits, self.weights.vocab_start, self.tp, self.group)
         return (picked, logits) if return_logits else picked
 
 

@@ -33,6 +33,7 @@ from types import SimpleNamespace
 import torch
 
 from ..kernels.decoder_glue import (
+    argmax_rows,
     embed_tokens,
     gated_rms_norm,
     gelu,
@@ -364,7 +365,7 @@ class RipesunRunner(PagedStepRunner):
             return self.lm_head_argmax(final, weights.head)
         head = weights.head.t()
         logits = torch.mm(final, head) if self.dtype == torch.float32 else torch.mm(final, head, out_dtype=torch.float32)
-        tokens = logits.argmax(dim=-1)
+        tokens = argmax_rows(logits)
         return (tokens, softcap_(logits, self.shape.logit_softcap)) if return_logits else tokens
 
     # -- mixers ---------------------------------------------------------------------------------

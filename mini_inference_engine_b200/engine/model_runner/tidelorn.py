@@ -25,7 +25,14 @@ from dataclasses import dataclass
 import torch
 
 from ..kernels.linear import linear
-from ..kernels.decoder_glue import clamped_glu, embed_tokens, qkv_norm_mix_write, sinusoid_turns, sum_rms_norm
+from ..kernels.decoder_glue import (
+    argmax_rows,
+    clamped_glu,
+    embed_tokens,
+    qkv_norm_mix_write,
+    sinusoid_turns,
+    sum_rms_norm,
+)
 from ..kv_cache.sink_attention import (
     attention_rows,
     sink_decode_attention,
@@ -285,7 +292,7 @@ class TidelornRunner(PagedStepRunner):
         if not return_logits and self.can_fuse_lm_head(final, self.weights.head):
             return self.lm_head_argmax(final, self.weights.head)
         logits = self._logits(final)
-        tokens = logits.argmax(dim=-1)
+        tokens = argmax_rows(logits)
         return (tokens, logits) if return_logits else tokens
 
     # -- the layers -----------------------------------------------------------------------------

@@ -83,3 +83,40 @@ def test_qkv_rows_of_odd_head_counts_and_alignments(heads, offset, device, statu
         want_q, want_s = hot_path.quantize_kv_rows(dense.cpu())
         assert torch.equal(pool[:, :, which], want_q)
         assert torch.equal(scales[:, :, which].cpu(), want_s)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,cols,pad", [(1, 1, 0), (3, 7, 0), (2, 2049, 3), (5, 16384, 8), (4, 151936, 0)])
+def test_greedy_tokens_of_logit_rows(dtype, rows, cols, pad, device):
+    """The first of the largest values, whatever the alignment; infinities, zeros of both signs, NaN."""
+
+    from mini_inference_engine_b200.engine.kernels.decoder_glue import argmax_rows
+
+    generator = torch.Generator().manual_seed(cols)
+    logits = torch.randn(rows, cols + pad, generator=generator).to(dtype)[:, :cols]
+    logits[0] = -float("inf")
+    if rows > 2:
+        logits[1], logits[1, cols // 2], logits[1, cols // 3] = -1.0, 0.0, -0.0
+        logits[2, [cols // 2, cols - 1]] = float("inf")
+    if rows > 3:
+        logits[3, [cols // 3, cols // 2]] = float("nan")
+    wide = torch.empty(rows, cols + pad, dtype=dtype, device=device)
+    wide[:, :cols] = logits.to(device)
+    values = torch.nan_to_num(logits.float(), nan=float("inf"), posinf=3.4e38)  # NaN above infinity
+    values = torch.where(logits.isnan(), torch.full_like(values, float("inf")), values)
+    want = (values == values.amax(dim=1, keepdim=True)).int().argmax(dim=1)
+    assert torch.equal(argmax_rows(wide[:, :cols]).cpu(), want)
+
+
+@pytest.mark.parametrize("count,offset", [(1, 0), (2, 3), (5, 1), (1023, 2), (4096, 0), (4099, 3)])
+def test_soft_cap_of_any_alignment(count, offset, device):
+    from mini_inference_engine_b200.engine.kernels.decoder_glue import softcap_
+
+    x = torch.randn(count + offset + 3, generator=torch.Generator().manual_seed(count)) * 50
+    x[offset] = float("inf")
+    held = x.to(device)
+    softcap_(held[offset:offset + count], 30.0)
+    want = x.double()
+    want[offset:offset + count] = 30.0 * torch.tanh(want[offset:offset + count] / 30.0)
+    # tanhf is within 2 units in the last place, the division and the product add half a unit each
+    assert ((held.cpu().double() - want).abs() <= 4 * 2 ** -24 * want.abs() * 2).all()
