@@ -36,17 +36,21 @@ __device__ __forceinline__ uint2 pack4(const float (&v)[4]) {
 }
 
 // a / b from y, an approximation of 1 / b: quotient, its exact remainder, correction.  Correctly rounded when y is the
-// correctly rounded reciprocal (Markstein's theorem), else within a little more than half a unit in the last place.
-// Three instructions where an IEEE division takes about ten.  b and y must be finite.
+// correctly rounded reciprocal (Markstein's theorem), else but for quotients within 2^-20 units of a tie.  Three
+// instructions where an IEEE division takes about ten.  a, b and y must be finite.
 __device__ __forceinline__ float corrected_quotient(float a, float b, float y) {
   const float q = a * y;
   return fmaf(-fmaf(q, b, -a), y, q);  // signs placed so that a zero keeps its own
 }
 
 // g / (1 + exp(-slope g)).
-__device__ __forceinline__ float gate_sigmoid(float g, float slope = 1.f) {
+__device__ __forceinline__ float gate_sigmoid(float g, float slope = 1.f) { return g / (1.f + expf(-slope * g)); }
+
+// The same for a result that is rounded to 16 bits: SiLU of every bf16 value comes out as with the division.
+__device__ __forceinline__ float gate_sigmoid16(float g, float slope = 1.f) {
   const float d = 1.f + expf(-slope * g);
-  if (d > 1e37f) return __fdiv_rn(g, d);  // reciprocal near or below the smallest normal number
+  // a reciprocal near or below the smallest normal number, an infinite gate
+  if (d > 1e37f || fabsf(g) > 3.4e38f) return __fdiv_rn(g, d);
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
   return corrected_quotient(g, d, y);

@@ -120,3 +120,41 @@ def test_soft_cap_of_any_alignment(count, offset, device):
     want[offset:offset + count] = 30.0 * torch.tanh(want[offset:offset + count] / 30.0)
     # tanhf is within 2 units in the last place, the division and the product add half a unit each
     assert ((held.cpu().double() - want).abs() <= 4 * 2 ** -24 * want.abs() * 2).all()
+
+
+def test_gated_activations_of_any_value(device):
+    """SiLU(gate) * up of every bf16 gate, infinities and NaN included: the division's own results."""
+
+    from mini_inference_engine_b200.engine.kernels import fused
+
+    gate = torch.arange(65536, dtype=torch.int32).to(torch.uint16).view(torch.bfloat16).view(64, 1024).to(device)
+    for factor in (1.0, -0.37):
+        up = torch.full_like(gate, factor)
+        wide = gate.float()
+        want = (wide / (1.0 + torch.exp(-wide))).to(torch.bfloat16) * up
+        got = fused.silu_mul(gate, up)
+        assert torch.equal(got.isnan(), want.isnan())
+        assert torch.equal(torch.nan_to_num(got), torch.nan_to_num(want))
+    # The quantised form: an infinite value makes its group's scale infinite.
+    gate = torch.ones(1, 256, dtype=torch.bfloat16, device=device)
+    gate[0, 5] = float("inf")
+    q, scales = torch.empty(1, 256, dtype=torch.uint8, device=device), torch.empty(2, 1, device=device)
+    _lib.check(_lib.load().mie_silu_mul(_lib.ptr(gate), _lib.ptr(torch.ones_like(gate)), 256, None, _lib.ptr(q), 256,
+                                        _lib.ptr(scales), 1, 1, 256, _lib.stream_arg(device)))
+    assert scales[0].item() == float("inf") and 0 < scales[1].item() < 1
+
+
+@pytest.mark.parametrize("slope", [1.0, 1.702, 1e-6])
+def test_clamped_gates_are_ieee_quotients(slope, device):
+    """The fp32 form stores the quotient unrounded; gates from subnormal to infinite, no clamp."""
+
+    from mini_inference_engine_b200.engine.kernels.decoder_glue import clamped_glu
+
+    generator = torch.Generator(device=device).manual_seed(5)
+    gate = torch.randn(512, 4096, generator=generator, device=device)
+    gate[256:] *= torch.exp(torch.linspace(-100, 85, 256, device=device))[:, None]
+    gate[0, :4] = torch.tensor([0.0, -0.0, float("inf"), 1e-42], device=device)
+    both = torch.cat([gate, torch.zeros_like(gate)], dim=1)
+    got = clamped_glu(both, limit=float("inf"), slope=slope, up_offset=1.0)
+    want = gate / (1.0 + torch.exp(-slope * gate))
+    assert torch.equal(got, want)
