@@ -168,7 +168,7 @@ __global__ void rope_kernel(const __nv_bfloat16* x, long long sb, long long sh, 
 // q/k RMSNorm + RoPE + KV-cache write over a merged qkv row (head_dim 128).  A block per token (or several), 16 lanes per head, eight
 // consecutive dims a lane (partner dims d +/- 64 sit 8 lanes away): a lane's cos / sin entries, position and page serve
 // all the heads of its half-warp, whose rows are in flight together.  A warp per (token, head) with 8-byte accesses
-// looked all of that up per head: 12032 tokens of 48 heads 185 us, now 129 us (147 MB in, 147 MB out).
+// looked all of that up per head: 12032 tokens of 48 heads 185 us, now 131 us (147 MB in, 147 MB out).
 // ---------------------------------------------------------------------------
 // Eight bf16 values, 16-byte aligned when `wide`, else 8-byte.
 __device__ __forceinline__ uint4 load8(const __nv_bfloat16* p, bool wide) {
@@ -224,12 +224,7 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvParams p) {
       const bool is_q = h < p.q_heads, is_v = h >= p.q_heads + p.kv_heads, live = h < heads_total;
       float v[8], w[8], o[8];
       unpack8(raw[u], v);
-      float ss = 0.f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
-#pragma unroll
-      for (int d = 8; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
-      const float inv = rsqrtf(ss / 128.f + p.eps);
+      const float inv = rsqrtf(half_warp_square_sum(v, l16) / 128.f + p.eps);
       unpack8(load8((is_q ? p.q_weight : p.k_weight) + l16 * 8, p.wide), w);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
