@@ -322,12 +322,18 @@ int mie_fp8_quantize(const void* x, int64_t ldx, int32_t dtype, void* q, int64_t
  * promise, tests/test_sm89_fp8_exact.py); max_split = 0 lets the library
  * choose, other values cap the factor.  Uses no global scratch memory.
  *
- * flags: MIE_GEMM_NO_WEIGHT_PREFETCH, or 0.  By default the weight tiles of the
- * first pipeline stages are requested while the kernel queued before this one
- * may still be running (programmatic dependent launch), so w8 must not be
- * written by that kernel; pass the flag (or set MIE_GEMM_PREFETCH=0) when it is.
+ * flags: 0 or MIE_GEMM_STATIC_WEIGHTS.  With the flag the caller promises that
+ * nothing still queued or running on the stream writes w8 (a model's
+ * parameters): the weight tiles of the first pipeline stages are then requested
+ * before the kernels queued ahead have finished.  That reaches more than one
+ * launch back, because the kernels of this library let their successor start
+ * before they have waited for their predecessor (programmatic dependent launch).
+ * Without the flag w8 is read after all queued work, like every other operand.
+ * MIE_GEMM_NO_WEIGHT_PREFETCH, or MIE_GEMM_PREFETCH=0 in the environment, takes
+ * the flag's effect away.
  */
 #define MIE_GEMM_NO_WEIGHT_PREFETCH 1
+#define MIE_GEMM_STATIC_WEIGHTS 2
 int mie_fp8_gemm(const void* x8, int64_t ldx, const float* a_scale, int32_t a_scale_ld, const void* w8,
                  int64_t ldw, const float* w_scale, int32_t w_scale_ld, void* y, int64_t ldy, int32_t out_dtype,
                  int32_t m, int32_t n, int32_t k, int32_t max_split, int32_t flags, int32_t* status, void* stream);
@@ -449,10 +455,13 @@ int mie_lm_head_argmax(const void* x, int64_t ldx, const void* w, int64_t ldw, i
  * Projection of up to MIE_LINEAR_MAX_ROWS bf16 rows: y[m, n] = x[m, k] w[n, k]^T (+ bias[n]), fp32 sums rounded once
  * to bf16 (the decode-sized products of the bf16 designs; larger ones are library products).  k must be a multiple of
  * 8, operand rows 16-byte aligned; strides in elements.  Part of the launch chain: the weights may be requested before
- * the kernels queued earlier on the stream have finished, so those must not be kernels of this library that write
- * them.  kernel: 0 picks by the number of rows, 1 the register kernel (at most 32 rows), 2 the tensor-memory kernel.
+ * the kernels queued earlier on the stream have finished, so none of those, however far back, may write them.  kernel:
+ * 0 picks by the number of rows, 1 the register kernel (at most 32 rows), 2 the tensor-memory kernel; add
+ * MIE_LINEAR_NO_WEIGHT_PREFETCH (or set MIE_GEMM_PREFETCH=0 in the environment) to have the weights read after all
+ * queued work.
  */
 #define MIE_LINEAR_MAX_ROWS 128
+#define MIE_LINEAR_NO_WEIGHT_PREFETCH 4
 int mie_linear(const void* x, int64_t ldx, const void* w, int64_t ldw, const void* bias, void* y, int64_t ldy,
                int32_t m, int32_t n, int32_t k, int32_t kernel, int32_t* status, void* stream);
 

@@ -141,7 +141,7 @@ def gemm(args, device) -> dict:
 
     def run_all():
         for weight in weights:
-            sm89_fp8.launch_fp8_gemm(quantized, a_scales, weight, scales, out, args.rows, k)
+            sm89_fp8.launch_fp8_gemm(quantized, a_scales, weight, scales, out, args.rows, k, static_weight=True)
 
     run_all()
     torch.cuda.synchronize(device)

@@ -27,6 +27,7 @@ STATUS_BAD_TOKEN = 256
 STATUS_BAD_SLOT = 512
 
 GEMM_NO_WEIGHT_PREFETCH = 1
+GEMM_STATIC_WEIGHTS = 2
 
 STATUS_MESSAGES = {
     STATUS_BAD_LENGTH: "sequence_lengths exceed the available block-table capacity",

@@ -45,6 +45,7 @@ int cuda_fail(cudaError_t err, const char* what);
 int sm_count();
 void count_launch();  // every kernel launch of this library bumps a host-side counter
 bool chained_launch_enabled();  // false when MIE_PDL=0
+bool weight_prefetch_enabled();  // false when MIE_GEMM_PREFETCH=0
 // Once per kernel and device: ask for the largest shared-memory carve-out, so that a small kernel and the
 // GEMM / attention kernel chained after it (200 KB of shared memory) can be resident on one SM together.
 void prefer_shared_carveout(const void* kernel);
@@ -56,7 +57,9 @@ void prefer_shared_carveout(const void* kernel);
 // global memory that another kernel of the stream writes: the wait returns once the previous kernel has finished (and
 // so, as that one waited too, all before it) and its writes are visible.  Releasing before waiting lets a GEMM two
 // launches ahead set up and request its weights while the GEMM before it is still running; a kernel is only scheduled
-// when every block of the one before it has released, so a waiting block never keeps an earlier one off the GPU.
+// when every block of the one before it has released, so a waiting block never keeps an earlier one off the GPU.  What is
+// read before the wait may therefore not be written by ANY kernel still queued, however far back: only weights that the
+// caller promises to be static are.
 // Releasing after the wait is left to kernels whose successor relies on their wait (the first launch of a two-launch
 // GEMM).  Both are no-ops for a kernel launched the ordinary way.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -26,7 +26,6 @@
 //   * Every mbarrier wait is bounded; a wait that runs out sets
 //     MIE_STATUS_WAIT_TIMEOUT, the roles fall through to the common exit and
 //     TMEM is released.
-#include <cstdlib>
 #include <mutex>
 #include <unordered_map>
 
@@ -59,7 +58,7 @@ struct GemmParams {
   long long ldy;
   int out_f16;
   int* status;
-  int prefetch;           // weights of the first K blocks are requested before the launch-chain wait
+  int prefetch;           // weights of the first K blocks are requested before the launch-chain wait (static weights)
   // Wide kernel only: this launch covers output tiles [tile_begin, tile_end).  late_wait: the launch-chain
   // wait is taken at the end of the kernel instead of the start (second launch of a two-launch GEMM, whose
   // inputs are already known to be complete because the first launch waited for them).
@@ -263,7 +262,7 @@ __global__ void __launch_bounds__(kNarrowThreads<BN>, GemmSmem<BN>::kCtasPerSm)
   const int kb_last = (int)((long long)kb_total * (part + 1) / split);  // exclusive
 
   // Everything up to the launch-chain wait overlaps the kernels queued before this one.  So does the weight half of
-  // the first stages (the caller promises that those kernels do not write the weights): the producer requests it
+  // the first stages when the caller promises that none of those kernels writes the weights: the producer requests it
   // before the TMEM allocation, which may have to wait for an earlier kernel's, and adds the activation half after
   // the wait.
   uint32_t prefetched = 0;
@@ -632,7 +631,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                 it.tn * BN);
   };
   // Barriers, tensor-map prefetch and the TMEM allocation above overlap the tail of the previous kernel.
-  // So can the weights (nothing on the stream writes them): the producer requests the weight half of its
+  // So can static weights (nothing on the stream writes them): the producer requests the weight half of its
   // first stages before the launch-chain wait and adds the activation half afterwards.
   uint32_t prefetched = 0;
   if (p.prefetch && warp == E && lane == 0) {
@@ -1164,7 +1163,7 @@ int gemm_params(GemmParams& p, const void* x8, int64_t ldx, const float* a_scale
   MIE_CHECK_ARG(((reinterpret_cast<uintptr_t>(x8) | reinterpret_cast<uintptr_t>(w8)) & 15) == 0,
                 "operands must be 16-byte aligned");
   MIE_CHECK_ARG(a_scale_ld >= m && w_scale_ld >= (k + 127) / 128, "invalid leading dimension");
-  MIE_CHECK_ARG((flags & ~(MIE_GEMM_NO_WEIGHT_PREFETCH)) == 0, "unknown flag bits %d", flags);
+  MIE_CHECK_ARG((flags & ~(MIE_GEMM_NO_WEIGHT_PREFETCH | MIE_GEMM_STATIC_WEIGHTS)) == 0, "unknown flag bits %d", flags);
   p = GemmParams{};
   p.m = m;
   p.n = n;
@@ -1174,11 +1173,7 @@ int gemm_params(GemmParams& p, const void* x8, int64_t ldx, const float* a_scale
   p.w_scale = w_scale;
   p.w_scale_ld = w_scale_ld;
   p.status = status;
-  static const int prefetch = [] {
-    const char* v = getenv("MIE_GEMM_PREFETCH");
-    return v != nullptr && v[0] == '0' ? 0 : 1;  // MIE_GEMM_PREFETCH=0 turns it off
-  }();
-  p.prefetch = prefetch && !(flags & MIE_GEMM_NO_WEIGHT_PREFETCH);
+  p.prefetch = weight_prefetch_enabled() && flags == MIE_GEMM_STATIC_WEIGHTS;
   return MIE_OK;
 }
 

@@ -2,8 +2,8 @@
 //
 // Such a product streams the weights once and does little else, and in a decode step it is one link of a chain of short
 // kernels: besides HBM bandwidth the time between the end of the kernel before it and its own end counts.  Both kernels
-// request their first weights before the launch-chain wait (the caller promises that the kernels queued before do not
-// write them) and are launched in the same programmatic chain as the rest of the library.
+// request their first weights before the launch-chain wait (the caller promises that no kernel queued before, however
+// far back, writes them) and are launched in the same programmatic chain as the rest of the library.
 //
 //   * linear_rows_kernel, few rows: weights go from global memory straight into registers, as the A operand of mma.sync
 //     (16 weight rows x 8 tokens).  A warp keeps D units of 16 rows x 64 columns in flight; a block of 8 warps takes 16
@@ -32,6 +32,7 @@ struct LinearParams {
   __nv_bfloat16* y;
   long long ldy;
   int* status;
+  int prefetch;  // weights are requested before the launch-chain wait
 };
 
 // ---------------------------------------------------------------------------
@@ -77,6 +78,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 2) linear_rows_kernel(const L
   RowsUnit<NT> ring[D];
 
   chain_release();
+  if (!p.prefetch) chain_wait();
 
   auto load_weights = [&](RowsUnit<NT>& u, int tile, int unit) {
     const int col = unit * kRowsUnit + t * 8;
@@ -302,7 +304,7 @@ __global__ void __launch_bounds__(kTileThreads, TileSmem<BN>::kCtasPerSm)
     mbar_init(done_bar, 1);
     mbar_fence_init();
     const uint64_t policy = l2_evict_first_policy();
-    for (; prefetched < kb_count && prefetched < kStages; ++prefetched) {
+    for (; p.prefetch && prefetched < kb_count && prefetched < kStages; ++prefetched) {
       mbar_expect_tx(&full_bar[prefetched], S::kStageBytes);
       tma_load_2d_hint(ring + (size_t)prefetched * S::kStageBytes, &map_w, &full_bar[prefetched],
                        (kb_first + prefetched) * kTileK, tile * kTileRows, policy);
@@ -526,10 +528,12 @@ extern "C" int mie_linear(const void* x, int64_t ldx, const void* w, int64_t ldw
   MIE_CHECK_ARG(ldx % 8 == 0 && ldw % 8 == 0 &&
                     ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0,
                 "operand rows must be 16-byte aligned");
+  const int prefetch = weight_prefetch_enabled() && !(kernel & MIE_LINEAR_NO_WEIGHT_PREFETCH);
+  kernel &= ~MIE_LINEAR_NO_WEIGHT_PREFETCH;
   MIE_CHECK_ARG(kernel >= 0 && kernel <= 2 && (kernel != 1 || m <= 32), "unknown kernel %d for %d rows", kernel, m);
   if (m == 0) return MIE_OK;
   const LinearParams p{(const __nv_bfloat16*)w, ldw, (const __nv_bfloat16*)x, ldx, m, n, k, (const __nv_bfloat16*)bias,
-                       (__nv_bfloat16*)y, ldy, status};
+                       (__nv_bfloat16*)y, ldy, status, prefetch};
   // The register kernel has the shorter start and end, the tensor-memory kernel the better stream: at one row (norm
   // included, us) 256 x 2048 3.5 against 5.1, 4096 x 2048 6.2 / 6.8, 8192 x 2048 12.3 / 8.8; at 16 rows 2048 x 256
   // 3.3 / 5.5, 2048 x 2048 7.2 / 6.8.

@@ -37,6 +37,14 @@ bool chained_launch_enabled() {
   return enabled;
 }
 
+bool weight_prefetch_enabled() {
+  static const bool enabled = [] {
+    const char* v = getenv("MIE_GEMM_PREFETCH");
+    return !(v != nullptr && v[0] == '0');
+  }();
+  return enabled;
+}
+
 void prefer_shared_carveout(const void* kernel) {
   static const bool enabled = [] {
     const char* v = getenv("MIE_CARVEOUT");

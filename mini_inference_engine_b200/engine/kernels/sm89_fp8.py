@@ -189,8 +189,8 @@ def _gemm_weight(weight: torch.Tensor) -> tuple[torch.Tensor, bool]:
     a copy was written just now on the current stream.
 
     Model weights (K a multiple of 16) pass through untouched.  Odd shapes are copied into a padded buffer
-    the first time they are seen; the GEMM that follows that copy must not request weight tiles ahead of
-    its launch-chain wait (``MIE_GEMM_NO_WEIGHT_PREFETCH``), later calls reuse the buffer.
+    the first time they are seen; for the GEMM that follows that copy the weight is not static
+    (``MIE_GEMM_STATIC_WEIGHTS``), later calls reuse the buffer.
     """
 
     k = weight.shape[1]
@@ -212,8 +212,11 @@ def _gemm_weight(weight: torch.Tensor) -> tuple[torch.Tensor, bool]:
 
 def launch_fp8_gemm(quantized: torch.Tensor, scales_kmajor: torch.Tensor, weight: torch.Tensor,
                     weight_scale_inv: torch.Tensor, output: torch.Tensor, m: int, k: int,
-                    status: torch.Tensor | None = None, max_split: int | None = None) -> None:
-    """``output[m, n] = fp8 block-scaled product``; thin call into ``mie_fp8_gemm``."""
+                    status: torch.Tensor | None = None, max_split: int | None = None,
+                    static_weight: bool = False) -> None:
+    """``output[m, n] = fp8 block-scaled product``; thin call into ``mie_fp8_gemm``.  ``static_weight`` promises that
+    nothing queued on the stream writes the weight (a runner's parameters): the GEMM then requests it before the kernels
+    ahead of it have finished."""
 
     device = output.device
     w, fresh_copy = _gemm_weight(weight)
@@ -224,7 +227,7 @@ def launch_fp8_gemm(quantized: torch.Tensor, scales_kmajor: torch.Tensor, weight
         _lib.ptr(w), w.stride(0), _lib.ptr(scales_w), scales_w.stride(0),
         _lib.ptr(output), output.stride(0), _lib.DTYPE_CODES[output.dtype], m, int(weight.shape[0]), k,
         int(_DEFAULT_MAX_SPLIT if max_split is None else max_split),
-        _lib.GEMM_NO_WEIGHT_PREFETCH if fresh_copy else 0, _lib.ptr(word), _lib.stream_arg(device),
+        _lib.GEMM_STATIC_WEIGHTS if static_weight and not fresh_copy else 0, _lib.ptr(word), _lib.stream_arg(device),
     ))
 
 

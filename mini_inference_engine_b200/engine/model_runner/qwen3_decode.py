@@ -364,7 +364,8 @@ class Qwen3DecodeRunner(PagedStepRunner):
     def _gemm(self, quantized, weight, weight_scale, rows: int, k: int, out: torch.Tensor | None = None) -> torch.Tensor:
         if out is None:
             out = torch.empty(rows, weight.shape[0], dtype=torch.bfloat16, device=self.device)
-        sm89_fp8.launch_fp8_gemm(quantized[0], quantized[1], weight, weight_scale, out, rows, k, status=self.status)
+        sm89_fp8.launch_fp8_gemm(quantized[0], quantized[1], weight, weight_scale, out, rows, k, status=self.status,
+                                 static_weight=True)
         return out
 
     def _quantize(self, x: torch.Tensor):
@@ -397,7 +398,7 @@ class Qwen3DecodeRunner(PagedStepRunner):
             _lib.ptr(quantized[0]), quantized[0].stride(0), _lib.ptr(quantized[1]), quantized[1].stride(0),
             _lib.ptr(weight), weight.stride(0), _lib.ptr(layer.gate_up_scale), layer.gate_up_scale.stride(0), _lib.ptr(q),
             q.stride(0), _lib.ptr(scales), scales.stride(0), rows, inter, self.shape.hidden,
-            sm89_fp8.default_max_split(), 0, _lib.ptr(self.status), _lib.stream_arg(self.device)))
+            sm89_fp8.default_max_split(), _lib.GEMM_STATIC_WEIGHTS, _lib.ptr(self.status), _lib.stream_arg(self.device)))
         return q, scales
 
     def _row_parallel_then_norm(self, quantized, weight, weight_scale, rows: int, k: int, residual, norm_weight,
@@ -462,8 +463,8 @@ class Qwen3DecodeRunner(PagedStepRunner):
             _lib.ptr(layer.q_norm), _lib.ptr(layer.k_norm), _lib.ptr(self.rope), int(self.rope.shape[0]),
             _lib.index_arg(positions), _lib.index_arg(token_to_sequence), _lib.index_arg(block_tables),
             _lib.ptr(queries), *cache, tokens, shape.hidden, self.local_q_heads, self.local_kv_heads, shape.page,
-            self.total_pages, table_rows, int(block_tables.shape[1]), shape.rms_eps, sm89_fp8.default_max_split(), 0,
-            _lib.ptr(self.status), _lib.stream_arg(self.device)))
+            self.total_pages, table_rows, int(block_tables.shape[1]), shape.rms_eps, sm89_fp8.default_max_split(),
+            _lib.GEMM_STATIC_WEIGHTS, _lib.ptr(self.status), _lib.stream_arg(self.device)))
 
     # -- the decode forward -------------------------------------------------------------------
 

@@ -132,3 +132,34 @@ def test_rows_do_not_depend_on_the_batch_in_invariant_mode(name, device, status_
         assert torch.equal(single, full[999:1000])
     finally:
         sm89_fp8.set_batch_invariant(previous)
+
+
+@pytest.mark.parametrize("m", [1, 40, 300])
+def test_weights_written_by_queued_kernels_are_read_after_them(m, device, status_clean):
+    """A product without the static-weights promise reads weights that a kernel two launches ahead of it writes."""
+
+    from mini_inference_engine_b200 import _lib
+    from mini_inference_engine_b200.engine.kernels.decoder_glue import softcap_
+
+    n, k = 19456, 2560
+    lib, stream = _lib.load(), _lib.stream_arg(device)
+    generator = torch.Generator(device=device).manual_seed(m)
+    sources = [torch.randn(n, k, generator=generator, device=device).to(torch.bfloat16) for _ in range(2)]
+    q, scales = sm89_fp8.quantize_activation_kmajor(torch.randn(m, k, generator=generator, device=device).bfloat16())
+    w8, row_scales = torch.empty(n, k, dtype=torch.float8_e4m3fn, device=device), torch.empty(k // 128, n, device=device)
+    w_scale, between = torch.full((n // 128, k // 128), 1e-3, device=device), torch.ones(4, device=device)
+    out = torch.empty(m, n, dtype=torch.bfloat16, device=device)
+
+    def step(source, wait):
+        _lib.check(lib.mie_fp8_quantize(_lib.ptr(source), k, _lib.DTYPE_CODES[source.dtype], _lib.ptr(w8), k,
+                                        _lib.ptr(row_scales), n, n, k, stream))
+        softcap_(between, 30.0)
+        if wait:
+            torch.cuda.synchronize()
+        sm89_fp8.launch_fp8_gemm(q, scales, w8, w_scale, out, m, k)
+        return out.clone()
+
+    want = [step(source, True) for source in sources]
+    assert not torch.equal(*want)
+    for i in range(40):
+        assert torch.equal(step(sources[i % 2], False), want[i % 2])

@@ -69,3 +69,18 @@ def test_library_path_override(monkeypatch, tmp_path):
     monkeypatch.setenv("MIE_LIBRARY_PATH", str(tmp_path / "elsewhere.so"))
     with pytest.raises(_lib.MieLibraryError, match="elsewhere.so is missing"):
         _lib.load()
+
+
+def test_weights_are_requested_early_only_on_request(library):
+    """``MIE_GEMM_STATIC_WEIGHTS`` is a promise of the caller, not the default (an empty product returns before any
+    launch, after its flags were looked at)."""
+
+    lib = _lib.load()
+    aligned = ctypes.c_void_p(4096)
+
+    def gemm(flags):
+        return lib.mie_fp8_gemm(aligned, 128, aligned, 1, aligned, 128, aligned, 1, aligned, 128, 1, 0, 128, 128, 0, flags,
+                                None, None)
+
+    assert "MIE_GEMM_STATIC_WEIGHTS 2" in HEADER.read_text() and _lib.GEMM_STATIC_WEIGHTS == 2
+    assert [gemm(flags) for flags in (0, 1, 2, 3, 4)] == [0, 0, 0, 0, -1]

@@ -54,3 +54,29 @@ def test_what_the_kernels_do_not_take_goes_to_the_library(device):
     for a, b in ((x, w), (x.bfloat16(), w.bfloat16()), (x[:0].bfloat16(), w.bfloat16())):
         assert not linear_supported(a, b)
         torch.testing.assert_close(linear(a, b, status=status), torch.nn.functional.linear(a, b))
+
+
+@pytest.mark.parametrize("m,n,k", [(3, 4096, 512), (20, 12288, 4096)])
+def test_weights_written_by_a_queued_kernel(m, n, k, device):
+    """``MIE_LINEAR_NO_WEIGHT_PREFETCH``: the weights are read after the kernel of this library that writes them."""
+
+    from mini_inference_engine_b200 import _lib
+    from mini_inference_engine_b200.engine.kernels.decoder_glue import gelu
+
+    generator = torch.Generator(device=device).manual_seed(m)
+    sources = [torch.randn(n, k, generator=generator, device=device).bfloat16() for _ in range(2)]
+    x = torch.randn(m, k, generator=generator, device=device).bfloat16()
+    status, out = torch.zeros(1, dtype=torch.int32, device=device), torch.empty(m, n, dtype=torch.bfloat16, device=device)
+
+    def step(source, wait):
+        w = gelu(source)
+        if wait:
+            torch.cuda.synchronize()
+        _lib.check(_lib.load().mie_linear(_lib.ptr(x), k, _lib.ptr(w), k, None, _lib.ptr(out), n, m, n, k, 4,
+                                          _lib.ptr(status), _lib.stream_arg(device)))
+        return out.clone()
+
+    want = [step(source, True) for source in sources]
+    for i in range(20):
+        assert torch.equal(step(sources[i % 2], False), want[i % 2])
+    assert int(status.item()) == 0
