@@ -534,11 +534,12 @@ extern "C" int mie_linear(const void* x, int64_t ldx, const void* w, int64_t ldw
   if (m == 0) return MIE_OK;
   const LinearParams p{(const __nv_bfloat16*)w, ldw, (const __nv_bfloat16*)x, ldx, m, n, k, (const __nv_bfloat16*)bias,
                        (__nv_bfloat16*)y, ldy, status, prefetch};
-  // The register kernel has the shorter start and end, the tensor-memory kernel the better stream: at one row (norm
-  // included, us) 256 x 2048 3.5 against 5.1, 4096 x 2048 6.2 / 6.8, 8192 x 2048 12.3 / 8.8; at 16 rows 2048 x 256
-  // 3.3 / 5.5, 2048 x 2048 7.2 / 6.8.
+  // The register kernel has the shorter start and end, the tensor-memory kernel the better stream and K cut in parts: at
+  // one row (norm included, us) 256 x 2048 3.6 against 5.0, 4096 x 2048 6.4 / 6.5, 8192 x 2048 12.7 / 8.6, and of long
+  // sums, which a block of the first goes through alone, 256 x 4096 7.4 / 6.2, 512 x 12288 22.6 / 11.4; at 16 rows
+  // 2048 x 512 4.2 / 6.0, 2048 x 2048 7.9 / 7.0, 128 x 8192 18.4 / 9.0.
   const long long work = (long long)n * k;
-  const bool few = (m <= 8 && work <= 4096ll * 2048) || (m <= 16 && work <= 1024ll * 1024);
+  const bool few = k <= 2048 && ((m <= 8 && work <= 4096ll * 2048) || (m <= 16 && work <= 1024ll * 1024));
   if (kernel == 1 || (kernel == 0 && few)) {
     if (m <= 8) return launch_rows<1>(p, stream);
     if (m <= 16) return launch_rows<2>(p, stream);

@@ -22,9 +22,10 @@ def linear_supported(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor |
 def prefers_own_kernel(rows: int, n: int, k: int) -> bool:
     """Where the kernels of ``csrc/linear.cu`` beat the library product inside a launch chain (a norm before each
     product, weights from HBM; us, library / this): up to 8 rows everywhere (2048 x 2048 9.8 / 5.2, 4096 x 12288
-    37.7 / 21.1); up to 16 rows also small outputs (4096 x 2048 7.7 / 7.5, but 12288 x 2048 12.8 / 13.6); up to 64 rows
-    long sums (4096 x 12288 26.9 / 24.1, 16384 x 4096 28.5 / 27.4, but 4096 x 2048 7.9 / 9.2), where the library cuts K
-    too little.  At 128 rows reading the activations once per weight tile costs more than it saves (7.6 / 14)."""
+    37.7 / 21.1; at worst even, 12288 x 2048 of 8 rows 13.2 / 13.4); up to 16 rows also small outputs (4096 x 2048
+    8.9 / 7.8, but 16384 x 2048 16.3 / 17.0); up to 64 rows long sums (4096 x 12288 28.7 / 24.9, 256 x 4096 10.6 / 8.0,
+    12288 x 4096 24.9 / 22.7, but 4096 x 2048 7.9 / 9.2), where the library cuts K too little.  At 128 rows reading the
+    activations once per weight tile costs more than it saves (7.6 / 14)."""
 
     return rows <= 8 or (rows <= 16 and n <= 4096) or (rows <= 64 and k >= 4096)
 

@@ -80,3 +80,19 @@ def test_weights_written_by_a_queued_kernel(m, n, k, device):
     for i in range(20):
         assert torch.equal(step(sources[i % 2], False), want[i % 2])
     assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("m,n,k,kernel", [(8, 4096, 2048, 1), (8, 2040, 4096, 2), (8, 680, 12288, 2), (16, 512, 2048, 1),
+                                          (16, 240, 4096, 2)])
+def test_which_kernel_takes_a_product(m, n, k, kernel, device):
+    """Long sums belong to the kernel that cuts K.  The two add in different orders, and the halves of every sum nearly
+    cancel, so the bits tell them apart."""
+
+    generator = torch.Generator(device=device).manual_seed(n)
+    x = torch.randn(m, k, generator=generator, device=device).bfloat16()
+    w = torch.randn(n, k, generator=generator, device=device).bfloat16()
+    w[:, k // 2:] = -w[:, :k // 2]
+    x[:, k // 2:] = x[:, :k // 2] * (1 + 2.0 ** -7)
+    status = torch.zeros(1, dtype=torch.int32, device=device)
+    picked, named, other = (linear(x, w, status=status, kernel=which) for which in (0, kernel, 3 - kernel))
+    assert torch.equal(picked, named) and not torch.equal(picked, other)
