@@ -10,13 +10,22 @@ MAX_ROWS = 128  # MIE_LINEAR_MAX_ROWS
 
 
 def linear_supported(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None) -> bool:
-    """Whether ``mie_linear`` takes the product: a few bf16 rows, 16-byte aligned, whole 16-byte groups."""
+    """Whether ``mie_linear`` takes the product: a few bf16 rows that do not overlap, 16-byte aligned, whole 16-byte
+    groups, nothing that autograd follows."""
 
-    return bool(x.dtype == weight.dtype == torch.bfloat16 and x.ndim == 2 and 0 < x.shape[0] <= MAX_ROWS
-                and x.is_cuda and x.shape[1] % 8 == 0 and x.stride(1) == weight.stride(1) == 1
+    if not (x.ndim == weight.ndim == 2 and 0 < x.shape[0] <= MAX_ROWS and x.dtype == weight.dtype == torch.bfloat16):
+        return False
+    (n, k), operands = weight.shape, [x, weight]
+    if bias is not None:
+        operands.append(bias)
+        if bias.dtype != torch.bfloat16 or tuple(bias.shape) != (n,) or not bias.is_contiguous():
+            return False
+    return bool(x.is_cuda and x.shape[1] == k and n > 0 and k > 0 and k % 8 == 0
+                and all(t.device == x.device for t in operands)
+                and x.stride(1) == weight.stride(1) == 1 and x.stride(0) >= k and weight.stride(0) >= k
                 and x.stride(0) % 8 == 0 and weight.stride(0) % 8 == 0
                 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
-                and (bias is None or (bias.dtype == torch.bfloat16 and bias.is_contiguous())))
+                and not (torch.is_grad_enabled() and any(t.requires_grad for t in operands)))
 
 
 def prefers_own_kernel(rows: int, n: int, k: int) -> bool:
@@ -35,8 +44,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     """``x [rows, k] @ weight [n, k]^T (+ bias)`` for weights that no queued kernel of this library writes (a model's
     parameters).  ``kernel``: 0 picks, 1 / 2 name one of the two kernels."""
 
+    if not linear_supported(x, weight, bias):
+        return torch.nn.functional.linear(x, weight, bias)
     (rows, k), n = x.shape, int(weight.shape[0])
-    if not linear_supported(x, weight, bias) or not (kernel or prefers_own_kernel(rows, n, k)):
+    if not (kernel or prefers_own_kernel(rows, n, k)):
         return torch.nn.functional.linear(x, weight, bias)
     out = torch.empty(rows, n, dtype=x.dtype, device=x.device)
     _lib.check(_lib.load().mie_linear(_lib.ptr(x), x.stride(0), _lib.ptr(weight), weight.stride(0), _lib.ptr(bias),

@@ -96,3 +96,29 @@ def test_which_kernel_takes_a_product(m, n, k, kernel, device):
     status = torch.zeros(1, dtype=torch.int32, device=device)
     picked, named, other = (linear(x, w, status=status, kernel=which) for which in (0, kernel, 3 - kernel))
     assert torch.equal(picked, named) and not torch.equal(picked, other)
+
+
+def test_whatever_the_library_product_takes(device):
+    """Shapes and strides that the kernels do not take: as ``torch.nn.functional.linear``, before and after."""
+
+    generator = torch.Generator(device=device).manual_seed(1)
+    x, w = (torch.randn(r, 64, generator=generator, device=device).bfloat16() for r in (4, 32))
+    bias, status = torch.randn(32, device=device).bfloat16(), torch.zeros(1, dtype=torch.int32, device=device)
+    for a, b, c in ((x.view(2, 2, 64), w, None), (x[0], w, bias), (x[:1].expand(3, 64), w, bias), (x, w[:1].expand(5, 64), None),
+                    (x, w[0], None), (x.t().contiguous().t(), w, None), (x, w[:0], None), (x[:, :0], w[:, :0], None),
+                    (x, w, bias.float().bfloat16().expand(32)), (x.as_strided((4, 64), (8, 1)), w, None)):
+        torch.testing.assert_close(linear(a, b, c, status=status), torch.nn.functional.linear(a, b, c))
+    weight = w.clone().requires_grad_()
+    linear(x, weight, bias, status=status).sum().backward()
+    torch.testing.assert_close(weight.grad, x.sum(0).expand(32, 64), rtol=2 ** -7, atol=2 ** -6)
+
+
+def test_operands_that_do_not_belong_together_are_refused(device):
+    """A weight of other columns (its rows would be read past their end), a bias of another length."""
+
+    x, w = torch.randn(4, 64, device=device).bfloat16(), torch.randn(32, 48, device=device).bfloat16()
+    status = torch.zeros(1, dtype=torch.int32, device=device)
+    for a, b, c in ((x, w, None), (x[:, :48], w, torch.zeros(31, device=device).bfloat16()), (x[:, :48], w.cpu(), None)):
+        assert not linear_supported(a, b, c)
+        with pytest.raises(RuntimeError):
+            linear(a, b, c, status=status)
