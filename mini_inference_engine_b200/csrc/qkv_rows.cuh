@@ -8,6 +8,7 @@
 namespace mie {
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+inline bool aligned8(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; }
 
 struct QkvParams {
   const __nv_bfloat16* qkv;  // [tokens][ld]: q heads | k heads | v heads
@@ -118,6 +119,7 @@ __device__ __forceinline__ void qkv_row_warp(const QkvParams& p, int t, int h, i
 // Host side: the cache (bf16 pages or the e4m3 pool), then everything else.
 inline int qkv_bf16_pages(QkvParams& p, const mie_view4_t& key_blocks, const mie_view4_t& value_blocks) {
   MIE_CHECK_ARG(key_blocks.ptr && value_blocks.ptr, "null pointer");
+  MIE_CHECK_ARG(aligned8(key_blocks.ptr) && aligned8(value_blocks.ptr), "pages must be 8-byte aligned");
   MIE_CHECK_ARG(key_blocks.stride[3] == 1 && value_blocks.stride[3] == 1, "pages must be contiguous in head_dim");
   for (int i = 0; i < 3; ++i) {
     MIE_CHECK_ARG(key_blocks.stride[i] % 4 == 0 && value_blocks.stride[i] % 4 == 0, "page strides must be multiples of 4");
@@ -135,8 +137,8 @@ inline int qkv_bf16_pages(QkvParams& p, const mie_view4_t& key_blocks, const mie
 inline int qkv_e4m3_pool(QkvParams& p, void* kv_pool, int64_t page_stride_bytes, float* kv_scales, int32_t kv_heads) {
   MIE_CHECK_ARG(kv_pool && kv_scales, "null pointer");
   MIE_CHECK_ARG(page_stride_bytes >= (long long)kv_heads * 4096 && page_stride_bytes % 4 == 0 &&
-                    (reinterpret_cast<uintptr_t>(kv_pool) & 3) == 0,
-                "the e4m3 pool needs a page stride of at least kv_heads * 4096 bytes");
+                    ((reinterpret_cast<uintptr_t>(kv_pool) | reinterpret_cast<uintptr_t>(kv_scales)) & 3) == 0,
+                "the e4m3 pool needs a page stride of at least kv_heads * 4096 bytes, pool and scales 4-byte alignment");
   p.key_blocks = p.value_blocks = nullptr;
   for (int i = 0; i < 3; ++i) p.kb_s[i] = p.vb_s[i] = 0;
   p.kv8_pool = (uint8_t*)kv_pool;
@@ -151,6 +153,8 @@ inline int qkv_common(QkvParams& p, const void* q_weight, const void* k_weight, 
                       int32_t block_size, int32_t num_blocks, int32_t table_rows, int32_t table_width, float eps,
                       int32_t* status) {
   MIE_CHECK_ARG(q_weight && k_weight && cos_sin && positions.ptr && block_tables.ptr && q_out, "null pointer");
+  MIE_CHECK_ARG(aligned8(q_weight) && aligned8(k_weight) && aligned8(cos_sin) && aligned8(q_out),
+                "norm weights, rotation table and query rows must be 8-byte aligned");
   MIE_CHECK_ARG(tokens >= 0 && q_heads >= 1 && kv_heads >= 1 && max_pos >= 1, "invalid shape");
   p.qkv = nullptr;
   p.ld = 0;

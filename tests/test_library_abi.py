@@ -84,3 +84,29 @@ def test_weights_are_requested_early_only_on_request(library):
 
     assert "MIE_GEMM_STATIC_WEIGHTS 2" in HEADER.read_text() and _lib.GEMM_STATIC_WEIGHTS == 2
     assert [gemm(flags) for flags in (0, 1, 2, 3, 4)] == [0, 0, 0, 0, -1]
+
+
+def test_misaligned_cache_writes_are_refused(library):
+    """The q/k/v rows are read and written eight bytes at a time; every operand is checked on the host (no rows here)."""
+
+    lib = _lib.load()
+    index = _lib.IndexT(4096, 0, 1, 1)
+
+    def view(address):
+        return _lib.View4T(address, (ctypes.c_int64 * 4)(2048, 2048, 128, 1))
+
+    def calls(norms=4096, rope=4096, queries=4096, pages=4096, pool=4096, scales=4096):
+        shared = (norms, norms, rope, 64, index, index, index, queries)
+        yield lib.mie_qkv_norm_rope_write(4096, 384, *shared, view(pages), view(4096), 0, 1, 1, 16, 1, 1, 1, 1e-6, None, None)
+        yield lib.mie_qkv_norm_rope_write_kv8(4096, 384, *shared, pool, 4096, scales, 0, 1, 1, 1, 1, 1, 1e-6, None, None)
+        product = (4096, 128, 4096, 1, 4096, 128, 4096, 1)
+        sizes = (0, 128, 1, 1, 16, 1, 1, 1, 1e-6, 0, 0, None, None)
+        yield lib.mie_fp8_gemm_qkv(*product, *shared, view(pages), view(4096), None, 0, None, *sizes)
+        yield lib.mie_fp8_gemm_qkv(*product, *shared, view(4096), view(4096), pool, 4096, scales, *sizes)
+
+    assert list(calls()) == [0, 0, 0, 0]
+    for name in ("norms", "rope", "queries"):
+        assert list(calls(**{name: 4096 + 2})) == [-1, -1, -1, -1], name
+    assert list(calls(pages=4096 + 4)) == [-1, 0, -1, 0]
+    for name in ("pool", "scales"):
+        assert list(calls(**{name: 4096 + 2})) == [0, -1, 0, -1], name
