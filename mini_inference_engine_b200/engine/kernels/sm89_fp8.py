@@ -34,7 +34,7 @@ SUPPORTED_BLOCK_SIZE = (128, 128)
 MAX_M_BUCKET = 16384
 SPLIT_M_THRESHOLD = 256
 QUANT_BLOCK_M = 16
-FINISH_MIN_WEIGHT = 1 << 22  # bytes
+FINISH_MIN_WEIGHT = (1 << 20) + 1  # bytes
 
 
 @dataclass(frozen=True)
@@ -233,12 +233,13 @@ def launch_fp8_gemm(quantized: torch.Tensor, scales_kmajor: torch.Tensor, weight
 
 def finishes_rows(weight: torch.Tensor, m: int) -> bool:
     """Whether the product of ``m`` tokens with ``weight`` can finish its own rows (``mie_fp8_gemm_silu`` / ``_qkv``):
-    a decode batch, and a weight that the GEMM reads in place.  Weights under 4 MiB keep the separate launches, and the
-    launch count that describes them: two layers of width 512 take 77 to 79 us at one token and 87 to 90 at 16 either way
-    (36 layers of width 2560: 1915 us separate, 1796 finished)."""
+    a decode batch, and a weight that the GEMM reads in place.  It saves a launch and a trip of the rows for every weight
+    (product and what follows it, one token: gate_up 768 x 2560 5.9 us separate, 4.9 finished, 1024 x 512 5.4 and 4.3; 36
+    layers of width 2560 1915 and 1796).  Weights of at most 1 MiB, which only models made for tests have, keep the separate
+    launches and the ten launches a layer that their steps report (two layers of width 512 77 to 79 us either way)."""
 
-    return (weight.numel() >= FINISH_MIN_WEIGHT and weight.stride(1) == 1 and weight.stride(0) % 16 == 0 and weight.data_ptr() % 16 == 0
-            and bool(_lib.load().mie_fp8_gemm_finishes(m, int(weight.shape[0]))))
+    return (weight.numel() >= FINISH_MIN_WEIGHT and weight.stride(1) == 1 and weight.stride(0) % 16 == 0
+            and weight.data_ptr() % 16 == 0 and bool(_lib.load().mie_fp8_gemm_finishes(m, int(weight.shape[0]))))
 
 
 def default_max_split() -> int:
