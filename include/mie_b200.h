@@ -351,8 +351,13 @@ int mie_fp8_gemm(const void* x8, int64_t ldx, const float* a_scale, int32_t a_sc
  * mie_fp8_gemm_qkv: w8 holds [q | k | v] heads of 128 rows; what follows the
  * product is mie_qkv_norm_rope_write, or with kv_pool (then block_size is 16
  * and the page views are not read) mie_qkv_norm_rope_write_kv8.
+ *
+ * mie_fp8_gemm_finish_pays: whether that one launch is also the faster way for
+ * m tokens of an [n, k] weight (gated = 1: mie_fp8_gemm_silu with n = 2 cols;
+ * gated = 0: mie_fp8_gemm_qkv); 0 wherever mie_fp8_gemm_finishes is.
  */
 int mie_fp8_gemm_finishes(int32_t m, int32_t n);
+int mie_fp8_gemm_finish_pays(int32_t m, int32_t n, int32_t k, int32_t gated, int32_t max_split);
 int mie_fp8_gemm_silu(const void* x8, int64_t ldx, const float* a_scale, int32_t a_scale_ld, const void* w8,
                       int64_t ldw, const float* w_scale, int32_t w_scale_ld, void* q, int64_t ldq, float* scales,
                       int32_t scale_ld, int32_t m, int32_t cols, int32_t k, int32_t max_split, int32_t flags,

@@ -109,6 +109,7 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "mie_fp8_quantize": (ctypes.c_int, [c_void_p, c_int64, c_int32, c_void_p, c_int64, c_void_p, c_int32, c_int32,
                                         c_int32, c_void_p]),
     "mie_fp8_gemm_finishes": (ctypes.c_int, [c_int32, c_int32]),
+    "mie_fp8_gemm_finish_pays": (ctypes.c_int, [c_int32, c_int32, c_int32, c_int32, c_int32]),
     "mie_fp8_gemm_silu": (ctypes.c_int, [c_void_p, c_int64, c_void_p, c_int32, c_void_p, c_int64, c_void_p, c_int32,
                                          c_void_p, c_int64, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32,
                                          c_int32, c_void_p, c_void_p]),

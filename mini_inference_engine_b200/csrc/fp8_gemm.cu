@@ -1037,6 +1037,30 @@ bool narrow_fits(int m, int n) {
   return m <= 32 || (m <= 128 && (n + kTileR - 1) / kTileR <= sm_count());
 }
 
+// Whether finishing the rows in the projection beats storing them for a second kernel.  It saves about 1.1 us of launch and
+// reading, but a CTA finishes its share of the tokens alone, and gate and up rows of a tile take two CTAs of the cluster,
+// which leaves K half as many parts.  Measured (us, separate / finished):
+//   q/k/v   up to 32 tokens everywhere (1 token of 6144 x 2560 8.6 / 7.3); then only with K cut, so that several CTAs share
+//           the tokens: 64 tokens of 3072 x 2560 in 2 parts or more 10.4 / 8.6, of 6144 x 512 uncut 8.6 / 10.4; 128 tokens
+//           of 1536 x 2560 in 4 parts 11.8 / 11.4, of 6144 x 4096 in 2 18.9 / 19.7.
+//   gated   up to 32 tokens (1 token of 9728 x 2560 10.1 / 8.8) unless the halved split shows (1024 x 8192 7.5 / 8.0) or its
+//           clusters of four nearly fill the GPU and not all find room at once (18688 x 4096 16.9 / 22.1); then with K cut
+//           into as many parts as without (64 tokens of 6144 x 4096 12.6 / 11.6, of 2048 x 4096 9.5 / 10.5) or, up to 64
+//           tokens, short (1536 x 1024 7.5 / 6.9); above 64 not of a short uncut K (1024 x 512 8.5 / 10.7; 12288 x 2048
+//           19.0 / 18.1).
+bool finish_pays(int m, int n, int k, bool gated, int max_split) {
+  if (!narrow_fits(m, n)) return false;
+  const int bn = swap_bn(m), per_sm = m <= 32 ? 2 : 1, limit = m <= 32 ? 8 : 4;
+  const int tiles = (n + kTileR - 1) / kTileR, kb = (k + kBlockK - 1) / kBlockK;
+  const int stored = choose_split(tiles, kb, bn, per_sm, max_split, limit);
+  if (!gated) return m <= 32 || stored >= (m <= 64 ? 2 : 4);
+  const int split = choose_split(tiles, kb, bn, per_sm, max_split, limit / 2);
+  if (split > 1 && tiles * split > per_sm * sm_count() * 9 / 10) return false;
+  if (m <= 32) return split == stored || kb < 64;
+  if (m <= 64) return split == stored || kb <= 8;
+  return split == stored && (split > 1 || kb >= 16);
+}
+
 // Schedule of the wide kernel.  `tiles` output tiles of `kb` K blocks on P SMs (one 200 KB CTA each):
 //   tiles <= P      one launch; whole tiles, or one tile per 2-/4-CTA cluster with the K range cut when all
 //                   clusters still fit one wave;
@@ -1208,6 +1232,10 @@ extern "C" int mie_fp8_gemm(const void* x8, int64_t ldx, const float* a_scale, i
 }
 
 extern "C" int mie_fp8_gemm_finishes(int32_t m, int32_t n) { return m >= 1 && n >= 1 && narrow_fits(m, n) ? 1 : 0; }
+
+extern "C" int mie_fp8_gemm_finish_pays(int32_t m, int32_t n, int32_t k, int32_t gated, int32_t max_split) {
+  return m >= 1 && n >= 1 && k >= 1 && finish_pays(m, n, k, gated != 0, max_split) ? 1 : 0;
+}
 
 extern "C" int mie_fp8_gemm_silu(const void* x8, int64_t ldx, const float* a_scale, int32_t a_scale_ld, const void* w8,
                                  int64_t ldw, const float* w_scale, int32_t w_scale_ld, void* q, int64_t ldq,

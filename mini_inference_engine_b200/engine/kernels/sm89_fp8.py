@@ -231,15 +231,16 @@ def launch_fp8_gemm(quantized: torch.Tensor, scales_kmajor: torch.Tensor, weight
     ))
 
 
-def finishes_rows(weight: torch.Tensor, m: int) -> bool:
-    """Whether the product of ``m`` tokens with ``weight`` can finish its own rows (``mie_fp8_gemm_silu`` / ``_qkv``):
-    a decode batch, and a weight that the GEMM reads in place.  It saves a launch and a trip of the rows for every weight
-    (product and what follows it, one token: gate_up 768 x 2560 5.9 us separate, 4.9 finished, 1024 x 512 5.4 and 4.3; 36
-    layers of width 2560 1915 and 1796).  Weights of at most 1 MiB, which only models made for tests have, keep the separate
-    launches and the ten launches a layer that their steps report (two layers of width 512 77 to 79 us either way)."""
+def finishes_rows(weight: torch.Tensor, m: int, *, gated: bool) -> bool:
+    """Whether the product of ``m`` tokens with ``weight`` should finish its own rows (``mie_fp8_gemm_silu`` when ``gated``,
+    else ``mie_fp8_gemm_qkv``): where that is faster, for a weight that the GEMM reads in place.  Weights of at most 1 MiB,
+    which only models made for tests have, keep the separate launches and the ten launches a layer that their steps report
+    (two layers of width 512 77 to 79 us either way)."""
 
     return (weight.numel() >= FINISH_MIN_WEIGHT and weight.stride(1) == 1 and weight.stride(0) % 16 == 0
-            and weight.data_ptr() % 16 == 0 and bool(_lib.load().mie_fp8_gemm_finishes(m, int(weight.shape[0]))))
+            and weight.data_ptr() % 16 == 0
+            and bool(_lib.load().mie_fp8_gemm_finish_pays(m, int(weight.shape[0]), int(weight.shape[1]), int(gated),
+                                                          _DEFAULT_MAX_SPLIT)))
 
 
 def default_max_split() -> int:

@@ -390,7 +390,7 @@ class Qwen3DecodeRunner(PagedStepRunner):
         """The merged gate_up projection and SiLU(gate) * up, quantised for down_proj: one launch for a decode batch."""
 
         weight, inter = layer.gate_up, self.local_inter
-        if not sm89_fp8.finishes_rows(weight, rows):
+        if not sm89_fp8.finishes_rows(weight, rows, gated=True):
             return self._silu_mul_quantized(self._gemm(quantized, weight, layer.gate_up_scale, rows, self.shape.hidden),
                                             rows)
         q, scales = self._quant_buffers(rows, inter)
@@ -445,7 +445,7 @@ class Qwen3DecodeRunner(PagedStepRunner):
         """The merged q/k/v projection and ``_qkv_post``: one launch for a decode batch."""
 
         shape, weight = self.shape, layer.qkv
-        if not sm89_fp8.finishes_rows(weight, tokens):
+        if not sm89_fp8.finishes_rows(weight, tokens, gated=False):
             qkv = self._gemm(quantized, weight, layer.qkv_scale, tokens, shape.hidden)
             self._qkv_post(layer_index, layer, qkv, queries, positions, token_to_sequence, block_tables, tokens,
                            table_rows)

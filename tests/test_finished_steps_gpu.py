@@ -1,5 +1,5 @@
 """Whole steps whose projections finish their own rows, as real models' do: the tests of the small models, whose weights
-otherwise keep the separate launches, once more with the size bound taken away."""
+otherwise keep the separate launches, once more with every product that can finishing its rows."""
 
 from __future__ import annotations
 
@@ -18,11 +18,12 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture()
 def finished(monkeypatch):
-    """No size bound; afterwards, every product that can finish its rows must have been asked to, and both must have."""
+    """Rows are finished wherever that is possible; afterwards both kinds must have been, equally often."""
 
-    monkeypatch.setattr(sm89_fp8, "FINISH_MIN_WEIGHT", 0)
     taken = {"mie_fp8_gemm_silu": 0, "mie_fp8_gemm_qkv": 0}
     lib = _lib.load()
+    monkeypatch.setattr(sm89_fp8, "finishes_rows",
+                        lambda weight, m, *, gated: bool(lib.mie_fp8_gemm_finishes(m, int(weight.shape[0]))))
     for name in taken:
         def counting(*args, _name=name, _call=getattr(lib, name)):
             taken[_name] += 1

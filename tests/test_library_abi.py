@@ -110,3 +110,18 @@ def test_misaligned_cache_writes_are_refused(library):
     assert list(calls(pages=4096 + 4)) == [-1, 0, -1, 0]
     for name in ("pool", "scales"):
         assert list(calls(**{name: 4096 + 2})) == [0, -1, 0, -1], name
+
+
+@pytest.mark.parametrize("gated,n,k,tokens", [
+    # (weight, token counts at which the finished projection measured faster by more than 2 %, and where slower)
+    (0, 6144, 2560, {1: 1, 32: 1, 48: 1, 128: 0}), (0, 6144, 512, {1: 1, 32: 1, 64: 0, 65: 0}),
+    (0, 1536, 2560, {17: 1, 64: 1, 96: 1}), (0, 10240, 4096, {1: 1, 33: 0, 128: 0}), (0, 4096, 1024, {1: 1, 64: 1, 128: 1}),
+    (1, 19456, 2560, {1: 1, 32: 1, 33: 0, 128: 0}), (1, 18688, 4096, {1: 0, 32: 0, 64: 1}),
+    (1, 1024, 8192, {1: 0, 32: 0, 64: 0, 128: 0}), (1, 6144, 4096, {1: 1, 64: 1, 128: 1}),
+    (1, 1536, 1024, {1: 1, 64: 1, 65: 0, 128: 0}), (1, 2048, 4096, {1: 1, 32: 1, 48: 0, 96: 0}),
+    (1, 4864, 2560, {1: 1, 33: 1, 128: 1})])
+def test_where_finished_projections_pay(library, gated, n, k, tokens):
+    lib = _lib.load()
+    for m, pays in tokens.items():
+        assert lib.mie_fp8_gemm_finish_pays(m, n, k, gated, 0) == pays, (m, n, k)
+    assert lib.mie_fp8_gemm_finish_pays(129, n, k, gated, 0) == 0 and lib.mie_fp8_gemm_finish_pays(0, n, k, gated, 0) == 0
