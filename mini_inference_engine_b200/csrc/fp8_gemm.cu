@@ -115,21 +115,6 @@ struct GemmSmem {
   static_assert(kStages * kStageBytes >= BN * kTileR * 4, "the stage ring also parks the fp32 rows");
 };
 
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_addr, uint32_t rank) {
-  uint32_t remote;
-  float4 v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(remote)
-               : "memory");
-  return v;
-}
-
 // Four outputs of a token from weight row n0 of the narrow kernel.
 __device__ __forceinline__ void store_row4(const GemmParams& p, int tok, int n0, const float (&v)[4], bool vec) {
   uint16_t* dst = reinterpret_cast<uint16_t*>(p.y) + (long long)tok * p.ldy + n0;
@@ -850,7 +835,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
 // --------------------------------------------------------------------------
 // Activation quantiser: per token, per 128 columns.  One half-warp per group, eight columns a lane.  Bound by HBM (3
 // bytes a value) with the quotients by corrected_quotient and 32-bit indices; with IEEE divisions and a 64-bit index
-// division it was bound by instructions (12032 x 4096: 50.3 us, now 39.6 us).
+// division it was bound by instructions (12032 x 4096: 52.4 us, now 39.7 us).
 // --------------------------------------------------------------------------
 template <typename T, typename Index>
 __global__ void quantize_kernel(const T* __restrict__ x, long long ldx, uint8_t* __restrict__ q, long long ldq,

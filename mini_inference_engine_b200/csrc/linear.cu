@@ -209,19 +209,6 @@ struct TileSmem {
   static_assert(kStages * kStageBytes >= kTileRows * BN * 4, "the ring also parks the fp32 sums");
 };
 
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_addr, uint32_t rank) {
-  uint32_t remote;
-  float4 v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(remote)
-               : "memory");
-  return v;
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
 // Rank r of a cluster adds the tokens of its slice over the sums that every CTA has parked ([token][row]), in rank
 // order.  A warp takes a token, a lane four weight rows; the loads of several tokens from all ranks are in flight
 // together.
@@ -400,8 +387,7 @@ __global__ void __launch_bounds__(kTileThreads, TileSmem<BN>::kCtasPerSm)
         asm volatile("st.shared.f32 [%0], %1;" ::"r"(park + (uint32_t)((j * kTileRows + row) * 4)), "f"(acc[j])
                      : "memory");
     }
-    cluster_arrive();
-    cluster_wait();
+    cluster_sync_all();
     if (warp < 4) {
       if (split == 2)
         reduce_slice<2>(p, park, rank, tile, warp, lane);
@@ -411,8 +397,7 @@ __global__ void __launch_bounds__(kTileThreads, TileSmem<BN>::kCtasPerSm)
         reduce_slice<8>(p, park, rank, tile, warp, lane);
     }
     __syncwarp();
-    cluster_arrive();  // no CTA leaves while a peer may still read its sums
-    cluster_wait();
+    cluster_sync_all();  // no CTA leaves while a peer may still read its sums
   }
   tc_fence_before();
   __syncthreads();
