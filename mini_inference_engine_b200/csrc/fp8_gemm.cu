@@ -1028,11 +1028,11 @@ bool narrow_fits(int m, int n) {
 //   q/k/v   up to 32 tokens everywhere (1 token of 6144 x 2560 8.6 / 7.3); then only with K cut, so that several CTAs share
 //           the tokens: 64 tokens of 3072 x 2560 in 2 parts or more 10.4 / 8.6, of 6144 x 512 uncut 8.6 / 10.4; 128 tokens
 //           of 1536 x 2560 in 4 parts 11.8 / 11.4, of 6144 x 4096 in 2 18.9 / 19.7.
-//   gated   up to 32 tokens (1 token of 9728 x 2560 10.1 / 8.8, of 19456 x 2560 13.1 / 12.7) unless the halved split shows (1024 x 8192 7.5 / 8.0) or its
-//           clusters of four nearly fill the GPU and not all find room at once (18688 x 4096 16.9 / 22.1); then with K cut
-//           into as many parts as without (64 tokens of 6144 x 4096 12.6 / 11.6, of 2048 x 4096 9.5 / 10.5) or, up to 64
-//           tokens, short (1536 x 1024 7.5 / 6.9); above 64 not of a short uncut K (1024 x 512 8.5 / 10.7; 12288 x 2048
-//           19.0 / 18.1).
+//   gated   up to 32 tokens (1 token of 9728 x 2560 10.1 / 8.8, of 19456 x 2560 13.1 / 12.7) unless the halved split shows
+//           (1024 x 8192 7.5 / 8.0) or its clusters of four nearly fill the GPU and not all find room at once (18688 x 4096
+//           16.9 / 22.1); then with K cut into as many parts as without (64 tokens of 6144 x 4096 12.6 / 11.6, of
+//           2048 x 4096 9.5 / 10.5) or, up to 64 tokens, short (1536 x 1024 7.5 / 6.9); above 64 not of a short uncut K
+//           (1024 x 512 8.5 / 10.7; 12288 x 2048 19.0 / 18.1).
 bool finish_pays(int m, int n, int k, bool gated, int max_split) {
   if (!narrow_fits(m, n)) return false;
   const int bn = swap_bn(m), per_sm = m <= 32 ? 2 : 1, limit = m <= 32 ? 8 : 4;
