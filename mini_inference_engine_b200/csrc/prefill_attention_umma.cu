@@ -69,24 +69,6 @@ bool pages_fit_slab_map(const mie_view4_t& v, int block_size, int dim) {
 namespace {
 
 constexpr int kDim = 128;
-constexpr int kSmemBytes = PrefillTile<2, 2>::kSmemBytes;
-
-template <typename T>
-int launch_umma(const CUtensorMap& kmap, const CUtensorMap& vmap,
-                const UmmaPrefillParams& p, int q_tiles, cudaStream_t stream) {
-  static bool configured[64] = {false};
-  int dev = 0;
-  MIE_CUDA(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < 64 && !configured[dev]) {
-    MIE_CUDA(cudaFuncSetAttribute(prefill_umma_kernel<T, 2, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    configured[dev] = true;
-  }
-  dim3 grid((unsigned)q_tiles, (unsigned)p.requests, (unsigned)p.kv_heads);
-  prefill_umma_kernel<T, 2, 2, false><<<grid, kThreads, kSmemBytes, stream>>>(kmap, vmap, p, q_tiles);
-  MIE_LAUNCH_CHECK("prefill_umma_kernel");
-  return MIE_OK;
-}
-
 }  // namespace
 
 // Returns MIE_ERR_UNSUPPORTED (without an error message) when the shape does not fit this kernel, so the
@@ -104,17 +86,14 @@ int prefill_attention_umma(const void* query, long long q_st, long long q_sh, lo
   if (total_tokens <= 0 || !(scale > 0.f)) return MIE_ERR_UNSUPPORTED;
   if (!pages_fit_slab_map(key_blocks, block_size, kDim) || !pages_fit_slab_map(value_blocks, block_size, kDim))
     return MIE_ERR_UNSUPPORTED;
-  if ((long long)table_width * block_size / kSub + kKv / kSub > kMaxIds) return MIE_ERR_UNSUPPORTED;
   CUtensorMap kmap, vmap;
   if (int rc = page_slab_map(key_blocks, num_blocks, kv_heads, block_size, kDim, 2, dtype, &kmap)) return rc;
   if (int rc = page_slab_map(value_blocks, num_blocks, kv_heads, block_size, kDim, 2, dtype, &vmap)) return rc;
   UmmaPrefillParams p{(const char*)query, q_st, q_sh, (char*)out, o_st, o_sh, IndexView(block_tables), IndexView(cu_seqlens), IndexView(kv_lens),
                       requests, q_heads, kv_heads, group, block_size, num_blocks, table_width,
                       scale * 1.4426950408889634f, status, kDim, kDim, 1, 1, 1, 0, nullptr};
-  const int tok_per_tile = kRows / group;
-  const int q_tiles = (max_query_len + tok_per_tile - 1) / tok_per_tile;
-  if (dtype == MIE_DTYPE_BF16) return launch_umma<__nv_bfloat16>(kmap, vmap, p, q_tiles, stream);
-  return launch_umma<__half>(kmap, vmap, p, q_tiles, stream);
+  if (dtype == MIE_DTYPE_BF16) return launch_prefill<__nv_bfloat16, 2, 2, false>(kmap, vmap, p, total_tokens, max_query_len, stream);
+  return launch_prefill<__half, 2, 2, false>(kmap, vmap, p, total_tokens, max_query_len, stream);
 }
 
 }  // namespace mie

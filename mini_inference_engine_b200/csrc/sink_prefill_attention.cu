@@ -11,30 +11,11 @@ int page_tensor_map(const mie_view4_t& pages, int num_blocks, int kv_heads, int 
 
 namespace {
 
-template <int KH, int VH>
-int launch_sink_prefill(const CUtensorMap& kmap, const CUtensorMap& vmap, const UmmaPrefillParams& p, int q_tiles,
-                        cudaStream_t stream) {
-  using T = __nv_bfloat16;
-  using Tile = PrefillTile<KH, VH>;
-  static bool configured[64] = {false};
-  int dev = 0;
-  MIE_CUDA(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < 64 && !configured[dev]) {
-    MIE_CUDA(cudaFuncSetAttribute(prefill_umma_kernel<T, KH, VH, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  Tile::kSmemBytes));
-    configured[dev] = true;
-  }
-  dim3 grid((unsigned)q_tiles, (unsigned)p.requests, (unsigned)(p.kv_heads * p.v_passes));
-  prefill_umma_kernel<T, KH, VH, true><<<grid, kThreads, Tile::kSmemBytes, stream>>>(kmap, vmap, p, q_tiles);
-  MIE_LAUNCH_CHECK("prefill_umma_kernel");
-  return MIE_OK;
-}
-
 template <int KH>
 int launch_sink_prefill_v(int vh, const CUtensorMap& kmap, const CUtensorMap& vmap, const UmmaPrefillParams& p,
-                          int q_tiles, cudaStream_t stream) {
-  return vh == 1 ? launch_sink_prefill<KH, 1>(kmap, vmap, p, q_tiles, stream)
-                 : launch_sink_prefill<KH, 2>(kmap, vmap, p, q_tiles, stream);
+                          long long tokens, int max_query_len, cudaStream_t stream) {
+  return vh == 1 ? launch_prefill<__nv_bfloat16, KH, 1, true>(kmap, vmap, p, tokens, max_query_len, stream)
+                 : launch_prefill<__nv_bfloat16, KH, 2, true>(kmap, vmap, p, tokens, max_query_len, stream);
 }
 
 int page_map(const mie_view4_t& pages, int num_blocks, int kv_heads, int block_size, int dim, int box_groups, bool slab,
@@ -94,12 +75,11 @@ extern "C" int mie_sink_prefill_attention(const void* query, int64_t q_token_str
                       IndexView(block_tables), IndexView(cu_seqlens), IndexView(kv_lens), requests, q_heads, kv_heads,
                       group, block_size, num_blocks, table_width, scale * 1.4426950408889634f, status, dim, value_dim,
                       (value_dim + vh * 64 - 1) / (vh * 64), k_slab ? 1 : 0, v_slab ? 1 : 0, window, sinks};
-  const int tokens_per_tile = kRows / group;
-  const int q_tiles = (max_query_len + tokens_per_tile - 1) / tokens_per_tile;
+  const long long tokens = (long long)requests * max_query_len;  // at most
   switch (kh) {
-    case 1: return launch_sink_prefill_v<1>(vh, kmap, vmap, p, q_tiles, stream);
-    case 2: return launch_sink_prefill_v<2>(vh, kmap, vmap, p, q_tiles, stream);
-    case 3: return launch_sink_prefill_v<3>(vh, kmap, vmap, p, q_tiles, stream);
-    default: return launch_sink_prefill_v<4>(vh, kmap, vmap, p, q_tiles, stream);
+    case 1: return launch_sink_prefill_v<1>(vh, kmap, vmap, p, tokens, max_query_len, stream);
+    case 2: return launch_sink_prefill_v<2>(vh, kmap, vmap, p, tokens, max_query_len, stream);
+    case 3: return launch_sink_prefill_v<3>(vh, kmap, vmap, p, tokens, max_query_len, stream);
+    default: return launch_sink_prefill_v<4>(vh, kmap, vmap, p, tokens, max_query_len, stream);
   }
 }

@@ -1,0 +1,49 @@
+"""Prefill attention where a cluster shares a pair of query tiles (its K/V tiles, or one query tile each)."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from mini_inference_engine_b200 import workloads
+from test_prefill_attention_gpu import ATOL, _oracle, _run
+from test_sink_attention_gpu import Case
+
+pytestmark = pytest.mark.gpu
+
+# prefixes, chunks, query and key/value heads: six and eight ranks for one query tile; two ranks beside a request with too
+# few tiles; the first tile count that is shared (eight) and the last that is not; a rank per query tile; query tiles that
+# end in different K/V tiles; groups of 1, 2 and 8 heads.
+SHARED = [
+    ((3000,), (16,), 32, 8), ((4100,), (1,), 8, 2), ((1673, 375), (386, 126), 32, 8), ((992, 960), (32, 64), 8, 2),
+    ((500, 0), (100, 97), 32, 8), ((1500,), (300,), 8, 8), ((2040,), (129,), 4, 2), ((900, 1500), (33, 200), 8, 1),
+]
+
+
+@pytest.mark.parametrize("shape", SHARED, ids=str)
+def test_ranks_of_a_pair(shape, device, status_clean):
+    """Bound as for the unshared kernel: bf16 probabilities and outputs of unit values."""
+
+    prefixes, chunks, heads, kv_heads = shape
+    case = workloads.prefill_case(seed=11, prefix_lengths=prefixes, chunk_lengths=chunks, q_heads=heads,
+                                  kv_heads=kv_heads)
+    _, _, expected = _oracle(case)
+    _, out = _run(case, device)
+    assert (out.float() - expected.float()).abs().max().item() <= ATOL
+
+
+# length and new tokens of each request; heads, key/value heads, dim, vdim, window; sinks.
+WIDE = [
+    ([(2500, 40), (1200, 130)], (8, 2, 128, 128, None), "random"), ([(2500, 40)], (4, 4, 192, 128, None), "large"),
+    ([(2600, 90)], (8, 2, 128, 128, 1024), "none"), ([(1400, 300)], (4, 2, 64, 64, 1100), "random"),
+    ([(1500, 20)], (2, 1, 72, 200, None), "zeros"), ([(1300, 260)], (3, 3, 256, 256, 1030), "random"),
+]
+
+
+@pytest.mark.parametrize("spans,sizes,sinks", WIDE, ids=str)
+def test_ranks_with_sinks_and_windows(spans, sizes, sinks, device):
+    """Only the first rank counts the sink; a rank may see no key of a windowed row."""
+
+    case = Case([n for n, _ in spans], [c for _, c in spans], *sizes, 16, torch.bfloat16, seed=12, sinks=sinks)
+    case.prefill(device)
+    case.check()
