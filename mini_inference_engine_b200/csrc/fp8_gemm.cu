@@ -65,6 +65,7 @@ struct GemmParams {
   // early_release: the next launch may start before this one's wait (not when it is the second launch of a
   // two-launch GEMM, which takes the first one's wait for its own).
   int tile_begin, tile_end, late_wait, early_release;
+  int band;  // wide kernel: token tiles per band (see wide_item)
   // Finish::kSilu: the quantised result (y is not written).
   uint8_t* q;
   long long ldq;
@@ -448,12 +449,17 @@ __global__ void __launch_bounds__(kNarrowThreads<BN>, GemmSmem<BN>::kCtasPerSm)
 //     in rank order (a fixed order: results do not depend on timing) and stores bf16.  No global scratch.
 //   * Two 256-column accumulators ping-pong in TMEM, each with its own MMA issuer thread, and a K block has one
 //     commit, on the barrier that both frees its stage and hands its accumulator over: one thread's wait, four MMAs
-//     and commit take about 770 cycles, the MMAs 512 (two issuers measured 512 with nothing to promote).
+//     and commit take about 770 cycles, the MMAs 512 (two issuers measured 512 with nothing to promote).  An issuer has
+//     the operands' barrier behind it and its descriptors at hand when the accumulator comes back.
 //   * 20 warps: 16 promotion warps, one TMA producer, two MMA issuers, one idle.  A promotion warp keeps 32 rows x 64
 //     columns of the fp32 result in registers and adds a K block in two loads of 32 columns (packed fp32x2
 //     multiply-adds); four warps per scheduler hide the loads' latency (eight warps with 128 columns each and the
 //     loads pipelined by hand: 4736 x 19456 x 2560 307 us, sixteen 264).  The accumulator goes back to its issuer
-//     as soon as the second load has landed.  A thread requests its row's scale one K block ahead.
+//     as soon as the second load has landed.  A thread requests its row's scale one K block ahead, unconditionally (dead
+//     rows and columns read scales that nothing is stored from): under a condition the loads were waited for on the spot.
+//     With the issuers' order, 560 x 19456 x 2560 43.9 -> 38.9 us, 4736 tokens 256 -> 242, 12032 687 -> 622.
+//   * What bounds it now, 4736 x 19456 x 2560 (242 us): 174 us without operand loads and promotion, 212 with the promotion,
+//     208 with the loads: MMA operand reads and TMA writes share 128 bytes a clock of shared memory.
 //   * A pair of CTAs on one 256 x 256 tile (cta_group::2, a third less operand traffic) measured 3 % faster at 12032
 //     tokens and up to 20 % slower at a few hundred, where its tiles leave more rows empty.
 // --------------------------------------------------------------------------
@@ -474,15 +480,20 @@ struct WideItem {
   int tm, tn, k0, k1;
 };
 
-// Work of CTA (x, rank) of a (gridDim.x, split) grid over the tiles [first, tiles).  split == 1: tiles
+// Work of CTA (x, rank) of a (gridDim.x, split) grid over the launch's tiles.  split == 1: tiles
 // first + x, first + x + gridDim.x, ... whole.  split > 1 (one cluster per tile): tile first + x, the
-// rank-th part of its K range.
-__device__ __forceinline__ bool wide_item(int first, int tiles, int tiles_m, int kb_total, int split, int rank,
-                                          int idx, WideItem& it) {
-  const int tile = first + (int)blockIdx.x + idx * (int)gridDim.x;
-  if (tile >= tiles || (split > 1 && idx > 0)) return false;
-  it.tm = tile % tiles_m;
-  it.tn = tile / tiles_m;
+// rank-th part of its K range.  Tiles are numbered down the token tiles of a band, then along the weight tiles, then band
+// by band (band: see wide_band).
+__device__ __forceinline__ bool wide_item(const GemmParams& p, int idx, WideItem& it) {
+  const int tile = p.tile_begin + (int)blockIdx.x + idx * (int)gridDim.x;
+  const int split = gridDim.y, rank = blockIdx.y;
+  if (tile >= p.tile_end || (split > 1 && idx > 0)) return false;
+  const int tiles_m = (p.m + kTileR - 1) / kTileR, tiles_n = (p.n + kWideBN - 1) / kWideBN;
+  const int kb_total = (p.k + kBlockK - 1) / kBlockK;
+  const int band = tile / (p.band * tiles_n), in_band = tile - band * p.band * tiles_n;
+  const int rows = tiles_m - band * p.band < p.band ? tiles_m - band * p.band : p.band;
+  it.tn = in_band / rows;
+  it.tm = band * p.band + in_band - it.tn * rows;
   it.k0 = (int)((long long)kb_total * rank / split);
   it.k1 = (int)((long long)kb_total * (rank + 1) / split);
   return true;
@@ -500,6 +511,15 @@ __device__ __forceinline__ void tmem_ld_wait_pin(float (&a)[32]) {
                  "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
                :
                : "memory");
+}
+
+// Token tiles per band: all when the activations take less than about a quarter of L2, else equal bands of less.  12032 x
+// 2560 x 9728 (117 MB of activations, read again for every column of tiles): 320 us as one band, 284 in bands of 20;
+// 4736 x 19456 x 2560 (12 MB): 242 as one, 248 in bands of 20 (fewer CTAs at the same weights).
+inline int wide_band(int m, int k) {
+  const int tiles_m = (m + kTileR - 1) / kTileR;
+  const int bands = (int)(((long long)m * k + (32 << 20) - 1) / (32 << 20));
+  return (tiles_m + bands - 1) / bands;
 }
 
 // acc[0..32) += d[0..32) * s, two columns per instruction.
@@ -585,9 +605,6 @@ __global__ void __launch_bounds__(kWideThreads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + kAcc);
 
   const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
-  const int kb_total = (p.k + kBlockK - 1) / kBlockK;
-  const int tiles_m = (p.m + kTileR - 1) / kTileR;
-  const int tiles = p.tile_end;
   const int split = gridDim.y, rank = blockIdx.y;  // cluster = (1, split, 1)
 
   if (threadIdx.x == 0) {
@@ -621,7 +638,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
   uint32_t prefetched = 0;
   if (p.prefetch && warp == E && lane == 0) {
     WideItem first;
-    if (wide_item(p.tile_begin, tiles, tiles_m, kb_total, split, rank, 0, first)) {
+    if (wide_item(p, 0, first)) {
       for (int kb = first.k0; kb < first.k1 && prefetched < (uint32_t)kStages; ++kb, ++prefetched) {
         mbar_expect_tx(&full_bar[prefetched], kStageBytes);
         load_w(prefetched, kb, first);
@@ -636,7 +653,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
   uint32_t total_blocks = 0;
   {
     WideItem it;
-    for (int idx = 0; wide_item(p.tile_begin, tiles, tiles_m, kb_total, split, rank, idx, it); ++idx)
+    for (int idx = 0; wide_item(p, idx, it); ++idx)
       total_blocks += (uint32_t)(it.k1 - it.k0);
   }
 
@@ -647,7 +664,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
       uint32_t n = 0;
       bool ok = true;
       WideItem it;
-      for (int idx = 0; ok && wide_item(p.tile_begin, tiles, tiles_m, kb_total, split, rank, idx, it); ++idx) {
+      for (int idx = 0; ok && wide_item(p, idx, it); ++idx) {
         for (int kb = it.k0; kb < it.k1; ++kb, ++n) {
           const uint32_t s = n % kStages;
           if (n < prefetched) {  // the weight half is already on its way
@@ -667,26 +684,30 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     } else if (warp == E + 1 || warp == E + 2) {
       // ---------------- MMA issuers, one per accumulator ----------------
       constexpr uint32_t idesc = instr_desc_f8(BN);
+      static_assert(kStages == 2 * kAcc, "issuer b has stages b and b + 2");
       const int b = warp - (E + 1);
+      const uint32_t addr = smem_u32(stage_base + (size_t)b * kStageBytes), tmem_d = tmem_base + b * BN;
+      const uint64_t da0 = smem_desc_k128(addr), db0 = smem_desc_k128(addr + kTileR * kBlockK);
+      uint32_t second = 0, parity = 0;  // stage b or b + kAcc, phase of that stage
+#pragma unroll 1
       for (uint32_t n = b; n < total_blocks; n += kAcc) {
-        const int s = n % kStages;
-        // In this order: the stage's previous block may be the other issuer's, and a released accumulator (of a block no
-        // older, kAcc <= kStages) tells that its barrier phase is over.
-        if (!warp_wait_bounded(&tmem_empty[b], ((n / kAcc) & 1u) ^ 1u) ||
-            !warp_wait_bounded(&full_bar[s], (n / kStages) & 1u)) {
+        const uint64_t da = da0 + second * (kAcc * kStageBytes >> 4), db = db0 + second * (kAcc * kStageBytes >> 4);
+        uint64_t* done = &done_bar[b + second * kAcc];
+        if (!warp_wait_bounded(&full_bar[b + second * kAcc], parity) ||
+            !warp_wait_bounded(&tmem_empty[b], second ^ 1u)) {
           raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
           break;
         }
         tc_fence_after();
-        if (!elect_one()) continue;
-        const uint32_t a_addr = smem_u32(stage_base + (size_t)s * kStageBytes);
-        const uint64_t da = smem_desc_k128(a_addr), db = smem_desc_k128(a_addr + kTileR * kBlockK);
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < kBlockK / kUmmaK; ++k) {
-          umma_f8(tmem_base + b * BN, da + (uint64_t)(k * kUmmaK / 16), db + (uint64_t)(k * kUmmaK / 16), idesc,
-                  k > 0 ? 1u : 0u);
+          for (int k = 0; k < kBlockK / kUmmaK; ++k)
+            umma_f8(tmem_d, da + (uint64_t)(k * kUmmaK / 16), db + (uint64_t)(k * kUmmaK / 16), idesc, k > 0 ? 1u : 0u);
+          umma_commit(done);  // frees the smem stage and hands the accumulator to the promotion warps
         }
-        umma_commit(&done_bar[s]);  // frees the smem stage and hands the accumulator to the promotion warps
+        __syncwarp();
+        parity ^= second;
+        second ^= 1u;
       }
     }
     __syncwarp();
@@ -708,14 +729,14 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     uint32_t n = 0;
     bool ok = true;
     WideItem it;
-    for (int idx = 0; ok && wide_item(p.tile_begin, tiles, tiles_m, kb_total, split, rank, idx, it); ++idx) {
+    for (int idx = 0; ok && wide_item(p, idx, it); ++idx) {
       const int tok0 = it.tm * kTileR;
       // The scales of this thread's row and of its columns' weight block, requested a K block ahead.
       const int blk = it.tn * 2 + col0 / 128;
       const bool row_live = tok0 + row_in_tile < p.m, col_live = blk * 128 < p.n;
       const float* a_at = p.a_scale + (long long)it.k0 * p.a_scale_ld + (row_live ? tok0 + row_in_tile : 0);
       const float* w_at = p.w_scale + (col_live ? (long long)blk * p.w_scale_ld : 0) + it.k0;
-      float a_next = row_live ? *a_at : 0.f, w_next = col_live ? *w_at : 0.f;
+      float a_next = __ldg(a_at), w_next = __ldg(w_at);
       for (int kb = it.k0; kb < it.k1; ++kb, ++n) {
         const uint32_t taddr = lane_addr + (n & 1) * BN;
         if (!mbar_wait_bounded(&done_bar[n % kStages], (n / kStages) & 1u)) {
@@ -725,11 +746,10 @@ __global__ void __launch_bounds__(kWideThreads, 1)
         }
         tc_fence_after();
         const float s = a_next * w_next;
-        if (kb + 1 < it.k1) {
-          a_at += p.a_scale_ld;
-          if (row_live) a_next = *a_at;
-          if (col_live) w_next = *++w_at;
-        }
+        a_at += kb + 1 < it.k1 ? p.a_scale_ld : 0;
+        w_at += kb + 1 < it.k1 ? 1 : 0;
+        a_next = __ldg(a_at);
+        w_next = __ldg(w_at);
         float buf[32];
         tmem_ld32(taddr, buf);
         tmem_ld_wait_pin(buf);
@@ -1095,6 +1115,7 @@ WidePlan plan_wide(long long tiles, int kb, int max_split) {
 int launch_wide_range(const CUtensorMap& mx, const CUtensorMap& mw, GemmParams p, int tile_begin, int tile_end,
                       int split, bool late_wait, bool tail_follows, cudaStream_t stream) {
   p.tile_begin = tile_begin;
+  p.band = wide_band(p.m, p.k);
   p.tile_end = tile_end;
   p.late_wait = late_wait ? 1 : 0;
   p.early_release = tail_follows ? 0 : 1;
