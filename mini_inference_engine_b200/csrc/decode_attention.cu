@@ -595,15 +595,18 @@ int launch_merge(const DecodeParams& q, int heads, cudaStream_t stream) {
 }
 
 template <typename T>
-int launch_fast(const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, cudaStream_t stream) {
+int launch_fast(const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, int policy, cudaStream_t stream) {
+  const int share = policy == 1 ? decode_share(p.batch, p.kv_heads, (long long)p.table_width * p.block_size, 512) : 0;
+  if (share > 0) return launch_shared<T, 2, 2, false>(p, kmap, vmap, share, stream);
   static bool configured[64] = {false};
   int dev = 0;
   MIE_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    MIE_CUDA(cudaFuncSetAttribute(decode_kernel<T, 2, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDecodeSmem));
+    MIE_CUDA(cudaFuncSetAttribute(decode_kernel<T, 2, 2, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDecodeSmem));
     configured[dev] = true;
   }
-  MIE_CUDA(launch_chained(decode_kernel<T, 2, 2, false>, dim3(sm_count()), dim3(kWarps * 32), kDecodeSmem, stream, kmap, vmap, p));
+  MIE_CUDA(launch_chained(decode_kernel<T, 2, 2, false, false>, dim3(sm_count()), dim3(kWarps * 32), kDecodeSmem, stream, kmap, vmap,
+                          p, 1));
   MIE_LAUNCH_CHECK("decode_kernel");
   // Groups wider than kMaxGroupMerge take several passes of head sub-groups.
   for (int g0 = 0; g0 < p.group; g0 += kMaxGroupMerge) {
@@ -713,8 +716,8 @@ extern "C" int mie_paged_decode_attention(mie_view4_t query, mie_view4_t out, mi
   CUtensorMap kmap, vmap;
   if (int rc = page_tensor_map(key_blocks, num_blocks, kv_heads, block_size, head_dim, dtype, &kmap)) return rc;
   if (int rc = page_tensor_map(value_blocks, num_blocks, kv_heads, block_size, head_dim, dtype, &vmap)) return rc;
-  if (dtype == MIE_DTYPE_BF16) return launch_fast<__nv_bfloat16>(p, kmap, vmap, stream);
-  return launch_fast<__half>(p, kmap, vmap, stream);
+  if (dtype == MIE_DTYPE_BF16) return launch_fast<__nv_bfloat16>(p, kmap, vmap, split_policy, stream);
+  return launch_fast<__half>(p, kmap, vmap, split_policy, stream);
 }
 
 // ---------------------------------------------------------------------------

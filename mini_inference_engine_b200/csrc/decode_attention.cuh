@@ -3,6 +3,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "umma.cuh"
 
 namespace mie {
 namespace {
@@ -16,6 +17,7 @@ constexpr int kPlanThreads = 1024;
 constexpr int kHeaderInts = 128;  // [0]=chunk [1]=seq_chunks [2]=items; [16..79] work counters
 constexpr int kCounterBase = 16;
 constexpr int kCounters = 64;
+constexpr int kMaxShare = 8;      // CTAs that share a (request, KV head)
 constexpr int kMaxGroupMerge = 4;  // query heads per KV head the merge kernel handles in one block
 
 // Tile geometry for key rows of KH and value rows of VH 64-dim boxes.  A head size that is no multiple of 64
@@ -278,12 +280,117 @@ struct DecodeParams {
   const float* sinks;
 };
 
+// The end of a (request, KV head) that a cluster shares (kShare): every warp has the part `o`, `m`, `l` of its tokens.  The
+// CTA's parts meet in shared memory, the cluster's in rank 0, which writes the result.
+template <typename T, int KH, int VH, bool kExt>
+__device__ __forceinline__ void finish_shared(const DecodeParams& p, const float (&o)[VH * 8][4], float m, float l, int b,
+                                              int head0, int rows, uint8_t* stage0, int* pids0, int split, int rank) {
+  using Tile = DecodeTile<KH, VH>;
+  constexpr int kWarps = Tile::kWarps, kRowFloats = VH * 64 + 8;  // padded: rows start in different banks
+  constexpr int kPartFloats = Tile::kStages * Tile::kStageBytes / 4, kCols = (VH + 1) / 2;
+  static_assert(8 * kRowFloats <= kPartFloats && kPidBatch * 4 >= 8 * 16, "a warp's part fits its ring, its sums its page ids");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  float* parts = reinterpret_cast<float*>(stage0);     // [warp] kPartFloats apart
+  float4* sums = reinterpret_cast<float4*>(pids0);     // [warp] kPidBatch / 4 apart: (maximum, sum) of each row
+  float* mine = parts + warp * kPartFloats + g * kRowFloats;
+#pragma unroll
+  for (int n = 0; n < VH * 8; ++n) *reinterpret_cast<float2*>(mine + n * 8 + 2 * t) = make_float2(o[n][0], o[n][1]);
+  if (t == 0) sums[warp * (kPidBatch / 4) + g] = make_float4(m, l, 0.f, 0.f);
+  __syncthreads();
+  auto weight = [](float mi, float top) { return mi == -INFINITY ? 0.f : exp2f(mi - top); };
+  for (int r = warp; r < rows; r += kWarps) {  // a warp has a row, a lane four dims of every 128
+    float top = -INFINITY, sum = 0.f;
+    float4 acc[kCols];
+#pragma unroll
+    for (int x = 0; x < kCols; ++x) acc[x] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) top = fmaxf(top, sums[w * (kPidBatch / 4) + r].x);
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const float4 s = sums[w * (kPidBatch / 4) + r];
+      const float f = weight(s.x, top);
+      sum += s.y * f;
+#pragma unroll
+      for (int x = 0; x < kCols; ++x) {
+        if (x * 128 + lane * 4 >= VH * 64) continue;
+        const float4 v = *reinterpret_cast<const float4*>(parts + w * kPartFloats + r * kRowFloats + x * 128 + lane * 4);
+        acc[x].x += v.x * f, acc[x].y += v.y * f, acc[x].z += v.z * f, acc[x].w += v.w * f;
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int x = 0; x < kCols; ++x)  // in place of warp 0's part, which no other lane reads here
+      if (x * 128 + lane * 4 < VH * 64) *reinterpret_cast<float4*>(parts + r * kRowFloats + x * 128 + lane * 4) = acc[x];
+    if (lane == 0) sums[r] = make_float4(top, sum, 0.f, 0.f);
+  }
+  __syncwarp();
+  cluster_sync_all();
+  if (rank == 0) {
+    for (int r = warp; r < rows; r += kWarps) {
+      float4 s[kMaxShare], v[kCols][kMaxShare];
+      float top = -INFINITY, sum = 0.f;
+#pragma unroll
+      for (int i = 0; i < kMaxShare; ++i) {  // every rank's loads in flight together
+        if (i >= split) break;
+        s[i] = ld_cluster_f4(smem_u32(&sums[r]), i);
+#pragma unroll
+        for (int x = 0; x < kCols; ++x)
+          v[x][i] = ld_cluster_f4(smem_u32(parts + r * kRowFloats + (x * 128 + lane * 4 < VH * 64 ? x * 128 + lane * 4 : 0)), i);
+      }
+#pragma unroll
+      for (int i = 0; i < kMaxShare; ++i)
+        if (i < split) top = fmaxf(top, s[i].x);
+      float4 acc[kCols];
+#pragma unroll
+      for (int x = 0; x < kCols; ++x) acc[x] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < kMaxShare; ++i) {
+        if (i >= split) break;
+        const float f = weight(s[i].x, top);
+        sum += s[i].y * f;
+#pragma unroll
+        for (int x = 0; x < kCols; ++x)
+          acc[x].x += v[x][i].x * f, acc[x].y += v[x][i].y * f, acc[x].z += v[x][i].z * f, acc[x].w += v[x][i].w * f;
+      }
+      const float inv = 1.f / fmaxf(sum, 1.17549435e-38f);
+      const int head = head0 + r;
+      T* orow = reinterpret_cast<T*>(p.out.ptr) + (long long)b * p.out.s[0] + (long long)head * p.out.s[1];
+#pragma unroll
+      for (int x = 0; x < kCols; ++x) {
+        const int d = x * 128 + lane * 4;
+        float a[4] = {round_act<T>(acc[x].x * inv), round_act<T>(acc[x].y * inv), round_act<T>(acc[x].z * inv),
+                      round_act<T>(acc[x].w * inv)};
+        const int dims = kExt ? p.vdim : kHeadDim;
+        if (d < dims) {
+          *reinterpret_cast<uint32_t*>(orow + d) = Mma16816<T>::pack(a[0], a[1]);
+          *reinterpret_cast<uint32_t*>(orow + d + 2) = Mma16816<T>::pack(a[2], a[3]);
+        }
+        if (!kExt && p.out_q8 != nullptr) {
+          const float amax = warp_max(fmaxf(fmaxf(fabsf(a[0]), fabsf(a[1])), fmaxf(fabsf(a[2]), fabsf(a[3]))));
+          const float scale = __fdiv_rn(amax, 448.0f), denom = fmaxf(scale, 1e-12f);
+          __nv_fp8x2_storage_t* qrow =
+              reinterpret_cast<__nv_fp8x2_storage_t*>(p.out_q8 + (long long)b * p.ldq8 + head * kHeadDim + d);
+          qrow[0] = __nv_cvt_float2_to_fp8x2(make_float2(__fdiv_rn(a[0], denom), __fdiv_rn(a[1], denom)), __NV_SATFINITE,
+                                             __NV_E4M3);
+          qrow[1] = __nv_cvt_float2_to_fp8x2(make_float2(__fdiv_rn(a[2], denom), __fdiv_rn(a[3], denom)), __NV_SATFINITE,
+                                             __NV_E4M3);
+          if (lane == 0) p.out_scales[(long long)head * p.out_scale_ld + b] = scale;
+        }
+      }
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();  // nobody's shared memory goes before rank 0 has read it
+}
+
 // kExt = false: head_dim 128, GQA group <= 8, scores rounded to the activation dtype as the reference's bf16
 // product is.  kExt = true: other head sizes, any group, fp32 scores, sliding window, sinks, no e4m3 output.
-template <typename T, int KH, int VH, bool kExt>
+// kShare = false: persistent warps take (request, chunk, KV head) items of the work plan and leave partials for the merge
+// kernel.  kShare = true, for few requests: a cluster per (request, KV head), whose warps have equal parts of its tokens.
+template <typename T, int KH, int VH, bool kExt, bool kShare>
 __global__ void __launch_bounds__(DecodeTile<KH, VH>::kWarps * 32, 1)
     decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
-                  const DecodeParams p) {
+                  const DecodeParams p, const int split) {
   using Tile = DecodeTile<KH, VH>;
   constexpr int kWarps = Tile::kWarps, kStages = Tile::kStages, kStageBytes = Tile::kStageBytes;
   extern __shared__ uint8_t smem_raw[];
@@ -305,8 +412,9 @@ __global__ void __launch_bounds__(DecodeTile<KH, VH>::kWarps * 32, 1)
   chain_wait();
 
   const int g = lane >> 2, t = lane & 3;
-  const int chunk = p.sc.header[0];
-  const int total_items = p.sc.header[2];
+  const int chunk = kShare ? 0 : p.sc.header[0];
+  const int total_items = kShare ? 0 : p.sc.header[2];
+  const int rank = kShare ? (int)blockIdx.x % split : 0;
   int* counter = p.sc.header + kCounterBase + p.counter_slot;
   const long long capacity_tokens = (long long)p.table_width * p.block_size;
   uint32_t parity = 0;
@@ -320,21 +428,28 @@ __global__ void __launch_bounds__(DecodeTile<KH, VH>::kWarps * 32, 1)
 
   while (true) {
     int item = 0;
-    if (lane == 0) item = atomicAdd(counter, 1);
-    item = __shfl_sync(0xffffffffu, item, 0);
-    if (item >= total_items) break;
+    if constexpr (kShare) {
+      item = (int)blockIdx.x / split;
+    } else {
+      if (lane == 0) item = atomicAdd(counter, 1);
+      item = __shfl_sync(0xffffffffu, item, 0);
+      if (item >= total_items) break;
+    }
     const int item_heads = kExt ? p.item_heads : p.kv_heads;
     const int sci = item / item_heads, hi = item % item_heads;
     const int subs = kExt ? item_heads / p.kv_heads : 1;          // query sub-groups of a KV head
     const int h = kExt ? hi / subs : hi, sub0 = kExt ? (hi % subs) * 8 : 0;
     const int rows = kExt && p.group - sub0 > 8 ? 8 : p.group - sub0;  // query heads of this item
-    const int b = p.sc.item_seq[sci], ck = p.sc.item_chunk[sci];
-    const long long rl = read_length(p.lengths, p.positions, b, capacity_tokens, nullptr);
-    const int nchunks = p.sc.offsets[b + 1] - p.sc.offsets[b];
+    const int b = kShare ? sci : p.sc.item_seq[sci], ck = kShare ? rank * kWarps + warp : p.sc.item_chunk[sci];
+    const bool reports = kShare && hi == 0 && ck == 0 && lane == 0;  // otherwise the plan kernel has
+    const long long rl = read_length(p.lengths, p.positions, b, capacity_tokens, kShare && reports ? p.status : nullptr);
+    const int nchunks = kShare ? 0 : p.sc.offsets[b + 1] - p.sc.offsets[b];
     const long long first = kExt ? window_start(rl, p.window) : 0;
     const long long first_seen = kExt && p.window > 0 && rl > p.window ? rl - p.window : 0;
-    const long long t_begin = first + (long long)ck * chunk;
-    const long long t_end = rl < t_begin + chunk ? rl : t_begin + chunk;
+    const long long tiles = (rl - first + kTileTokens - 1) / kTileTokens, parts = kShare ? split * kWarps : 1;
+    const long long t_begin = kShare ? first + tiles * ck / parts * kTileTokens : first + (long long)ck * chunk;
+    const long long t_stop = kShare ? first + tiles * (ck + 1) / parts * kTileTokens : t_begin + chunk;
+    const long long t_end = rl < t_stop ? rl : t_stop;
     const int ntiles = (int)((t_end - t_begin + kTileTokens - 1) / kTileTokens);
 
     // Query fragments: rows g < group are real heads, the rest of the 16 MMA rows are zero.
@@ -498,12 +613,17 @@ __global__ void __launch_bounds__(DecodeTile<KH, VH>::kWarps * 32, 1)
     }
     if (timed_out) {
       if (lane == 0) raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
-      break;
+      if (!kShare) break;
     }
 
     // Row sum over the quad, then write the result (final or partial).
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
+    if (kShare) {
+      finish_shared<T, KH, VH, kExt>(p, o, m, l, b, h * p.group + sub0, rows, smem,
+                                     pids - warp * kPidBatch, split, rank);
+      return;
+    }
     const bool head_live = g < rows;
     const int head = h * p.group + sub0 + (head_live ? g : 0);
     const int out_dim = kExt ? p.vdim : kHeadDim;
@@ -568,6 +688,52 @@ __global__ void __launch_bounds__(DecodeTile<KH, VH>::kWarps * 32, 1)
       }
     }
   }
+}
+
+// CTAs per (request, KV head) when a cluster shares it, or 0: work plan, queue and merge kernel.  What that path costs before
+// and behind the streaming (plan, queue, item and page look-ups one after the other, a second launch) is 5 us: one request
+// of 611 tokens 11.0 -> 6.3 us, of 3000 14.3 -> 8.7, four of 200 10.9 -> 6.0, four of 3000 18.8 -> 15.8, sixteen of 200
+// 11.8 -> 9.5.  But the shares are fixed before lengths are known, so they have to do for the longest request that the block
+// table has room for: any, if it gets 64 CTAs (30000 tokens: 35.0 us against 35.9), else 512 KiB a CTA, 1 MiB in clusters
+// of four (eight of 3000, two CTAs a head: 33.8 us against 25.8; sixteen of 1000, one CTA: 25.0 against 19.7).
+inline int decode_share(int batch, int item_heads, long long capacity_tokens, int token_bytes) {
+  const long long clusters = (long long)batch * item_heads;
+  if (clusters > sm_count() || capacity_tokens <= kMinChunk) return 0;  // (one chunk a request: nothing is cut)
+  int split = 1;
+  while (split < 4 && clusters * split * 2 <= sm_count()) split *= 2;
+  if (clusters * 16 <= sm_count()) split = 8;  // sixteen clusters of eight do not fit the GPU at once
+  const long long share = capacity_tokens * token_bytes / split;
+  return split * item_heads >= 64 || share <= (split >= 4 ? 1 << 20 : 512 << 10) ? split : 0;
+}
+
+template <typename T, int KH, int VH, bool kExt>
+int launch_shared(const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, int split, cudaStream_t stream) {
+  using Tile = DecodeTile<KH, VH>;
+  static bool configured[64] = {false};
+  int dev = 0;
+  MIE_CUDA(cudaGetDevice(&dev));
+  if (dev >= 0 && dev < 64 && !configured[dev]) {
+    MIE_CUDA(cudaFuncSetAttribute(decode_kernel<T, KH, VH, kExt, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)Tile::kSmem));
+    configured[dev] = true;
+  }
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3((unsigned)(p.batch * p.item_heads * split));
+  config.blockDim = dim3(Tile::kWarps * 32);
+  config.dynamicSmemBytes = Tile::kSmem;
+  config.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)split;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attr;
+  config.numAttrs = chained_launch_enabled() ? 2 : 1;
+  prefer_shared_carveout(reinterpret_cast<const void*>(decode_kernel<T, KH, VH, kExt, true>));
+  MIE_CUDA(cudaLaunchKernelEx(&config, decode_kernel<T, KH, VH, kExt, true>, kmap, vmap, p, split));
+  MIE_LAUNCH_CHECK("decode_kernel");
+  return MIE_OK;
 }
 
 // Split-KV partials of the extended kernels: one block per (request, query head), values of up to VH 64-dim boxes.

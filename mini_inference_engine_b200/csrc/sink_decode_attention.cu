@@ -14,19 +14,24 @@ namespace {
 constexpr int kMaxBoxes = 4;  // head sizes up to 256
 
 template <int KH, int VH>
-int launch_sink(const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, cudaStream_t stream) {
+int launch_sink(const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, int policy, cudaStream_t stream) {
   using Tile = DecodeTile<KH, VH>;
   using T = __nv_bfloat16;
+  // A windowed request reads no more than its window and a tile.
+  const long long room = (long long)p.table_width * p.block_size;
+  const long long longest = p.window > 0 && p.window + kTileTokens < room ? p.window + kTileTokens : room;
+  const int share = policy == 1 ? decode_share(p.batch, p.item_heads, longest, (KH + VH) * 128) : 0;
+  if (share > 0) return launch_shared<T, KH, VH, true>(p, kmap, vmap, share, stream);
   static bool configured[64] = {false};
   int dev = 0;
   MIE_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    MIE_CUDA(cudaFuncSetAttribute(decode_kernel<T, KH, VH, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    MIE_CUDA(cudaFuncSetAttribute(decode_kernel<T, KH, VH, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)Tile::kSmem));
     configured[dev] = true;
   }
-  MIE_CUDA(launch_chained(decode_kernel<T, KH, VH, true>, dim3(sm_count()), dim3(Tile::kWarps * 32), Tile::kSmem,
-                          stream, kmap, vmap, p));
+  MIE_CUDA(launch_chained(decode_kernel<T, KH, VH, true, false>, dim3(sm_count()), dim3(Tile::kWarps * 32), Tile::kSmem,
+                          stream, kmap, vmap, p, 1));
   MIE_LAUNCH_CHECK("decode_kernel");
   MIE_CUDA(launch_chained(merge_rows_kernel<T, VH>, dim3((unsigned)(p.batch * p.q_heads)), dim3(kMergeWarps * 32), 0,
                           stream, p));
@@ -35,13 +40,13 @@ int launch_sink(const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMa
 }
 
 template <int KH>
-int launch_sink_v(int vh, const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap,
+int launch_sink_v(int vh, const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, int policy,
                   cudaStream_t stream) {
   switch (vh) {
-    case 1: return launch_sink<KH, 1>(p, kmap, vmap, stream);
-    case 2: return launch_sink<KH, 2>(p, kmap, vmap, stream);
-    case 3: return launch_sink<KH, 3>(p, kmap, vmap, stream);
-    default: return launch_sink<KH, 4>(p, kmap, vmap, stream);
+    case 1: return launch_sink<KH, 1>(p, kmap, vmap, policy, stream);
+    case 2: return launch_sink<KH, 2>(p, kmap, vmap, policy, stream);
+    case 3: return launch_sink<KH, 3>(p, kmap, vmap, policy, stream);
+    default: return launch_sink<KH, 4>(p, kmap, vmap, policy, stream);
   }
 }
 
@@ -114,9 +119,9 @@ extern "C" int mie_sink_decode_attention(const void* query, int64_t q_row_stride
   if (int rc = page_tensor_map(key_blocks, num_blocks, kv_heads, block_size, dim, dtype, &kmap)) return rc;
   if (int rc = page_tensor_map(value_blocks, num_blocks, kv_heads, block_size, value_dim, dtype, &vmap)) return rc;
   switch (kh) {
-    case 1: return launch_sink_v<1>(vh, p, kmap, vmap, stream);
-    case 2: return launch_sink_v<2>(vh, p, kmap, vmap, stream);
-    case 3: return launch_sink_v<3>(vh, p, kmap, vmap, stream);
-    default: return launch_sink_v<4>(vh, p, kmap, vmap, stream);
+    case 1: return launch_sink_v<1>(vh, p, kmap, vmap, split_policy, stream);
+    case 2: return launch_sink_v<2>(vh, p, kmap, vmap, split_policy, stream);
+    case 3: return launch_sink_v<3>(vh, p, kmap, vmap, split_policy, stream);
+    default: return launch_sink_v<4>(vh, p, kmap, vmap, split_policy, stream);
   }
 }
