@@ -287,10 +287,16 @@ __global__ void clamped_glu_kernel(const T* gate, const T* up, long long ld_in, 
   Vec<T, VEC>::load(gate + row * ld_in + c, g);
   Vec<T, VEC>::load(up + row * ld_in + c, u);
 #pragma unroll
-  for (int j = 0; j < VEC; ++j) {
-    const float a = fminf(g[j], limit), b = fminf(fmaxf(u[j], -limit), limit) + up_offset;
-    g[j] = (sizeof(T) == 2 ? gate_sigmoid16(a, slope) : gate_sigmoid(a, slope)) * b;
+  for (int j = 0; j < VEC; ++j) g[j] = fminf(g[j], limit);
+  float f[VEC];
+  if constexpr (VEC == 8 && sizeof(T) == 2) {
+    gate8(g, slope, f);
+  } else {
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) f[j] = gate_sigmoid(g[j], slope);
   }
+#pragma unroll
+  for (int j = 0; j < VEC; ++j) g[j] = f[j] * (fminf(fmaxf(u[j], -limit), limit) + up_offset);
   Vec<T, VEC>::store(out + row * ldo + c, g);
 }
 

@@ -192,8 +192,7 @@ __device__ __forceinline__ void finish_rows(const GemmParams& p, const QkvParams
         const __nv_bfloat162* u2 = reinterpret_cast<const __nv_bfloat162*>(&up2);
 #pragma unroll
         for (int i = 0; i < 2; ++i)
-          r2[i] = __hmul2(__floats2bfloat162_rn(gate_sigmoid16(round_bf16(v[2 * i])),
-                                                gate_sigmoid16(round_bf16(v[2 * i + 1]))),
+          r2[i] = __hmul2(__floats2bfloat162_rn(silu16(round_bf16(v[2 * i])), silu16(round_bf16(v[2 * i + 1]))),
                           u2[i]);
         unpack4(raw, v);
         const float amax = warp_max(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));

@@ -13,7 +13,11 @@ namespace mie {
 namespace {
 
 // ---------------------------------------------------------------------------
-// Row RMSNorm: one CTA per row, cols a multiple of 8 (<= 8 * 1024).
+// Row RMSNorm: a CTA per row, eight columns a thread, cols a multiple of 8 (<= 8 * 1024).  With many rows a CTA goes from
+// row to row and requests the next one before it reduces this one; the weight is read once.  Bound by HBM (2 bytes a value
+// and tensor, 1 for e4m3), if the arithmetic is packed: 12032 x 2560 with residual, sum and e4m3
+// 54.3 us with a CTA per row, now 46.5; 560 rows 5.9 and 4.1, one row 2.9 and 2.1.  (Three CTAs of 320 threads per SM; four
+// 50.3, five 55.0; a warp per row 69.)
 // ---------------------------------------------------------------------------
 struct RowNormParams {
   const __nv_bfloat16* x;
@@ -30,47 +34,56 @@ struct RowNormParams {
   float eps;
 };
 
-__global__ void __launch_bounds__(1024) row_norm_kernel(RowNormParams p) {
-  __shared__ float red[32];
+// kThreads: the most of the instantiation; kCtas: how many of them an SM holds, all of which go from row to row.
+template <int kThreads, int kCtas>
+
+__global__ void __launch_bounds__(kThreads, kCtas) row_norm_kernel(RowNormParams p) {
+  __shared__ float red[2][32];
   chain_release();
   chain_wait();
-  const int row = blockIdx.x;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = (blockDim.x + 31) >> 5;
   const int c0 = tid * 8;
   const bool active = c0 < p.cols;
-  float v[8];
-  float ss = 0.f;
-  if (active) {
-    unpack8(*reinterpret_cast<const uint4*>(p.x + (long long)row * p.ldx + c0), v);
+  Bf16x8 x, r, w;
+  x.raw = r.raw = w.raw = make_uint4(0, 0, 0, 0);
+  auto load = [&](int row) {
+    if (!active || row >= p.rows) return;
+    x.raw = *reinterpret_cast<const uint4*>(p.x + (long long)row * p.ldx + c0);
+    if (p.residual != nullptr) r.raw = *reinterpret_cast<const uint4*>(p.residual + (long long)row * p.cols + c0);
+  };
+  load(blockIdx.x);
+  if (active) w.raw = *reinterpret_cast<const uint4*>(p.weight + c0);  // fetched with the row, not after the reduction
+  int turn = 0;
+  for (int row = blockIdx.x; row < p.rows; row += gridDim.x, turn ^= 1) {
+    Bf16x8 v;
+    v.raw = x.raw;
     if (p.residual != nullptr) {
-      float r[8];
-      unpack8(*reinterpret_cast<const uint4*>(p.residual + (long long)row * p.cols + c0), r);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = round_bf16(v[j] + r[j]);
-      if (p.summed != nullptr) *reinterpret_cast<uint4*>(p.summed + (long long)row * p.cols + c0) = pack8(v);
+      for (int i = 0; i < 4; ++i) v.pair[i] = __hadd2_rn(x.pair[i], r.pair[i]);
     }
+    load(row + gridDim.x);
+    if (active && p.summed != nullptr) *reinterpret_cast<uint4*>(p.summed + (long long)row * p.cols + c0) = v.raw;
+    float f[8], ss = 0.f;
+    unpack8(v.raw, f);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
-  } else {
+    for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    ss = warp_sum(ss);
+    if (lane == 0) red[turn][warp] = ss;  // the other half may still be read: the barrier of this row is behind that
+    __syncthreads();
+    float total = 0.f;
+    for (int i = 0; i < warps; ++i) total += red[turn][i];
+    const float inv = rsqrtf(total / (float)p.cols + p.eps);
+    Bf16x8 n;
+    scale8(f, inv, n);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = 0.f;
-  }
-  float w8[8];  // fetched with the row, not after the reduction
-  if (active) unpack8(*reinterpret_cast<const uint4*>(p.weight + c0), w8);
-  ss = warp_sum(ss);
-  if (lane == 0) red[warp] = ss;
-  __syncthreads();
-  float total = 0.f;
-  const int warps = (blockDim.x + 31) >> 5;
-  for (int w = 0; w < warps; ++w) total += red[w];
-  const float inv = rsqrtf(total / (float)p.cols + p.eps);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) v[j] = active ? round_bf16(w8[j] * round_bf16(v[j] * inv)) : 0.f;
-  if (active && p.out != nullptr) *reinterpret_cast<uint4*>(p.out + (long long)row * p.cols + c0) = pack8(v);
-  if (p.q != nullptr) {
-    // Lanes past the row end (cols is a multiple of 128 here) hold zeros and write nothing.
-    quantize_group_store(v, active ? p.q + (long long)row * p.ldq + c0 : nullptr,
-                         active ? p.scales + (long long)(c0 / 128) * p.scale_ld + row : nullptr, (tid & 15) == 0);
+    for (int i = 0; i < 4; ++i) n.pair[i] = __hmul2_rn(w.pair[i], n.pair[i]);
+    if (active && p.out != nullptr) *reinterpret_cast<uint4*>(p.out + (long long)row * p.cols + c0) = n.raw;
+    if (p.q != nullptr) {
+      // Lanes past the row end (cols is a multiple of 128 here) hold nothing and write nothing.
+      unpack8(n.raw, f);
+      quantize_group_store(f, active ? p.q + (long long)row * p.ldq + c0 : nullptr,
+                           active ? p.scales + (long long)(c0 / 128) * p.scale_ld + row : nullptr, (tid & 15) == 0);
+    }
   }
 }
 
@@ -100,41 +113,59 @@ __global__ void head_norm_kernel(const __nv_bfloat16* x, long long outer_stride,
 }
 
 // ---------------------------------------------------------------------------
-// SiLU(gate) * up, optional fused quantisation.  One thread per 8 columns.  HBM traffic (5 bytes a result when
-// quantised) bounds it only with few instructions per value: the divisions are corrected quotients, the product with
-// `up` is a packed bf16 multiplication (the same single rounding) and indices are 32-bit; with IEEE divisions and
-// 64-bit index divisions 12032 x 9728 took 244 us, now 159 us.
+// SiLU(gate) * up, optional fused quantisation.  Bound by HBM (5 bytes a result when quantised) only with few instructions
+// per value: gates by gate8, the product with `up` a packed bf16 multiplication (the same single rounding), corrected
+// quotients for e4m3, no index division.  Where a row is whole groups of 128 columns eight lanes have a group, 8 columns and
+// the 8 that lie 64 further, so that what a group takes once (its maximum, its scale and reciprocal) is shared by 16 values
+// of a lane.  12032 x 9728: 244 us with IEEE divisions, 158 with corrected quotients and 16 lanes a group, now 127
+// (4096 rows 56.0 and 45.2).
 // ---------------------------------------------------------------------------
-template <typename Index>
-__global__ void silu_mul_kernel(const __nv_bfloat16* gate, const __nv_bfloat16* up, long long ld_in,
-                                __nv_bfloat16* out, uint8_t* q, long long ldq, float* scales, int scale_ld,
-                                int rows, int cols) {
+template <bool kGroups>
+__global__ void __launch_bounds__(512)
+    silu_mul_kernel(const __nv_bfloat16* gate, const __nv_bfloat16* up, long long ld_in, __nv_bfloat16* out, uint8_t* q,
+                    long long ldq, float* scales, int scale_ld, int cols, int blocks_per_row) {
+  constexpr int kParts = kGroups ? 2 : 1;  // eight columns each
   chain_release();
   chain_wait();
-  const Index per_row = (Index)(cols / 8);
-  const Index idx = (Index)blockIdx.x * (Index)blockDim.x + threadIdx.x;
-  const bool live = idx < (Index)rows * per_row;
-  const int row = live ? (int)(idx / per_row) : 0, c0 = live ? (int)(idx - (Index)row * per_row) * 8 : 0;
-  uint4 raw = make_uint4(0, 0, 0, 0);
-  if (live) {
-    const uint4 g4 = *reinterpret_cast<const uint4*>(gate + (long long)row * ld_in + c0);
-    const uint4 u4 = *reinterpret_cast<const uint4*>(up + (long long)row * ld_in + c0);
-    float g[8];
-    unpack8(g4, g);
-    const __nv_bfloat162* u2 = reinterpret_cast<const __nv_bfloat162*>(&u4);
-    __nv_bfloat162* v2 = reinterpret_cast<__nv_bfloat162*>(&raw);
+  const int row = blockIdx.x / blocks_per_row;
+  const int in_row = (blockIdx.x - row * blocks_per_row) * blockDim.x + threadIdx.x;
+  const bool live = in_row < cols / (8 * kParts);
+  const int c0 = kGroups ? in_row / 8 * 128 + in_row % 8 * 8 : in_row * 8;
+  Bf16x8 v[kParts], u[kParts];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      v2[j] = __hmul2(__floats2bfloat162_rn(gate_sigmoid16(g[2 * j]), gate_sigmoid16(g[2 * j + 1])), u2[j]);
+  for (int x = 0; x < kParts; ++x) {
+    v[x].raw = u[x].raw = make_uint4(0, 0, 0, 0);
+    if (live) {
+      v[x].raw = *reinterpret_cast<const uint4*>(gate + (long long)row * ld_in + c0 + x * 64);
+      u[x].raw = *reinterpret_cast<const uint4*>(up + (long long)row * ld_in + c0 + x * 64);
+    }
   }
-  if (live && out != nullptr) *reinterpret_cast<uint4*>(out + (long long)row * cols + c0) = raw;
-  if (q != nullptr) {
-    float v[8];
-    unpack8(raw, v);
-    quantize_group_store(v, live ? q + (long long)row * ldq + c0 : nullptr,
-                         live ? scales + (long long)(c0 / 128) * scale_ld + row : nullptr,
-                         (threadIdx.x & 15) == 0);
+  float f[kParts][8], amax = 0.f;
+#pragma unroll
+  for (int x = 0; x < kParts; ++x) {
+    float g[8];
+    unpack8(v[x].raw, g);
+    gate8(g, 1.f, f[x]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      v[x].pair[i] = __hmul2_rn(__floats2bfloat162_rn(f[x][2 * i], f[x][2 * i + 1]), u[x].pair[i]);
+    if (live && out != nullptr) *reinterpret_cast<uint4*>(out + (long long)row * cols + c0 + x * 64) = v[x].raw;
+    unpack8(v[x].raw, f[x]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(f[x][j]));
   }
+  if (!kGroups || q == nullptr) return;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  const float scale = __fdiv_rn(amax, 448.0f), denom = fmaxf(scale, 1e-12f);
+  if (!live) return;
+#pragma unroll
+  for (int x = 0; x < kParts; ++x) {
+    uint32_t packed[2];
+    quantize_values(f[x], denom, packed);
+    *reinterpret_cast<uint2*>(q + (long long)row * ldq + c0 + x * 64) = make_uint2(packed[0], packed[1]);
+  }
+  if ((threadIdx.x & 7) == 0) scales[(long long)(c0 / 128) * scale_ld + row] = scale;
 }
 
 // ---------------------------------------------------------------------------
@@ -168,7 +199,8 @@ __global__ void rope_kernel(const __nv_bfloat16* x, long long sb, long long sh, 
 // q/k RMSNorm + RoPE + KV-cache write over a merged qkv row (head_dim 128).  A block per token (or several), 16 lanes per head, eight
 // consecutive dims a lane (partner dims d +/- 64 sit 8 lanes away): a lane's cos / sin entries, position and page serve
 // all the heads of its half-warp, whose rows are in flight together.  A warp per (token, head) with 8-byte accesses
-// looked all of that up per head: 12032 tokens of 48 heads 185 us, now 131 us (147 MB in, 147 MB out).
+// looked all of that up per head: 12032 tokens of 48 heads 185 us; fp32 arithmetic with a rounding after each operation 137,
+// packed bf16 90 (147 MB in, 147 MB out; 4096 tokens 49 and 33).
 // ---------------------------------------------------------------------------
 // Eight bf16 values, 16-byte aligned when `wide`, else 8-byte.
 __device__ __forceinline__ uint4 load8(const __nv_bfloat16* p, bool wide) {
@@ -210,9 +242,11 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvParams p) {
   qkv_place(p, t, threadIdx.x == 0 && blockIdx.y == 0, pos, page);
   const long long cpos = pos < 0 ? 0 : (pos >= p.max_pos ? p.max_pos - 1 : pos);
   const __nv_bfloat16* cs = p.cos_sin + cpos * 256 + l16 * 8;
-  float c[8], s[8];
-  unpack8(load8(cs, p.wide), c);
-  unpack8(load8(cs + 128, p.wide), s);
+  Bf16x8 c, s;  // rotate_half is (-x2, x1): the sign goes to the sines of the lower half
+  c.raw = load8(cs, p.wide);
+  s.raw = load8(cs + 128, p.wide);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) s.word[i] ^= l16 < 8 ? 0x80008000u : 0u;
   const int slot = (int)((pos < 0 ? 0 : pos) % p.block_size);
 
   for (int h0 = h_first; h0 - h_first < heads_total; h0 += kQkvBatch * half_warps) {
@@ -222,18 +256,20 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvParams p) {
       const int h = h0 + u * half_warps;  // a half-warp past the last head stays for the shuffles
       if (h - h_first >= heads_total) break;
       const bool is_q = h < p.q_heads, is_v = h >= p.q_heads + p.kv_heads, live = h < heads_total;
-      float v[8], w[8], o[8];
+      float v[8];
       unpack8(raw[u], v);
       const float inv = rsqrtf(half_warp_square_sum(v, l16) / 128.f + p.eps);
-      unpack8(load8((is_q ? p.q_weight : p.k_weight) + l16 * 8, p.wide), w);
+      Bf16x8 w, n, o;
+      w.raw = load8((is_q ? p.q_weight : p.k_weight) + l16 * 8, p.wide);
+      scale8(v, inv, n);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float n = round_bf16(w[j] * round_bf16(v[j] * inv));
-        const float partner = __shfl_xor_sync(0xffffffffu, n, 8);
-        const float rot = l16 < 8 ? -partner : partner;  // rotate_half: (-x2, x1)
-        o[j] = round_bf16(n * c[j]) + round_bf16(rot * s[j]);
+      for (int i = 0; i < 4; ++i) {
+        n.pair[i] = __hmul2_rn(w.pair[i], n.pair[i]);
+        Bf16x8 partner;
+        partner.word[0] = __shfl_xor_sync(0xffffffffu, n.word[i], 8);
+        o.pair[i] = __hadd2_rn(__hmul2_rn(n.pair[i], c.pair[i]), __hmul2_rn(partner.pair[0], s.pair[i]));
       }
-      const uint4 result = is_v ? raw[u] : pack8(o);
+      const uint4 result = is_v ? raw[u] : o.raw;
       // e4m3 pool: one scale per (token, KV head), amax of the 128 bf16 values / 448, the row divided by it and rounded
       // to e4m3 (the activation quantiser's rule).  Every half-warp takes part, whatever its head is.
       uint32_t packed[2];
@@ -288,7 +324,14 @@ extern "C" int mie_rms_norm(const void* x, int64_t ldx, const void* residual, vo
                   (const __nv_bfloat16*)weight, (__nv_bfloat16*)out, (uint8_t*)q, ldq, scales, scale_ld, rows, cols,
                   eps};
   const int threads = ((cols / 8) + 31) / 32 * 32;
-  MIE_CUDA(launch_chained(row_norm_kernel, dim3(rows), dim3(threads), 0, (cudaStream_t)stream, p));
+  const auto launch = [&](auto kernel, int per_sm) {
+    const int ctas = sm_count() * per_sm;
+    return launch_chained(kernel, dim3(rows < ctas ? rows : ctas), dim3(threads), 0, (cudaStream_t)stream, p);
+  };
+  MIE_CUDA(threads <= 256   ? launch(row_norm_kernel<256, 4>, 4)
+           : threads <= 384 ? launch(row_norm_kernel<384, 3>, 3)
+           : threads <= 512 ? launch(row_norm_kernel<512, 2>, 2)
+                            : launch(row_norm_kernel<1024, 1>, 1));
   MIE_LAUNCH_CHECK("row_norm_kernel");
   return MIE_OK;
 }
@@ -316,12 +359,13 @@ extern "C" int mie_silu_mul(const void* gate, const void* up, int64_t ld_in, voi
   MIE_CHECK_ARG(!q || (scales && cols % 128 == 0 && scale_ld >= rows && ldq >= cols && ldq % 8 == 0),
                 "fused quantisation needs cols %% 128 == 0 and scale storage");
   if (rows == 0) return MIE_OK;
-  const int threads = 256;
-  const long long blocks = ((long long)rows * (cols / 8) + threads - 1) / threads;
-  const auto kernel = blocks * threads < (1ll << 31) ? silu_mul_kernel<uint32_t> : silu_mul_kernel<uint64_t>;
-  MIE_CUDA(launch_chained(kernel, dim3((unsigned)blocks), dim3(threads), 0, (cudaStream_t)stream,
-                          (const __nv_bfloat16*)gate, (const __nv_bfloat16*)up, ld_in, (__nv_bfloat16*)out,
-                          (uint8_t*)q, ldq, scales, scale_ld, rows, cols));
+  const bool groups = cols % 128 == 0;
+  const int lanes = cols / (groups ? 16 : 8), most = rows <= sm_count() ? 128 : 512;  // few rows: more, smaller blocks
+  const int per_row = (lanes + most - 1) / most, threads = ((lanes + per_row - 1) / per_row + 31) / 32 * 32;
+  MIE_CHECK_ARG((long long)rows * per_row <= 0x7fffffff, "too many rows (%d)", rows);
+  MIE_CUDA(launch_chained(groups ? silu_mul_kernel<true> : silu_mul_kernel<false>, dim3((unsigned)(rows * per_row)),
+                          dim3(threads), 0, (cudaStream_t)stream, (const __nv_bfloat16*)gate, (const __nv_bfloat16*)up,
+                          ld_in, (__nv_bfloat16*)out, (uint8_t*)q, ldq, scales, scale_ld, cols, per_row));
   MIE_LAUNCH_CHECK("silu_mul_kernel");
   return MIE_OK;
 }

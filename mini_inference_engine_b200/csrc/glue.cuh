@@ -35,6 +35,20 @@ __device__ __forceinline__ uint2 pack4(const float (&v)[4]) {
   return raw;
 }
 
+// Eight bf16 values as they come from memory.  A product or a sum of two bf16 values that is rounded to bf16 is one packed
+// instruction for two of them (the _rn forms are never contracted): the same bits as fp32 arithmetic and a rounding - exact
+// products have 16 bits, and a sum that fp32 would round first has a summand below half a unit of the other.
+union Bf16x8 {
+  uint4 raw;
+  uint32_t word[4];
+  __nv_bfloat162 pair[4];
+};
+// bf16(v * f) of eight values.
+__device__ __forceinline__ void scale8(const float (&v)[8], float f, Bf16x8& out) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) out.pair[i] = __floats2bfloat162_rn(v[2 * i] * f, v[2 * i + 1] * f);
+}
+
 // a / b from y, an approximation of 1 / b: quotient, its exact remainder, correction.  Correctly rounded when y is the
 // correctly rounded reciprocal (Markstein's theorem), else but for quotients within 2^-20 units of a tie.  Three
 // instructions where an IEEE division takes about ten.  a, b and y must be finite.
@@ -46,14 +60,36 @@ __device__ __forceinline__ float corrected_quotient(float a, float b, float y) {
 // g / (1 + exp(-slope g)).
 __device__ __forceinline__ float gate_sigmoid(float g, float slope = 1.f) { return g / (1.f + expf(-slope * g)); }
 
-// The same for a result that is rounded to 16 bits: SiLU of every bf16 value comes out as with the division.
-__device__ __forceinline__ float gate_sigmoid16(float g, float slope = 1.f) {
-  const float d = 1.f + expf(-slope * g);
-  // a reciprocal near or below the smallest normal number, an infinite gate
-  if (d > 1e37f || fabsf(g) > 3.4e38f) return __fdiv_rn(g, d);
+// The same from the approximate exponential and reciprocal, for results that are rounded to 16 bits: within 2^-20 of the
+// quotient, and SiLU (slope 1) of every bf16 value is rounded to what the quotient is.  slope_log2e = slope * log2 e.
+// `denominator` above kGateLimit, whose reciprocal is flushed to zero, takes the quotient instead.
+constexpr float kGateLimit = 5e37f, kLog2e = 1.4426950408889634f;
+__device__ __forceinline__ float gate_denominator(float g, float slope_log2e) {
+  float t;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(g * -slope_log2e));
+  return 1.f + t;
+}
+__device__ __forceinline__ float gate_quotient(float g, float denominator) {
   float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
-  return corrected_quotient(g, d, y);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(denominator));
+  return g * y;
+}
+__device__ __forceinline__ float silu16(float g) {
+  const float d = gate_denominator(g, kLog2e);
+  return d > kGateLimit ? gate_sigmoid(g) : gate_quotient(g, d);
+}
+// Eight values with one test for all of them.
+__device__ __forceinline__ void gate8(const float (&g)[8], float slope, float (&f)[8]) {
+  float top = 0.f;  // NaN passes the test and comes through the quotient
+  const float k = slope * kLog2e;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    f[j] = gate_denominator(g[j], k);
+    top = fmaxf(top, f[j]);
+  }
+  const bool plain = top <= kGateLimit;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) f[j] = plain ? gate_quotient(g[j], f[j]) : gate_sigmoid(g[j], slope);
 }
 
 // v[0..n) / denom as e4m3, two values per 16 bits.  denom >= 1e-12; quotients that e4m3 does not round to zero are exact
