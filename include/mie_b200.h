@@ -352,6 +352,10 @@ int mie_fp8_gemm(const void* x8, int64_t ldx, const float* a_scale, int32_t a_sc
  * product is mie_qkv_norm_rope_write, or with kv_pool (then block_size is 16
  * and the page views are not read) mie_qkv_norm_rope_write_kv8.
  *
+ * mie_fp8_gemm_silu_wide: the same for any number of tokens, by whole tiles of
+ * the kernel for long steps; mie_fp8_gemm_silu_wide_pays: whether that is the
+ * faster way (0 wherever mie_fp8_gemm_finishes is 1).
+ *
  * mie_fp8_gemm_finish_pays: whether that one launch is also the faster way for
  * m tokens of an [n, k] weight (gated = 1: mie_fp8_gemm_silu with n = 2 cols;
  * gated = 0: mie_fp8_gemm_qkv); 0 wherever mie_fp8_gemm_finishes is.
@@ -362,6 +366,11 @@ int mie_fp8_gemm_silu(const void* x8, int64_t ldx, const float* a_scale, int32_t
                       int64_t ldw, const float* w_scale, int32_t w_scale_ld, void* q, int64_t ldq, float* scales,
                       int32_t scale_ld, int32_t m, int32_t cols, int32_t k, int32_t max_split, int32_t flags,
                       int32_t* status, void* stream);
+int mie_fp8_gemm_silu_wide_pays(int32_t m, int32_t cols, int32_t k, int32_t max_split);
+int mie_fp8_gemm_silu_wide(const void* x8, int64_t ldx, const float* a_scale, int32_t a_scale_ld, const void* w8,
+                           int64_t ldw, const float* w_scale, int32_t w_scale_ld, void* q, int64_t ldq, float* scales,
+                           int32_t scale_ld, int32_t m, int32_t cols, int32_t k, int32_t flags, int32_t* status,
+                           void* stream);
 int mie_fp8_gemm_qkv(const void* x8, int64_t ldx, const float* a_scale, int32_t a_scale_ld, const void* w8,
                      int64_t ldw, const float* w_scale, int32_t w_scale_ld, const void* q_weight,
                      const void* k_weight, const void* cos_sin, int32_t max_pos, mie_index_t positions,

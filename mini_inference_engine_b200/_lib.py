@@ -113,6 +113,10 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "mie_fp8_gemm_silu": (ctypes.c_int, [c_void_p, c_int64, c_void_p, c_int32, c_void_p, c_int64, c_void_p, c_int32,
                                          c_void_p, c_int64, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32,
                                          c_int32, c_void_p, c_void_p]),
+    "mie_fp8_gemm_silu_wide_pays": (ctypes.c_int, [c_int32, c_int32, c_int32, c_int32]),
+    "mie_fp8_gemm_silu_wide": (ctypes.c_int, [c_void_p, c_int64, c_void_p, c_int32, c_void_p, c_int64, c_void_p, c_int32,
+                                              c_void_p, c_int64, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32,
+                                              c_void_p, c_void_p]),
     "mie_fp8_gemm_qkv": (ctypes.c_int, [c_void_p, c_int64, c_void_p, c_int32, c_void_p, c_int64, c_void_p, c_int32,
                                         c_void_p, c_void_p, c_void_p, c_int32, IndexT, IndexT, IndexT, c_void_p,
                                         View4T, View4T, c_void_p, c_int64, c_void_p, c_int32, c_int32, c_int32,

@@ -587,6 +587,75 @@ __device__ __forceinline__ void wide_cluster_reduce(const GemmParams& p, uint32_
   }
 }
 
+// Finish::kSilu of the wide kernel: a tile has 128 gate columns and the 128 up columns that belong to them.  Warps w and
+// w + 8 have the gate and up values of the same 32 rows and 64 columns; each passes the other half of its columns and
+// finishes 32, whose largest value meets those of the row's three other warps.  The staging area holds 64 bytes a row and
+// warp: bf16 values for the partner, then, in the place a lane has just read, its maximum.
+__device__ __forceinline__ void wide_finish_silu(const GemmParams& p, const WideItem& it, const float (&acc)[64],
+                                                 uint8_t* stores, int warp, int lane, bool ok) {
+  const int quad = warp & 3, group = warp >> 2;
+  const bool gate = group < 2;  // keeps columns [0, 32) of its 64, the up warp [32, 64)
+  auto slot = [&](int w, int u) {
+    return reinterpret_cast<uint4*>(stores + w * 2048) + lane * 4 + ((u + (lane >> 1)) & 3);
+  };
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    uint32_t w[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int j = u * 8 + 2 * q;
+      w[q] = gate ? Mma16816<__nv_bfloat16>::pack(acc[32 + j], acc[33 + j]) : Mma16816<__nv_bfloat16>::pack(acc[j], acc[j + 1]);
+    }
+    *slot(warp, u) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 7)) : "memory");
+  float v[4][8], amax = 0.f;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    Bf16x8 theirs, mine, r;
+    theirs.raw = *slot(warp ^ 8, u);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int j = u * 8 + 2 * q;
+      mine.word[q] = gate ? Mma16816<__nv_bfloat16>::pack(acc[j], acc[j + 1]) : Mma16816<__nv_bfloat16>::pack(acc[32 + j], acc[33 + j]);
+    }
+    // The rounding points of the unfused chain: gate and up to bf16, SiLU to bf16, their product to bf16.
+    float g[8];
+    unpack8(gate ? mine.raw : theirs.raw, g);
+    gate8(g, 1.f, v[u]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      r.pair[q] = __hmul2_rn(__floats2bfloat162_rn(v[u][2 * q], v[u][2 * q + 1]), gate ? theirs.pair[q] : mine.pair[q]);
+    unpack8(r.raw, v[u]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[u][j]));
+  }
+  *reinterpret_cast<float*>(slot(warp ^ 8, 0)) = amax;
+  asm volatile("bar.sync %0, 128;" ::"r"(9 + quad) : "memory");
+#pragma unroll
+  for (int x = 0; x < 4; ++x) amax = fmaxf(amax, *reinterpret_cast<const float*>(slot(x * 4 + quad, 0)));
+  asm volatile("bar.sync %0, 128;" ::"r"(9 + quad) : "memory");  // before the next tile's values
+  const int row = it.tm * kTileR + quad * 32 + lane;
+  if (row >= p.m || !ok) return;
+  const float scale = __fdiv_rn(amax, 448.0f), denom = fmaxf(scale, 1e-12f);
+  uint8_t* dst = p.q + (long long)row * p.ldq + it.tn * 128 + (group & 1) * 64 + (gate ? 0 : 32);
+  const bool wide = ((reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
+#pragma unroll
+  for (int u = 0; u < 4; u += 2) {
+    uint32_t lo[2], hi[2];
+    quantize_values(v[u], denom, lo);
+    quantize_values(v[u + 1], denom, hi);
+    if (wide) {
+      *reinterpret_cast<uint4*>(dst + u * 8) = make_uint4(lo[0], lo[1], hi[0], hi[1]);
+    } else {
+      uint32_t* d = reinterpret_cast<uint32_t*>(dst + u * 8);
+      d[0] = lo[0], d[1] = lo[1], d[2] = hi[0], d[3] = hi[1];
+    }
+  }
+  if (group == 0) p.q_scales[(long long)it.tn * p.q_scale_ld + row] = scale;
+}
+
+template <Finish kFinish>
 __global__ void __launch_bounds__(kWideThreads, 1)
     fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                          const GemmParams p) {
@@ -629,8 +698,13 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     tma_load_2d(stage_base + (size_t)s * kStageBytes, &map_x, &full_bar[s], kb * kBlockK, it.tm * kTileR);
   };
   auto load_w = [&](uint32_t s, int kb, const WideItem& it) {
-    tma_load_2d(stage_base + (size_t)s * kStageBytes + kTileR * kBlockK, &map_w, &full_bar[s], kb * kBlockK,
-                it.tn * BN);
+    uint8_t* dst = stage_base + (size_t)s * kStageBytes + kTileR * kBlockK;
+    if constexpr (kFinish == Finish::kSilu) {  // boxes of 128 rows: gate, up
+      tma_load_2d(dst, &map_w, &full_bar[s], kb * kBlockK, it.tn * 128);
+      tma_load_2d(dst + 128 * kBlockK, &map_w, &full_bar[s], kb * kBlockK, p.n / 2 + it.tn * 128);
+    } else {
+      tma_load_2d(dst, &map_w, &full_bar[s], kb * kBlockK, it.tn * BN);
+    }
   };
   // Barriers, tensor-map prefetch and the TMEM allocation above overlap the tail of the previous kernel.
   // So can static weights (nothing on the stream writes them): the producer requests the weight half of its
@@ -729,15 +803,17 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     uint32_t n = 0;
     bool ok = true;
     WideItem it;
-    for (int idx = 0; ok && wide_item(p, idx, it); ++idx) {
+    // A failed wait only clears `ok` where warps meet at the end of a tile: all of them pass the same barriers.
+    constexpr bool kMeet = kFinish == Finish::kSilu;
+    for (int idx = 0; (ok || kMeet) && wide_item(p, idx, it); ++idx) {
       const int tok0 = it.tm * kTileR;
       // The scales of this thread's row and of its columns' weight block, requested a K block ahead.
-      const int blk = it.tn * 2 + col0 / 128;
+      const int blk = kFinish == Finish::kSilu ? it.tn + (col0 / 128) * (p.n / 256) : it.tn * 2 + col0 / 128;
       const bool row_live = tok0 + row_in_tile < p.m, col_live = blk * 128 < p.n;
       const float* a_at = p.a_scale + (long long)it.k0 * p.a_scale_ld + (row_live ? tok0 + row_in_tile : 0);
       const float* w_at = p.w_scale + (col_live ? (long long)blk * p.w_scale_ld : 0) + it.k0;
       float a_next = __ldg(a_at), w_next = __ldg(w_at);
-      for (int kb = it.k0; kb < it.k1; ++kb, ++n) {
+      for (int kb = it.k0; (ok || !kMeet) && kb < it.k1; ++kb, ++n) {
         const uint32_t taddr = lane_addr + (n & 1) * BN;
         if (!mbar_wait_bounded(&done_bar[n % kStages], (n / kStages) & 1u)) {
           raise_status(p.status, MIE_STATUS_WAIT_TIMEOUT);
@@ -762,10 +838,12 @@ __global__ void __launch_bounds__(kWideThreads, 1)
         if (lane == 0) mbar_arrive(&tmem_empty[n & 1]);
         promote32(acc + 32, buf, s);
       }
-      if (!ok) break;
+      if (!ok && !kMeet) break;
 
       const int r_glob = tok0 + row_in_tile;
-      if (split == 1) {
+      if constexpr (kFinish == Finish::kSilu) {
+        wide_finish_silu(p, it, acc, store_base, warp, lane, ok);
+      } else if (split == 1) {
         const int n0 = it.tn * BN + col0;
         const bool vec = (p.ldy % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.y) & 15) == 0) && (n0 + kCols <= p.n);
         if (vec) {
@@ -1114,6 +1192,7 @@ WidePlan plan_wide(long long tiles, int kb, int max_split) {
 
 int launch_wide_range(const CUtensorMap& mx, const CUtensorMap& mw, GemmParams p, int tile_begin, int tile_end,
                       int split, bool late_wait, bool tail_follows, cudaStream_t stream) {
+  const auto kernel = p.q != nullptr ? fp8_gemm_wide_kernel<Finish::kSilu> : fp8_gemm_wide_kernel<Finish::kStore>;
   p.tile_begin = tile_begin;
   p.band = wide_band(p.m, p.k);
   p.tile_end = tile_end;
@@ -1135,7 +1214,7 @@ int launch_wide_range(const CUtensorMap& mx, const CUtensorMap& mw, GemmParams p
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attr;
   config.numAttrs = chained_launch_enabled() ? 2 : 1;
-  MIE_CUDA(cudaLaunchKernelEx(&config, fp8_gemm_wide_kernel, mx, mw, p));
+  MIE_CUDA(cudaLaunchKernelEx(&config, kernel, mx, mw, p));
   MIE_LAUNCH_CHECK("fp8_gemm_wide_kernel");
   return MIE_OK;
 }
@@ -1146,13 +1225,15 @@ int launch_wide(const CUtensorMap& mx, const CUtensorMap& mw, const GemmParams& 
   int dev = 0;
   MIE_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    MIE_CUDA(cudaFuncSetAttribute(fp8_gemm_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kWideSmemBytes));
+    for (const void* kernel : {reinterpret_cast<const void*>(fp8_gemm_wide_kernel<Finish::kStore>),
+                               reinterpret_cast<const void*>(fp8_gemm_wide_kernel<Finish::kSilu>)})
+      MIE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmemBytes));
     configured[dev] = true;
   }
   const int kb = (p.k + kBlockK - 1) / kBlockK;
   const long long tiles = (long long)((p.m + kTileR - 1) / kTileR) * ((p.n + kWideBN - 1) / kWideBN);
   MIE_CHECK_ARG(tiles <= 0x7fffffff, "too many output tiles (%lld)", tiles);
+  if (p.q != nullptr) return launch_wide_range(mx, mw, p, 0, (int)tiles, 1, false, false, stream);  // whole tiles only
   const WidePlan plan = plan_wide(tiles, kb, max_split);
   if (int rc = launch_wide_range(mx, mw, p, 0, plan.main_tiles, plan.main_split, false, plan.tail_split > 0, stream)) return rc;
   if (plan.tail_split > 0) {
@@ -1241,6 +1322,47 @@ extern "C" int mie_fp8_gemm_finishes(int32_t m, int32_t n) { return m >= 1 && n 
 
 extern "C" int mie_fp8_gemm_finish_pays(int32_t m, int32_t n, int32_t k, int32_t gated, int32_t max_split) {
   return m >= 1 && n >= 1 && k >= 1 && finish_pays(m, n, k, gated != 0, max_split) ? 1 : 0;
+}
+
+// Whether the wide kernel should finish the gated rows itself.  It saves a launch and the rows' way through memory, but the
+// tensor core has two K blocks to go on with while a tile is finished (about 3 us), and a tail of tiles is not cut.  Measured
+// (us, separate / finished), weights [gate | up] of 9728 columns each, K 2560: 96 tokens 17.4 / 16.1, 560 44.8 / 43.4, 1024
+// (cut tail) 71.7 / 69.0, 4096 252.8 / 241.1, but 8192 512 / 536 and 12032 733 / 766: over 24 rounds only with a long K
+// (12288, K 4096, 12032 tokens 1486 / 1421).  A cut tail matters in the first rounds (9728, 200 tokens 28.5 / 29.3) and with a
+// long K (12288, K 4096, 1024 tokens 120 / 126).
+static bool wide_silu_pays(int m, int cols, int k, int max_split) {
+  const long long tiles = (long long)((m + kTileR - 1) / kTileR) * (cols / 128);
+  const int kb = (k + kBlockK - 1) / kBlockK;
+  if (cols % 128 != 0 || narrow_fits(m, 2 * cols) || tiles > 0x7fffffff) return false;
+  const WidePlan plan = plan_wide(tiles, kb, max_split);
+  if (plan.main_split > 1 || (tiles > 24ll * sm_count() && kb < 32)) return false;
+  return plan.tail_split == 0 || (plan.main_tiles >= 2 * sm_count() && kb <= 24);
+}
+
+extern "C" int mie_fp8_gemm_silu_wide_pays(int32_t m, int32_t cols, int32_t k, int32_t max_split) {
+  return m >= 1 && cols >= 1 && k >= 1 && wide_silu_pays(m, cols, k, max_split) ? 1 : 0;
+}
+
+extern "C" int mie_fp8_gemm_silu_wide(const void* x8, int64_t ldx, const float* a_scale, int32_t a_scale_ld,
+                                      const void* w8, int64_t ldw, const float* w_scale, int32_t w_scale_ld, void* q,
+                                      int64_t ldq, float* scales, int32_t scale_ld, int32_t m, int32_t cols, int32_t k,
+                                      int32_t flags, int32_t* status, void* stream) {
+  MIE_CHECK_ARG(q && scales, "null pointer");
+  MIE_CHECK_ARG(cols >= 128 && cols % 128 == 0 && cols <= 0x3fffffff, "cols must be a multiple of 128");
+  GemmParams p;
+  if (int rc = gemm_params(p, x8, ldx, a_scale, a_scale_ld, w8, ldw, w_scale, w_scale_ld, m, 2 * cols, k, flags, status))
+    return rc;
+  MIE_CHECK_ARG(scale_ld >= m && ldq >= cols && ldq % 4 == 0 && (reinterpret_cast<uintptr_t>(q) & 3) == 0,
+                "the quantised rows must be 4-byte aligned and have scale storage");
+  if (m == 0) return MIE_OK;
+  p.q = (uint8_t*)q;
+  p.ldq = ldq;
+  p.q_scales = scales;
+  p.q_scale_ld = scale_ld;
+  CUtensorMap mw, mx;
+  if (int rc = operand_map(x8, m, k, ldx, kTileR, &mx)) return rc;
+  if (int rc = operand_map(w8, 2 * cols, k, ldw, 128, &mw)) return rc;
+  return launch_wide(mx, mw, p, 1, (cudaStream_t)stream);
 }
 
 extern "C" int mie_fp8_gemm_silu(const void* x8, int64_t ldx, const float* a_scale, int32_t a_scale_ld, const void* w8,

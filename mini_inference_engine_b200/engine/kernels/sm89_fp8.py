@@ -237,10 +237,20 @@ def finishes_rows(weight: torch.Tensor, m: int, *, gated: bool) -> bool:
     which only models made for tests have, keep the separate launches and the ten launches a layer that their steps report
     (two layers of width 512 77 to 79 us either way)."""
 
+    return _read_in_place(weight) and bool(_lib.load().mie_fp8_gemm_finish_pays(
+        m, int(weight.shape[0]), int(weight.shape[1]), int(gated), _DEFAULT_MAX_SPLIT))
+
+
+def finishes_wide_rows(weight: torch.Tensor, m: int) -> bool:
+    """The same of a merged gate_up weight and the kernel for long steps (``mie_fp8_gemm_silu_wide``)."""
+
+    return _read_in_place(weight) and bool(_lib.load().mie_fp8_gemm_silu_wide_pays(
+        m, int(weight.shape[0]) // 2, int(weight.shape[1]), _DEFAULT_MAX_SPLIT))
+
+
+def _read_in_place(weight: torch.Tensor) -> bool:
     return (weight.numel() >= FINISH_MIN_WEIGHT and weight.stride(1) == 1 and weight.stride(0) % 16 == 0
-            and weight.data_ptr() % 16 == 0
-            and bool(_lib.load().mie_fp8_gemm_finish_pays(m, int(weight.shape[0]), int(weight.shape[1]), int(gated),
-                                                          _DEFAULT_MAX_SPLIT)))
+            and weight.data_ptr() % 16 == 0)
 
 
 def default_max_split() -> int:

@@ -387,18 +387,22 @@ class Qwen3DecodeRunner(PagedStepRunner):
         return q, scales
 
     def _gated_quantized(self, quantized, layer, rows: int):
-        """The merged gate_up projection and SiLU(gate) * up, quantised for down_proj: one launch for a decode batch."""
+        """The merged gate_up projection and SiLU(gate) * up, quantised for down_proj: one launch where that is faster."""
 
         weight, inter = layer.gate_up, self.local_inter
-        if not sm89_fp8.finishes_rows(weight, rows, gated=True):
+        narrow = sm89_fp8.finishes_rows(weight, rows, gated=True)
+        if not narrow and not sm89_fp8.finishes_wide_rows(weight, rows):
             return self._silu_mul_quantized(self._gemm(quantized, weight, layer.gate_up_scale, rows, self.shape.hidden),
                                             rows)
         q, scales = self._quant_buffers(rows, inter)
-        _lib.check(_lib.load().mie_fp8_gemm_silu(
-            _lib.ptr(quantized[0]), quantized[0].stride(0), _lib.ptr(quantized[1]), quantized[1].stride(0),
-            _lib.ptr(weight), weight.stride(0), _lib.ptr(layer.gate_up_scale), layer.gate_up_scale.stride(0), _lib.ptr(q),
-            q.stride(0), _lib.ptr(scales), scales.stride(0), rows, inter, self.shape.hidden,
-            sm89_fp8.default_max_split(), _lib.GEMM_STATIC_WEIGHTS, _lib.ptr(self.status), _lib.stream_arg(self.device)))
+        operands = (_lib.ptr(quantized[0]), quantized[0].stride(0), _lib.ptr(quantized[1]), quantized[1].stride(0),
+                    _lib.ptr(weight), weight.stride(0), _lib.ptr(layer.gate_up_scale), layer.gate_up_scale.stride(0),
+                    _lib.ptr(q), q.stride(0), _lib.ptr(scales), scales.stride(0), rows, inter, self.shape.hidden)
+        last = (_lib.GEMM_STATIC_WEIGHTS, _lib.ptr(self.status), _lib.stream_arg(self.device))
+        if narrow:
+            _lib.check(_lib.load().mie_fp8_gemm_silu(*operands, sm89_fp8.default_max_split(), *last))
+        else:
+            _lib.check(_lib.load().mie_fp8_gemm_silu_wide(*operands, *last))
         return q, scales
 
     def _row_parallel_then_norm(self, quantized, weight, weight_scale, rows: int, k: int, residual, norm_weight,

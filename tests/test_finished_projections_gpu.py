@@ -160,3 +160,26 @@ def test_repeated_products_are_identical(m, n, k, device, status_clean):
         flush.zero_()
         different += (_product(q, scales, w8, w_scale, m, k, 0) != first).any()
     assert int(different.item()) == 0
+
+
+# Token tiles that are whole, ragged and single; more tiles than SMs; K of one block, two, and one with a tail.
+WIDE = [(m, cols, k) for m in (1, 128, 129, 300) for cols, k in ((128, 128), (384, 256), (640, 2032))] + [(1000, 2560, 384)]
+
+
+@pytest.mark.parametrize("m,cols,k", WIDE)
+def test_gated_rows_of_long_steps(m, cols, k, device, status_clean):
+    """The same sums in the same order as the product that is not cut, and the same rounding points: equal bits."""
+
+    q, scales, w8, w_scale = _operands(m, 2 * cols, k, device)
+    lib, stream, groups = _lib.load(), _lib.stream_arg(device), cols // 128
+    got, got_s = torch.zeros(m, cols, dtype=torch.uint8, device=device), torch.zeros(groups, m + 2, device=device)
+    for _ in range(3):
+        _lib.check(lib.mie_fp8_gemm_silu_wide(
+            _lib.ptr(q), q.stride(0), _lib.ptr(scales), scales.stride(0), _lib.ptr(w8), w8.stride(0), _lib.ptr(w_scale),
+            w_scale.stride(0), _lib.ptr(got), cols, _lib.ptr(got_s), m + 2, m, cols, k, 0,
+            _lib.ptr(_lib.status_word(device)), stream))
+    both = _product(q, scales, w8, w_scale, m, k, 1)
+    want, want_s = torch.zeros_like(got), torch.zeros_like(got_s)
+    _lib.check(lib.mie_silu_mul(_lib.ptr(both), _lib.ptr(both[:, cols:]), 2 * cols, None, _lib.ptr(want), cols,
+                                _lib.ptr(want_s), m + 2, m, cols, stream))
+    assert torch.equal(got, want) and torch.equal(got_s, want_s)
