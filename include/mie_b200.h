@@ -158,7 +158,9 @@ int64_t mie_decode_scratch_bytes(int32_t batch, int32_t q_heads, int32_t kv_head
  * split_policy: 0 = one work item per (request, KV head) (no split-KV);
  *               1 = length-proportional split-KV chosen on the device from the
  *                   batch's total length (the partials are merged by a second
- *                   kernel); > 1 = fixed chunk of that many tokens (multiple of 16).
+ *                   kernel; few requests or short tables have a cluster per
+ *                   KV head that merges by itself); > 1 = fixed chunk of that
+ *                   many tokens (multiple of 16).
  * scratch: device buffer of at least mie_decode_scratch_bytes(...) bytes,
  * 256-byte aligned; contents need not be initialised.  plan_only / use_plan
  * let a model step build the work plan once (layer 0) and reuse it for the
