@@ -60,7 +60,7 @@ __device__ __forceinline__ float corrected_quotient(float a, float b, float y) {
 // g / (1 + exp(-slope g)).
 __device__ __forceinline__ float gate_sigmoid(float g, float slope = 1.f) { return g / (1.f + expf(-slope * g)); }
 
-// The same from the approximate exponential and reciprocal, for results that are rounded to 16 bits: within 2^-20 of the
+// The same from the approximate exponential and reciprocal, for results that are rounded to 16 bits: within 2^-18 of the
 // quotient, and SiLU (slope 1) of every bf16 value is rounded to what the quotient is.  slope_log2e = slope * log2 e.
 // `denominator` above kGateLimit, whose reciprocal is flushed to zero, takes the quotient instead.
 constexpr float kGateLimit = 5e37f, kLog2e = 1.4426950408889634f;

@@ -132,7 +132,7 @@ __device__ __forceinline__ float gelu_tanh(float z) {
   return 0.5f * z * (1.f + tanhf(inner));
 }
 
-// The same as z / (1 + exp(-2 inner)) with the approximate exponential and reciprocal, for 16-bit results: within 2^-20, and
+// The same as z / (1 + exp(-2 inner)) with the approximate exponential and reciprocal, for 16-bit results: within 2^-18, and
 // without the cancellation of 1 + tanh at negative z.
 __device__ __forceinline__ float gelu_tanh16(float z) {
   const float inner = 0.7978845608028654f * (z + 0.044715f * z * z * z);
