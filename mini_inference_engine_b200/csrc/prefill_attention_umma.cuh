@@ -543,35 +543,42 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_fence_after();
     const int d0 = v_box0 * 64;  // first output dim of this pass
     if (ranks == 1) {
-      // Rows through shared memory (over Q, which is done with), so that VH * 8 lanes write one together.
+      // Rows through shared memory, so that the lanes of a row write it together: over this query tile's own Q, which is
+      // done with, in passes where it is narrower than the output (the other tile may still have products to come).
       const float inv = 1.f / fmaxf(l, 1.17549435e-38f);
       const long long own_o = (q_begin + first_tok + (row_live ? tok_local : 0)) * p.o_st +
                               (long long)(kvh * p.group + (row_live ? head_local : 0)) * p.o_sh;
-      constexpr int kChunks = VH * 8;
+      constexpr int kGroups = KH < VH ? KH : VH, kChunks = kGroups * 8;  // of a pass: 64-dim groups, 16-byte chunks a row
+      static_assert(VH % kGroups == 0 && kRows * kChunks * 16 <= Tile::kQTile, "a pass fits the tile's own Q");
       if (ok && n_own > 0) {
-        uint8_t* rows = smem + t * (kRows * kChunks * 16) + quad * (32 * kChunks * 16);
+        uint8_t* rows = smem + t * Tile::kQTile + quad * (32 * kChunks * 16);
 #pragma unroll 1
-        for (int c = 0; c < VH * 64; c += 32) {
-          float ov[32];
-          tmem_ld32(tmem_o + c, ov);
-          tmem_ld_wait();
+        for (int first = 0; first < VH * 64; first += kGroups * 64) {
+          if (first > 0) __syncwarp();  // the last pass's rows have been read
+#pragma unroll 1
+          for (int c = 0; c < kGroups * 64; c += 32) {
+            float ov[32];
+            tmem_ld32(tmem_o + first + c, ov);
+            tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint32_t w[4];
+            for (int i = 0; i < 32; i += 8) {
+              uint32_t w[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) w[q] = Mma16816<T>::pack(ov[i + 2 * q] * inv, ov[i + 2 * q + 1] * inv);
-            *reinterpret_cast<uint4*>(rows + (lane * kChunks + (((c + i) / 8 ^ lane) & (kChunks - 1))) * 16) =
-                make_uint4(w[0], w[1], w[2], w[3]);
+              for (int q = 0; q < 4; ++q) w[q] = Mma16816<T>::pack(ov[i + 2 * q] * inv, ov[i + 2 * q + 1] * inv);
+              *reinterpret_cast<uint4*>(rows + (lane * kChunks + (((c + i) / 8 ^ lane) & (kChunks - 1))) * 16) =
+                  make_uint4(w[0], w[1], w[2], w[3]);
+            }
           }
-        }
-        __syncwarp();
+          __syncwarp();
+          const int d = d0 + first;
 #pragma unroll 4
-        for (int i = lane; i < 32 * kChunks; i += 32) {
-          const int x = i / kChunks, c = i % kChunks;
-          const long long at = __shfl_sync(0xffffffffu, own_o, x);
-          if ((live_rows >> x & 1) && (!kExt || d0 + c * 8 < p.vdim))
-            *reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.out) + at + d0 + c * 8) =
-                *reinterpret_cast<const uint4*>(rows + (x * kChunks + ((c ^ x) & (kChunks - 1))) * 16);
+          for (int i = lane; i < 32 * kChunks; i += 32) {
+            const int x = i / kChunks, c = i % kChunks;
+            const long long at = __shfl_sync(0xffffffffu, own_o, x);
+            if ((live_rows >> x & 1) && (!kExt || d + c * 8 < p.vdim))
+              *reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.out) + at + d + c * 8) =
+                  *reinterpret_cast<const uint4*>(rows + (x * kChunks + ((c ^ x) & (kChunks - 1))) * 16);
+          }
         }
       }
     } else {
