@@ -381,7 +381,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           __syncwarp();
         }
         if (ok && j + 1 < n_own) {
-          if (kKStages == 1 && t == 0) ok = warp_wait_bounded(&bars[kKFull], k_parity);
+          // One stage: K(j + 1) could not be waited for above, where S(1, j) had yet to read K(j).  The first query tile to
+          // use it waits, which is the second one when the first has had its last K/V tile.
+          if (kKStages == 1 && (t == 0 || j + 1 >= n0)) ok = warp_wait_bounded(&bars[kKFull], k_parity);
           if (ok) issue_s(t, ks, last);
         }
       }

@@ -24,3 +24,18 @@ def test_narrow_keys(sizes, window, device):
     for _ in range(3):
         case.prefill(device)
         case.check()
+
+
+# Keys that leave shared memory for one K stage: three and four 64-dim groups, one and two query heads a key/value head.
+WIDE_KEYS = [(3, 3, 192, 128), (4, 2, 192, 128), (3, 3, 256, 256)]
+
+
+@pytest.mark.parametrize("window", [None, 300])
+@pytest.mark.parametrize("sizes", WIDE_KEYS, ids=str)
+def test_wide_keys(sizes, window, device):
+    """The last K/V tile of a pair is seen by its second query tile alone."""
+
+    case = Case(LENGTHS, CHUNKS, *sizes, window, 16, torch.bfloat16, seed=32)
+    for _ in range(3):
+        case.prefill(device)
+        case.check()
