@@ -807,12 +807,13 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     constexpr bool kMeet = kFinish == Finish::kSilu;
     for (int idx = 0; (ok || kMeet) && wide_item(p, idx, it); ++idx) {
       const int tok0 = it.tm * kTileR;
-      // The scales of this thread's row and of its columns' weight block, requested a K block ahead.
+      // The scales of this thread's row and of its columns' weight block, requested a K block ahead.  Ordinary loads: the
+      // kernel before may have written them while this one was waiting, which the read-only path does not allow for.
       const int blk = kFinish == Finish::kSilu ? it.tn + (col0 / 128) * (p.n / 256) : it.tn * 2 + col0 / 128;
       const bool row_live = tok0 + row_in_tile < p.m, col_live = blk * 128 < p.n;
       const float* a_at = p.a_scale + (long long)it.k0 * p.a_scale_ld + (row_live ? tok0 + row_in_tile : 0);
       const float* w_at = p.w_scale + (col_live ? (long long)blk * p.w_scale_ld : 0) + it.k0;
-      float a_next = __ldg(a_at), w_next = __ldg(w_at);
+      float a_next = *a_at, w_next = *w_at;
       for (int kb = it.k0; (ok || !kMeet) && kb < it.k1; ++kb, ++n) {
         const uint32_t taddr = lane_addr + (n & 1) * BN;
         if (!mbar_wait_bounded(&done_bar[n % kStages], (n / kStages) & 1u)) {
@@ -824,8 +825,8 @@ __global__ void __launch_bounds__(kWideThreads, 1)
         const float s = a_next * w_next;
         a_at += kb + 1 < it.k1 ? p.a_scale_ld : 0;
         w_at += kb + 1 < it.k1 ? 1 : 0;
-        a_next = __ldg(a_at);
-        w_next = __ldg(w_at);
+        a_next = *a_at;
+        w_next = *w_at;
         float buf[32];
         tmem_ld32(taddr, buf);
         tmem_ld_wait_pin(buf);
@@ -936,8 +937,8 @@ __global__ void __launch_bounds__(kWideThreads, 1)
 // division it was bound by instructions (12032 x 4096: 52.4 us, now 39.7 us).
 // --------------------------------------------------------------------------
 template <typename T, typename Index>
-__global__ void quantize_kernel(const T* __restrict__ x, long long ldx, uint8_t* __restrict__ q, long long ldq,
-                                float* __restrict__ scales, int scale_ld, int m, int k) {
+__global__ void quantize_kernel(const T* x, long long ldx, uint8_t* q, long long ldq, float* scales, int scale_ld,
+                                int m, int k) {
   chain_release();
   chain_wait();
   const Index groups = (Index)((k + 127) / 128);
