@@ -585,8 +585,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     } else {
       // This rank's part of the softmax: O rows over Q and the rings (both query tiles' products are done with them),
-      // 16-byte chunks swizzled by the row; reference maximum and sum behind them.  A rank that saw no key of a row, or
-      // whose wait failed, counts for nothing.
+      // 16-byte chunks swizzled by the row; reference maximum and sum behind them.  A rank that had no K/V tile for a query
+      // tile, or whose wait failed, counts for nothing.
       constexpr int kChunks = VH * 16, kORow = VH * 256;
       asm volatile("bar.sync 1, 256;" ::: "memory");
       uint8_t* mine = smem + t * (kRows * kORow);
@@ -603,28 +603,31 @@ __global__ void __launch_bounds__(kThreads, 1)
               make_float4(ov[4 * i], ov[4 * i + 1], ov[4 * i + 2], ov[4 * i + 3]);
       }
       *reinterpret_cast<float4*>(smem + Tile::kOffState + (t * kRows + row) * 16) =
-          make_float4(counts ? m_ref : -INFINITY, counts ? l : 0.f, 0.f, 0.f);
+          make_float4(counts ? m_ref : -INFINITY, counts ? l : 0.f, counts ? 1.f : 0.f, 0.f);
       __syncwarp();
       cluster_sync_all();
       const uint32_t local = smem_u32(smem);
       float* weights = reinterpret_cast<float*>(smem + Tile::kOffWeight);
-      {  // what each rank's row counts for in the result, a thread a row
-        float top = -INFINITY, sum = 0.f, m[kMaxSplit], l[kMaxSplit];
+      {  // what each rank's row counts for in the result, a thread a row; -1: it has no such row
+        float top = -INFINITY, sum = 0.f;
+        float4 v[kMaxSplit];  // reference maximum, sum, whether it counts
 #pragma unroll
         for (int i = 0; i < kMaxSplit; ++i) {
-          const float4 v = i < ranks ? ld_cluster_f4(local + Tile::kOffState + threadIdx.x * 16, i)
-                                     : make_float4(-INFINITY, 0.f, 0.f, 0.f);
-          m[i] = v.x, l[i] = v.y;
-          top = fmaxf(top, m[i]);
+          v[i] = i < ranks ? ld_cluster_f4(local + Tile::kOffState + threadIdx.x * 16, i)
+                           : make_float4(-INFINITY, 0.f, 0.f, 0.f);
+          top = fmaxf(top, v[i].x);
         }
+        // A rank whose keys are all hidden from the row, or all NaN, has -inf as its maximum: the weight is 0, and what is
+        // not a number in its sum (or, below, in its values) still reaches the result, as it does without a split.
 #pragma unroll
         for (int i = 0; i < kMaxSplit; ++i) {
-          m[i] = m[i] == -INFINITY ? 0.f : ex2_approx(m[i] - top);
-          sum += l[i] * m[i];
+          v[i].x = v[i].x == -INFINITY ? 0.f : ex2_approx(v[i].x - top);
+          sum += v[i].y * v[i].x;
         }
-        const float inv = 1.f / fmaxf(sum, 1.17549435e-38f);
+        const float inv = sum != sum ? sum : 1.f / fmaxf(sum, 1.17549435e-38f);
 #pragma unroll
-        for (int i = 0; i < kMaxSplit; ++i) weights[i * (kTiles * kRows) + threadIdx.x] = m[i] * inv;
+        for (int i = 0; i < kMaxSplit; ++i)
+          weights[i * (kTiles * kRows) + threadIdx.x] = v[i].z != 0.f ? v[i].x * inv : -1.f;
       }
       asm volatile("bar.sync 1, 256;" ::: "memory");
       // VH * 16 lanes combine a row, 4 dims a lane; the ranks share the live rows.  A remote load takes about 1,300 clocks,
@@ -651,7 +654,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int i = 0; i < kRanks; ++i) {
               const float w = weights[i * (kTiles * kRows) + x[b]];
-              if (w != 0.f)  // no such rank, or it left no row
+              if (!(w < 0.f))
                 o.x += v[b][i].x * w, o.y += v[b][i].y * w, o.z += v[b][i].z * w, o.w += v[b][i].w * w;
             }
             if (y0 + b * ranks * kStep >= live || (kExt && d >= p.vdim)) continue;

@@ -47,3 +47,21 @@ def test_ranks_with_sinks_and_windows(spans, sizes, sinks, device):
     case = Case([n for n, _ in spans], [c for _, c in spans], *sizes, 16, torch.bfloat16, seed=12, sinks=sinks)
     case.prefill(device)
     case.check()
+
+
+# Groups of one and four heads, five to eight ranks; with NaN queries a rank has nothing but -inf as its maximum.
+@pytest.mark.parametrize("sizes", [(4, 4, 128, 128), (8, 2, 64, 64)], ids=str)
+def test_what_is_no_number_reaches_the_result(sizes, device):
+    """As without a split: a NaN query gives a NaN row, an infinite value no finite number, whatever its weight."""
+
+    case = Case([2600], [24], *sizes, None, 16, torch.bfloat16, seed=13, sinks="none")
+    case.queries[0][5] = float("nan")
+    page, slot = int(case.tables[0, 3]), 7  # a token of the first rank, and one that all but a few ranks lie behind
+    case.values[page, :, slot, 10] = float("inf")
+    case.keys[page, :, slot] *= 0.0
+    case.prefill(device)
+    bad = ~torch.isfinite(case.out.cpu().float())
+    want = torch.zeros_like(bad)
+    want[5] = True
+    want[..., 10] = True
+    assert torch.equal(bad, want) and bool(case.out[5].isnan().all())
