@@ -269,9 +269,10 @@ __global__ void qkv_mix_kernel(QkvMixParams p) {
 
 // ---------------------------------------------------------------------------
 // Clamped gated activation: g = min(gate, limit), u = clamp(up, -limit, limit),
-// out = g * sigmoid(slope * g) * (u + up_offset).  HBM-bound (6 bytes a result in bf16) with the gates of gate8 and a 32-bit
-// index: 9000 x 12288 in bf16 146 us with an IEEE division and a 64-bit one, 136 with corrected quotients, now 118.  fp32
-// results keep the division.
+// out = g * sigmoid(slope * g) * (u + up_offset).  HBM-bound (6 bytes a result in bf16) with a corrected quotient and a
+// 32-bit index: 9000 x 12288 in bf16 146 us with an IEEE division and a 64-bit one, now 136 us.  fp32 results keep the
+// division.  (With SiLU's approximate exponential and reciprocal it takes 118 us and is further off: at slope 0.9 twelve of
+// 400,000 results on the wrong side of a tie instead of three.)
 // ---------------------------------------------------------------------------
 template <typename T, int VEC, typename Index>
 __global__ void clamped_glu_kernel(const T* gate, const T* up, long long ld_in, T* out, long long ldo, int rows,
@@ -287,16 +288,10 @@ __global__ void clamped_glu_kernel(const T* gate, const T* up, long long ld_in, 
   Vec<T, VEC>::load(gate + row * ld_in + c, g);
   Vec<T, VEC>::load(up + row * ld_in + c, u);
 #pragma unroll
-  for (int j = 0; j < VEC; ++j) g[j] = fminf(g[j], limit);
-  float f[VEC];
-  if constexpr (VEC == 8 && sizeof(T) == 2) {
-    gate8(g, slope, f);
-  } else {
-#pragma unroll
-    for (int j = 0; j < VEC; ++j) f[j] = gate_sigmoid(g[j], slope);
+  for (int j = 0; j < VEC; ++j) {
+    const float a = fminf(g[j], limit), b = fminf(fmaxf(u[j], -limit), limit) + up_offset;
+    g[j] = (sizeof(T) == 2 ? gate_sigmoid16(a, slope) : gate_sigmoid(a, slope)) * b;
   }
-#pragma unroll
-  for (int j = 0; j < VEC; ++j) g[j] = f[j] * (fminf(fmaxf(u[j], -limit), limit) + up_offset);
   Vec<T, VEC>::store(out + row * ldo + c, g);
 }
 

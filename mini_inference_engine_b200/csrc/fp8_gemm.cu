@@ -622,7 +622,7 @@ __device__ __forceinline__ void wide_finish_silu(const GemmParams& p, const Wide
     // The rounding points of the unfused chain: gate and up to bf16, SiLU to bf16, their product to bf16.
     float g[8];
     unpack8(gate ? mine.raw : theirs.raw, g);
-    gate8(g, 1.f, v[u]);
+    silu8(g, v[u]);
 #pragma unroll
     for (int q = 0; q < 4; ++q)
       r.pair[q] = __hmul2_rn(__floats2bfloat162_rn(v[u][2 * q], v[u][2 * q + 1]), gate ? theirs.pair[q] : mine.pair[q]);

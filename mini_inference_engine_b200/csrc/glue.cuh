@@ -60,13 +60,22 @@ __device__ __forceinline__ float corrected_quotient(float a, float b, float y) {
 // g / (1 + exp(-slope g)).
 __device__ __forceinline__ float gate_sigmoid(float g, float slope = 1.f) { return g / (1.f + expf(-slope * g)); }
 
-// The same from the approximate exponential and reciprocal, for results that are rounded to 16 bits: within 2^-18 of the
-// quotient, and SiLU (slope 1) of every bf16 value is rounded to what the quotient is.  slope_log2e = slope * log2 e.
-// `denominator` above kGateLimit, whose reciprocal is flushed to zero, takes the quotient instead.
+// The same for a result that is rounded to 16 bits: a corrected quotient.
+__device__ __forceinline__ float gate_sigmoid16(float g, float slope) {
+  const float d = 1.f + expf(-slope * g);
+  // a reciprocal near or below the smallest normal number, an infinite gate
+  if (d > 1e37f || fabsf(g) > 3.4e38f) return __fdiv_rn(g, d);
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  return corrected_quotient(g, d, y);
+}
+
+// g / (1 + 2^e) from the approximate exponential and reciprocal, each within about 2^-22; a relative error of e carries over
+// as |e| ln 2 times as much.  The reciprocal of a denominator above kGateLimit is flushed to zero.
 constexpr float kGateLimit = 5e37f, kLog2e = 1.4426950408889634f;
-__device__ __forceinline__ float gate_denominator(float g, float slope_log2e) {
+__device__ __forceinline__ float gate_denominator(float e) {
   float t;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(g * -slope_log2e));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(e));
   return 1.f + t;
 }
 __device__ __forceinline__ float gate_quotient(float g, float denominator) {
@@ -74,22 +83,23 @@ __device__ __forceinline__ float gate_quotient(float g, float denominator) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(denominator));
   return g * y;
 }
+// SiLU of a bf16 value, to be rounded to bf16: every one of the 65,536 comes out as the division's result does, though before
+// the rounding the error grows with the gate, 2^-17 at -88.
 __device__ __forceinline__ float silu16(float g) {
-  const float d = gate_denominator(g, kLog2e);
+  const float d = gate_denominator(g * -kLog2e);
   return d > kGateLimit ? gate_sigmoid(g) : gate_quotient(g, d);
 }
-// Eight values with one test for all of them.
-__device__ __forceinline__ void gate8(const float (&g)[8], float slope, float (&f)[8]) {
+// Eight of them with one test for all.
+__device__ __forceinline__ void silu8(const float (&g)[8], float (&f)[8]) {
   float top = 0.f;  // NaN passes the test and comes through the quotient
-  const float k = slope * kLog2e;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    f[j] = gate_denominator(g[j], k);
+    f[j] = gate_denominator(g[j] * -kLog2e);
     top = fmaxf(top, f[j]);
   }
   const bool plain = top <= kGateLimit;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) f[j] = plain ? gate_quotient(g[j], f[j]) : gate_sigmoid(g[j], slope);
+  for (int j = 0; j < 8; ++j) f[j] = plain ? gate_quotient(g[j], f[j]) : gate_sigmoid(g[j]);
 }
 
 // v[0..n) / denom as e4m3, two values per 16 bits.  denom >= 1e-12; quotients that e4m3 does not round to zero are exact

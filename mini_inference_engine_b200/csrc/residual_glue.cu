@@ -132,11 +132,14 @@ __device__ __forceinline__ float gelu_tanh(float z) {
   return 0.5f * z * (1.f + tanhf(inner));
 }
 
-// The same as z / (1 + exp(-2 inner)) with the approximate exponential and reciprocal, for 16-bit results: within 2^-18, and
-// without the cancellation of 1 + tanh at negative z.
+// The same as z / (1 + exp(-2 inner)) with the approximate exponential and reciprocal, for 16-bit results, and without the
+// cancellation of 1 + tanh at negative z.  The error is that of the exponent, four or five roundings of a number that grows
+// with z: 2^-21 at |z| <= 1, 2^-17 at -9.  Against 64 bits, over all bf16 z in [-10, 10] and 200 factors of a table each, 31 of
+// 1.2 million results are rounded to the other side (all by a tie's width, 0.5003 units), with tanhf 29,092, up to 256 units
+// off.  Below -10 the result is -0, where it would be 1e-37 and less.
 __device__ __forceinline__ float gelu_tanh16(float z) {
   const float inner = 0.7978845608028654f * (z + 0.044715f * z * z * z);
-  return gate_quotient(z, gate_denominator(inner, 2.f * kLog2e));
+  return gate_quotient(z, gate_denominator(inner * (-2.f * kLog2e)));
 }
 
 // Bound by HBM (4 bytes an entry in bf16) with few instructions: tanhf and a 64-bit index division an item took 10000 x 6144

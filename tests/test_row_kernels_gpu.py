@@ -158,3 +158,52 @@ def test_clamped_gates_are_ieee_quotients(slope, device):
     got = clamped_glu(both, limit=float("inf"), slope=slope, up_offset=1.0)
     want = gate / (1.0 + torch.exp(-slope * gate))
     assert torch.equal(got, want)
+
+
+def _bf16_values(low: float, high: float, count: int) -> torch.Tensor:
+    values = torch.arange(65536, dtype=torch.int32).to(torch.uint16).view(torch.bfloat16)
+    values = values[(values.float() >= low) & (values.float() <= high)]
+    return values[:values.numel() // count * count]
+
+
+def _units(got: torch.Tensor, want: torch.Tensor) -> torch.Tensor:
+    """Errors in units in the last bf16 place."""
+
+    unit = torch.exp2(torch.floor(torch.log2(want.abs().clamp_min(2.0 ** -126))) - 7)
+    return (got.cpu().double() - want).abs() / unit
+
+
+@pytest.mark.parametrize("slope", [1.0, 1.702, 0.9, 4.0])
+def test_clamped_gates_are_those_of_the_quotient(slope, device):
+    """Every bf16 gate whose exponential is finite: half a unit and the fp32 chain's roundings of the exponent (one, which
+    |slope g| enlarges), the exponential (two units), the quotient and the product; and the same bits for rows that only
+    16-bit accesses fit."""
+
+    from mini_inference_engine_b200.engine.kernels.decoder_glue import clamped_glu
+
+    gates = _bf16_values(-80.0 / slope, 9.0, 8).expand(16, -1)
+    ups = torch.randn(gates.shape, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16) * 4
+    got = clamped_glu(torch.cat([gates, ups], 1).to(device), limit=7.0, slope=slope, up_offset=1.0)
+    z = gates.double().clamp(max=7.0)
+    scaled = torch.tensor(slope).double() * z
+    want = z / (1.0 + torch.exp(-scaled)) * (ups.double().clamp(-7.0, 7.0) + 1.0)
+    assert (_units(got, want) <= 0.5 + 256 * (scaled.abs() + 8) * 2.0 ** -24).all()
+    odd = clamped_glu(torch.cat([gates[:, :-3], ups[:, :-3]], 1).to(device), limit=7.0, slope=slope, up_offset=1.0)
+    assert torch.equal(odd, got[:, :-3])
+
+
+def test_gelu_of_any_value(device):
+    """Every bf16 value down to where the result is flushed: half a unit and five roundings of the exponent 2 |inner|."""
+
+    from mini_inference_engine_b200.engine.kernels.decoder_glue import gelu
+
+    z = _bf16_values(-9.5, 40.0, 8)
+    wide = z.double()
+    inner = 0.7978845608028654 * (wide + 0.044715 * wide ** 3)
+    want = wide / (1.0 + torch.exp(-2.0 * inner))
+    status = torch.zeros(1, dtype=torch.int32, device=device)
+    got = gelu(z.view(1, -1).to(device), status=status)[0]
+    assert (_units(got, want) <= 0.5 + 256 * (5 * 2 * inner.abs().clamp(max=64) + 8) * 2.0 ** -24).all()
+    far = gelu(torch.tensor([[-11.0, -1e30, -float("inf"), float("inf")]], dtype=torch.bfloat16, device=device),
+                    status=status)[0].cpu()
+    assert far[:2].eq(0).all() and far[2].isnan() and far[3] == float("inf")
