@@ -159,13 +159,14 @@ int64_t mie_decode_scratch_bytes(int32_t batch, int32_t q_heads, int32_t kv_head
  *               1 = length-proportional split-KV chosen on the device from the
  *                   batch's total length (the partials are merged by a second
  *                   kernel; few requests or short tables have a cluster per
- *                   KV head that merges by itself); > 1 = fixed chunk of that
- *                   many tokens (multiple of 16).
+ *                   KV head that merges by itself, without a plan kernel);
+ *                   > 1 = fixed chunk of that many tokens (multiple of 16).
  * scratch: device buffer of at least mie_decode_scratch_bytes(...) bytes,
  * 256-byte aligned; contents need not be initialised.  plan_only / use_plan
  * let a model step build the work plan once (layer 0) and reuse it for the
  * other layers: plan_only=1 builds the plan and returns; use_plan=1 skips the
- * plan kernel and uses slot `plan_slot` (0..63) of the plan's work counters.
+ * plan kernel and uses slot `plan_slot` (0..63) of the plan's work counters
+ * (calls with the same sizes and lengths, any split_policy).
  * out_q8 (optional): additionally writes the output quantised for the o_proj
  * FP8 GEMM, exactly what mie_fp8_quantize would produce from `out` viewed as
  * [batch, q_heads * head_dim]: e4m3 rows of ldq8 bytes and out_scales[head *

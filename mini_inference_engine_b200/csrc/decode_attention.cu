@@ -595,8 +595,7 @@ int launch_merge(const DecodeParams& q, int heads, cudaStream_t stream) {
 }
 
 template <typename T>
-int launch_fast(const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, int policy, cudaStream_t stream) {
-  const int share = policy == 1 ? decode_share(p.batch, p.kv_heads, (long long)p.table_width * p.block_size, 512) : 0;
+int launch_fast(const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, int share, cudaStream_t stream) {
   if (share > 0) return launch_shared<T, 2, 2, false>(p, kmap, vmap, share, stream);
   static bool configured[64] = {false};
   int dev = 0;
@@ -705,8 +704,10 @@ extern "C" int mie_paged_decode_attention(mie_view4_t query, mie_view4_t out, mi
   DecodeParams p{View4(query), View4(out), IndexView(block_tables), IndexView(sequence_lengths),
                  IndexView(query_positions), sc, batch, q_heads, kv_heads, group, block_size, num_blocks,
                  table_width, scale * 1.4426950408889634f, plan_slot, status, reinterpret_cast<uint8_t*>(out_q8), ldq8,
-                 out_scales, out_scale_ld, 0, head_dim, head_dim, kv_heads, 0, nullptr};
-  if (!use_plan) {
+                 out_scales, out_scale_ld, 0, head_dim, head_dim, kv_heads, 0, nullptr, use_plan ? 0 : 1};
+  const int share =
+      split_policy == 1 && !plan_only ? decode_share(batch, kv_heads, (long long)table_width * block_size, 512) : 0;
+  if (!use_plan && share == 0) {
     plan_kernel<<<1, plan_threads(batch), 0, stream>>>(p.lengths, p.positions, batch, (long long)table_width * block_size,
                                                 kv_heads, split_policy, sm_count() * kWarps, 128, 0ll, sc, status);
     MIE_LAUNCH_CHECK("plan_kernel");
@@ -716,8 +717,8 @@ extern "C" int mie_paged_decode_attention(mie_view4_t query, mie_view4_t out, mi
   CUtensorMap kmap, vmap;
   if (int rc = page_tensor_map(key_blocks, num_blocks, kv_heads, block_size, head_dim, dtype, &kmap)) return rc;
   if (int rc = page_tensor_map(value_blocks, num_blocks, kv_heads, block_size, head_dim, dtype, &vmap)) return rc;
-  if (dtype == MIE_DTYPE_BF16) return launch_fast<__nv_bfloat16>(p, kmap, vmap, split_policy, stream);
-  return launch_fast<__half>(p, kmap, vmap, split_policy, stream);
+  if (dtype == MIE_DTYPE_BF16) return launch_fast<__nv_bfloat16>(p, kmap, vmap, share, stream);
+  return launch_fast<__half>(p, kmap, vmap, share, stream);
 }
 
 // ---------------------------------------------------------------------------

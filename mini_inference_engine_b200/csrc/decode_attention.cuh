@@ -278,7 +278,19 @@ struct DecodeParams {
   int dim, vdim, item_heads;
   long long window;
   const float* sinks;
+  int leaves_plan;     // kShare: this call is to leave a work plan behind
 };
+
+// The work plan with one item per request and head; a request of unusable length has one too, of no tokens, whose rows are
+// zero.  By one block.
+__device__ __forceinline__ void plan_whole_requests(const DecodeParams& p) {
+  for (int i = threadIdx.x; i <= p.batch; i += blockDim.x) {
+    p.sc.offsets[i] = i;
+    if (i < p.batch) p.sc.item_seq[i] = i, p.sc.item_chunk[i] = 0;
+  }
+  for (int i = threadIdx.x; i < kCounters; i += blockDim.x) p.sc.header[kCounterBase + i] = 0;
+  if (threadIdx.x == 0) p.sc.header[0] = 0x7fffffff, p.sc.header[1] = p.batch, p.sc.header[2] = p.batch * p.item_heads;
+}
 
 // The end of a (request, KV head) that a cluster shares (kShare): every warp has the part `o`, `m`, `l` of its tokens.  The
 // CTA's parts meet in shared memory, the cluster's in rank 0, which writes the result.
@@ -386,7 +398,9 @@ __device__ __forceinline__ void finish_shared(const DecodeParams& p, const float
 // kExt = false: head_dim 128, GQA group <= 8, scores rounded to the activation dtype as the reference's bf16
 // product is.  kExt = true: other head sizes, any group, fp32 scores, sliding window, sinks, no e4m3 output.
 // kShare = false: persistent warps take (request, chunk, KV head) items of the work plan and leave partials for the merge
-// kernel.  kShare = true, for few requests: a cluster per (request, KV head), whose warps have equal parts of its tokens.
+// kernel.  kShare = true, for few requests: a cluster per (request, KV head), whose warps have equal parts of its tokens.  It
+// needs no plan, but a call with another split policy may reuse the one of this call: one CTA leaves the plan of requests
+// that are not cut.
 template <typename T, int KH, int VH, bool kExt, bool kShare>
 __global__ void __launch_bounds__(DecodeTile<KH, VH>::kWarps * 32, 1)
     decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
@@ -414,6 +428,7 @@ __global__ void __launch_bounds__(DecodeTile<KH, VH>::kWarps * 32, 1)
   const int g = lane >> 2, t = lane & 3;
   const int chunk = kShare ? 0 : p.sc.header[0];
   const int total_items = kShare ? 0 : p.sc.header[2];
+  if (kShare && p.leaves_plan && blockIdx.x == gridDim.x - 1) plan_whole_requests(p);
   const int rank = kShare ? (int)blockIdx.x % split : 0;
   int* counter = p.sc.header + kCounterBase + p.counter_slot;
   const long long capacity_tokens = (long long)p.table_width * p.block_size;
@@ -691,9 +706,9 @@ __global__ void __launch_bounds__(DecodeTile<KH, VH>::kWarps * 32, 1)
 }
 
 // CTAs per (request, KV head) when a cluster shares it, or 0: work plan, queue and merge kernel.  What that path costs before
-// and behind the streaming (plan, queue, item and page look-ups one after the other, a second launch) is 5 us: one request
-// of 611 tokens 11.0 -> 6.3 us, of 3000 14.3 -> 8.7, four of 200 10.9 -> 6.0, four of 3000 18.8 -> 15.8, sixteen of 200
-// 11.8 -> 9.5.  But the shares are fixed before lengths are known, so they have to do for the longest request that the block
+// and behind the streaming (queue, item and page look-ups one after the other, a second launch) is 5 us, and the plan kernel,
+// once a step, 7: one request of 611 tokens without the plan 11.0 -> 6.3 us, a single call 18.2 -> 6.2; of 3000 14.3 -> 8.7
+// and 21.6 -> 8.4, four of 200 10.9 -> 6.0, four of 3000 18.8 -> 15.8, sixteen of 200 11.8 -> 9.5.  But the shares are fixed before lengths are known, so they have to do for the longest request that the block
 // table has room for: any, if it gets 64 CTAs (30000 tokens: 35.0 us against 35.9), else 512 KiB a CTA, 1 MiB in clusters
 // of four (eight of 3000, two CTAs a head: 33.8 us against 25.8; sixteen of 1000, one CTA: 25.0 against 19.7).
 inline int decode_share(int batch, int item_heads, long long capacity_tokens, int token_bytes) {

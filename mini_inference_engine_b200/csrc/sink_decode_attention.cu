@@ -14,13 +14,9 @@ namespace {
 constexpr int kMaxBoxes = 4;  // head sizes up to 256
 
 template <int KH, int VH>
-int launch_sink(const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, int policy, cudaStream_t stream) {
+int launch_sink(const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, int share, cudaStream_t stream) {
   using Tile = DecodeTile<KH, VH>;
   using T = __nv_bfloat16;
-  // A windowed request reads no more than its window and a tile.
-  const long long room = (long long)p.table_width * p.block_size;
-  const long long longest = p.window > 0 && p.window + kTileTokens < room ? p.window + kTileTokens : room;
-  const int share = policy == 1 ? decode_share(p.batch, p.item_heads, longest, (KH + VH) * 128) : 0;
   if (share > 0) return launch_shared<T, KH, VH, true>(p, kmap, vmap, share, stream);
   static bool configured[64] = {false};
   int dev = 0;
@@ -40,13 +36,13 @@ int launch_sink(const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMa
 }
 
 template <int KH>
-int launch_sink_v(int vh, const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, int policy,
+int launch_sink_v(int vh, const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, int share,
                   cudaStream_t stream) {
   switch (vh) {
-    case 1: return launch_sink<KH, 1>(p, kmap, vmap, policy, stream);
-    case 2: return launch_sink<KH, 2>(p, kmap, vmap, policy, stream);
-    case 3: return launch_sink<KH, 3>(p, kmap, vmap, policy, stream);
-    default: return launch_sink<KH, 4>(p, kmap, vmap, policy, stream);
+    case 1: return launch_sink<KH, 1>(p, kmap, vmap, share, stream);
+    case 2: return launch_sink<KH, 2>(p, kmap, vmap, share, stream);
+    case 3: return launch_sink<KH, 3>(p, kmap, vmap, share, stream);
+    default: return launch_sink<KH, 4>(p, kmap, vmap, share, stream);
   }
 }
 
@@ -106,9 +102,13 @@ extern "C" int mie_sink_decode_attention(const void* query, int64_t q_row_stride
   DecodeParams p{View4(q), View4(o), IndexView(block_tables), IndexView(sequence_lengths), IndexView(), sc, batch,
                  q_heads, kv_heads, q_heads / kv_heads, block_size, num_blocks, table_width,
                  scale * 1.4426950408889634f, plan_slot, status, nullptr, 0, nullptr, 0, 0, dim, value_dim, item_heads,
-                 window, sinks};
+                 window, sinks, use_plan ? 0 : 1};
   const int kh = boxes(dim), vh = boxes(value_dim);
-  if (!use_plan) {
+  // A windowed request reads no more than its window and a tile.
+  const long long room = (long long)table_width * block_size;
+  const long long longest = window > 0 && window + kTileTokens < room ? window + kTileTokens : room;
+  const int share = split_policy == 1 ? decode_share(batch, item_heads, longest, (kh + vh) * 128) : 0;
+  if (!use_plan && share == 0) {
     const int warps = kh + vh <= 6 ? 8 : 6;
     plan_kernel<<<1, plan_threads(batch), 0, stream>>>(p.lengths, p.positions, batch,
                                                        (long long)table_width * block_size, item_heads, split_policy,
@@ -119,9 +119,9 @@ extern "C" int mie_sink_decode_attention(const void* query, int64_t q_row_stride
   if (int rc = page_tensor_map(key_blocks, num_blocks, kv_heads, block_size, dim, dtype, &kmap)) return rc;
   if (int rc = page_tensor_map(value_blocks, num_blocks, kv_heads, block_size, value_dim, dtype, &vmap)) return rc;
   switch (kh) {
-    case 1: return launch_sink_v<1>(vh, p, kmap, vmap, split_policy, stream);
-    case 2: return launch_sink_v<2>(vh, p, kmap, vmap, split_policy, stream);
-    case 3: return launch_sink_v<3>(vh, p, kmap, vmap, split_policy, stream);
-    default: return launch_sink_v<4>(vh, p, kmap, vmap, split_policy, stream);
+    case 1: return launch_sink_v<1>(vh, p, kmap, vmap, share, stream);
+    case 2: return launch_sink_v<2>(vh, p, kmap, vmap, share, stream);
+    case 3: return launch_sink_v<3>(vh, p, kmap, vmap, share, stream);
+    default: return launch_sink_v<4>(vh, p, kmap, vmap, share, stream);
   }
 }
