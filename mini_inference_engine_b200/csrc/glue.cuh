@@ -49,6 +49,25 @@ __device__ __forceinline__ void scale8(const float (&v)[8], float f, Bf16x8& out
   for (int i = 0; i < 4; ++i) out.pair[i] = __floats2bfloat162_rn(v[2 * i] * f, v[2 * i + 1] * f);
 }
 
+// Launch shape of a kernel that has `lanes` threads for a row: blocks of a part of a wide row, or of several narrow ones
+// (block y), as many as leave two blocks per SM.  One row a block: 10000 x 256 through gelu 10.8 us, now 2.9; 16384 x 128
+// through SiLU 17.4, now 3.7.
+struct RowBlocks {
+  int per_row, x, y;
+  long long blocks;
+  RowBlocks(int rows, int lanes) {
+    const int most = rows <= sm_count() ? 128 : 512;  // few rows: more, smaller blocks
+    per_row = (lanes + most - 1) / most;
+    x = per_row > 1 ? ((lanes + per_row - 1) / per_row + 31) / 32 * 32 : lanes;
+    const int room = 256 / x, enough = rows / (2 * sm_count());
+    y = room < enough ? room : enough;
+    if (per_row > 1 || y < 1) y = 1;
+    blocks = (long long)((rows + y - 1) / y) * per_row;
+  }
+  dim3 grid() const { return dim3((unsigned)blocks); }
+  dim3 block() const { return dim3((unsigned)x, (unsigned)y); }
+};
+
 // a / b from y, an approximation of 1 / b: quotient, its exact remainder, correction.  Correctly rounded when y is the
 // correctly rounded reciprocal (Markstein's theorem), else but for quotients within 2^-20 units of a tie.  Three
 // instructions where an IEEE division takes about ten.  a, b and y must be finite.

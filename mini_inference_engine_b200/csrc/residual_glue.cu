@@ -148,9 +148,10 @@ template <typename T, int VEC>
 __global__ void gelu_kernel(GeluParams p, int blocks_per_row) {
   chain_release();
   chain_wait();
-  const long long row = blockIdx.x / blocks_per_row;
-  const int c = (int)((blockIdx.x - (unsigned)row * blocks_per_row) * blockDim.x + threadIdx.x) * VEC;
-  if (c >= p.cols) return;
+  const int first = blockIdx.x / blocks_per_row;
+  const long long row = (long long)first * blockDim.y + threadIdx.y;
+  const int c = (int)((blockIdx.x - first * blocks_per_row) * blockDim.x + threadIdx.x) * VEC;
+  if (row >= p.rows || c >= p.cols) return;
   float v[VEC];
   Vec<T, VEC>::load(reinterpret_cast<const T*>(p.in) + row * p.ld_in + c, v);
 #pragma unroll
@@ -368,10 +369,10 @@ extern "C" int mie_gelu(const void* in, int64_t ld_in, mie_index_t ids, const vo
   const GeluParams p{in, ld_in, IndexView(ids), table, ld_table, vocab, out, ldo, rows, cols, status};
   const bool vec = cols % 8 == 0 && ld_in % 8 == 0 && ldo % 8 == 0 && aligned(in, 16) && aligned(out, 16) &&
                    (!table || (ld_table % 8 == 0 && aligned(table, 16)));
-  const int lanes = vec ? cols / 8 : cols, most = rows <= sm_count() ? 128 : 512;  // few rows: more, smaller blocks
-  const int per_row = (lanes + most - 1) / most, threads = ((lanes + per_row - 1) / per_row + 31) / 32 * 32;
-  MIE_CHECK_ARG((long long)rows * per_row <= 0x7fffffff, "too many rows (%d)", rows);
-  const dim3 grid((unsigned)(rows * per_row)), block((unsigned)threads);
+  const RowBlocks shape(rows, vec ? cols / 8 : cols);
+  MIE_CHECK_ARG(shape.blocks <= 0x7fffffff, "too many rows (%d)", rows);
+  const dim3 grid = shape.grid(), block = shape.block();
+  const int per_row = shape.per_row;
   if (dtype == MIE_DTYPE_BF16)
     MIE_CUDA(vec ? launch_chained(gelu_kernel<__nv_bfloat16, 8>, grid, block, 0, (cudaStream_t)stream, p, per_row)
                  : launch_chained(gelu_kernel<__nv_bfloat16, 1>, grid, block, 0, (cudaStream_t)stream, p, per_row));

@@ -207,3 +207,47 @@ def test_gelu_of_any_value(device):
     far = gelu(torch.tensor([[-11.0, -1e30, -float("inf"), float("inf")]], dtype=torch.bfloat16, device=device),
                     status=status)[0].cpu()
     assert far[:2].eq(0).all() and far[2].isnan() and far[3] == float("inf")
+
+
+# Rows a block: one, several, a last block that is not full; parts of a row; groups of eight and of sixteen lanes (the latter
+# up to 3 Mi values); rows of no whole group.
+ROW_SHAPES = [(1, 128), (148, 128), (593, 128), (1000, 384), (4100, 1024), (297, 9728), (700, 9728), (5, 12288), (601, 72),
+              (1200, 8), (300, 4616)]
+
+
+@pytest.mark.parametrize("rows,cols", ROW_SHAPES)
+def test_gated_rows_of_any_width(rows, cols, device):
+    """The division's results (SiLU of every bf16 gate is), and the quantiser's bytes and scales of them."""
+
+    from mini_inference_engine_b200.engine.kernels import fused
+
+    generator = torch.Generator(device=device).manual_seed(rows)
+    both = (torch.randn(rows, 2 * cols, generator=generator, device=device) * 3).to(torch.bfloat16)
+    wide = both[:, :cols].float()
+    want = (wide / (1.0 + torch.exp(-wide))).to(torch.bfloat16) * both[:, cols:]
+    assert torch.equal(fused.silu_mul(both[:, :cols], both[:, cols:]), want)
+    if cols % 128 == 0:
+        q = torch.zeros(rows, cols, dtype=torch.uint8, device=device)
+        scales = torch.zeros(cols // 128, rows + 3, device=device)
+        _lib.check(_lib.load().mie_silu_mul(_lib.ptr(both), _lib.ptr(both[:, cols:]), 2 * cols, None, _lib.ptr(q), cols,
+                                            _lib.ptr(scales), rows + 3, rows, cols, _lib.stream_arg(device)))
+        want_q, want_s = sm89_fp8.quantize_sm89_fp8_activation(want)
+        assert torch.equal(q, want_q.view(torch.uint8)) and torch.equal(scales[:, :rows].t(), want_s)
+
+
+@pytest.mark.parametrize("rows,cols", [*ROW_SHAPES, (2000, 37), (10, 1)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gelu_rows_of_any_width(rows, cols, dtype, device):
+    """Times a table row for each: the result's rounding to 16 bits, or those of a few fp32 operations and of 1 + tanh."""
+
+    from mini_inference_engine_b200.engine.kernels.decoder_glue import gelu
+
+    generator = torch.Generator().manual_seed(cols)
+    x, table = torch.randn(rows, cols, generator=generator).to(dtype), torch.randn(7, cols, generator=generator).to(dtype)
+    ids = torch.arange(rows) % 7
+    status = torch.zeros(1, dtype=torch.int32, device=device)
+    got = gelu(x.to(device), ids=ids.to(device), table=table.to(device), status=status).cpu().double()
+    z = x.double()
+    want = z / (1.0 + torch.exp(-2.0 * 0.7978845608028654 * (z + 0.044715 * z ** 3))) * table.double()[ids]
+    bound = want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -19)
+    assert ((got - want).abs() <= bound + (z * table.double()[ids]).abs() * 2.0 ** -21).all() and int(status.item()) == 0
