@@ -17,7 +17,8 @@ namespace {
 // row to row and requests the next one before it reduces this one; the weight is read once.  Bound by HBM (2 bytes a value
 // and tensor, 1 for e4m3), if the arithmetic is packed: 12032 x 2560 with residual, sum and e4m3
 // 54.3 us with a CTA per row, now 46.5; 560 rows 5.9 and 4.1, one row 2.9 and 2.1.  (Three CTAs of 320 threads per SM; four
-// 50.3, five 55.0; a warp per row 69.)
+// 50.3, five 55.0; a warp per row 69.)  Narrow rows take as many CTAs as the registers of an SM allow: 12032 x 1024 19.8 us
+// with a CTA per row, 25.2 with four per SM, now 17.4.
 // ---------------------------------------------------------------------------
 struct RowNormParams {
   const __nv_bfloat16* x;
@@ -36,7 +37,6 @@ struct RowNormParams {
 
 // kThreads: the most of the instantiation; kCtas: how many of them an SM holds, all of which go from row to row.
 template <int kThreads, int kCtas>
-
 __global__ void __launch_bounds__(kThreads, kCtas) row_norm_kernel(RowNormParams p) {
   __shared__ float red[2][32];
   chain_release();
@@ -328,7 +328,8 @@ extern "C" int mie_rms_norm(const void* x, int64_t ldx, const void* residual, vo
     const int ctas = sm_count() * per_sm;
     return launch_chained(kernel, dim3(rows < ctas ? rows : ctas), dim3(threads), 0, (cudaStream_t)stream, p);
   };
-  MIE_CUDA(threads <= 256   ? launch(row_norm_kernel<256, 4>, 4)
+  // 56 registers a thread, of 64 Ki an SM.
+  MIE_CUDA(threads <= 256   ? launch(row_norm_kernel<256, 4>, 1152 / threads)
            : threads <= 384 ? launch(row_norm_kernel<384, 3>, 3)
            : threads <= 512 ? launch(row_norm_kernel<512, 2>, 2)
                             : launch(row_norm_kernel<1024, 1>, 1));

@@ -251,3 +251,25 @@ def test_gelu_rows_of_any_width(rows, cols, dtype, device):
     want = z / (1.0 + torch.exp(-2.0 * 0.7978845608028654 * (z + 0.044715 * z ** 3))) * table.double()[ids]
     bound = want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -19)
     assert ((got - want).abs() <= bound + (z * table.double()[ids]).abs() * 2.0 ** -21).all() and int(status.item()) == 0
+
+
+@pytest.mark.parametrize("rows,cols", [(1400, 8), (9500, 128), (2700, 1024), (1500, 1792), (700, 2560), (310, 4096), (200, 8192)])
+def test_norm_rows_past_the_resident_blocks(rows, cols, device):
+    """Blocks that go from row to row: residual sum, norm and e4m3.  The sum's order can move a normed value by one bf16 step
+    (2^-7 of it at most); the product with the weight is rounded on both sides, half a step each: 2^-6 in all."""
+
+    generator = torch.Generator().manual_seed(cols)
+    x, residual, weight = (torch.randn(n, cols, generator=generator).to(torch.bfloat16).to(device) for n in (rows, rows, 1))
+    summed, out = torch.empty_like(x), torch.empty_like(x)
+    q, scales = torch.zeros(rows, cols, dtype=torch.uint8, device=device), torch.zeros(max(1, cols // 128), rows, device=device)
+    fits = cols % 128 == 0
+    _lib.check(_lib.load().mie_rms_norm(_lib.ptr(x), cols, _lib.ptr(residual), _lib.ptr(summed), _lib.ptr(weight),
+                                        _lib.ptr(out), _lib.ptr(q) if fits else None, cols, _lib.ptr(scales), rows, rows,
+                                        cols, 1e-6, _lib.stream_arg(device)))
+    assert torch.equal(summed, x + residual)
+    want = hot_path.rms_norm(summed.cpu(), weight[0].cpu(), 1e-6).float()
+    assert ((out.cpu().float() - want).abs() <= 2.0 ** -6 * want.abs()).all()
+    assert (out.cpu().float() != want).float().mean() < 0.02
+    if fits:
+        want_q, want_s = sm89_fp8.quantize_sm89_fp8_activation(out)
+        assert torch.equal(q, want_q.view(torch.uint8)) and torch.equal(scales.t(), want_s)
