@@ -89,12 +89,12 @@ struct ScaleStage {
   static constexpr int kFloats = kChunkKb * BN;  // one a_scale * w_scale product per (K block, token)
 };
 
-// Promotion warps of fp8_gemm_kernel: one per TMEM lane quadrant, from 64 tokens two and for 128 four, which share the
-// columns (96 tokens of 2560 x 9728: 13.9 us with two, 13.1 with four; 6144 x 2560 9.4 and 9.15).
-template <int BN>
-constexpr int kNarrowEpiWarps = BN >= 128 ? 16 : BN >= 64 ? 8 : 4;
-template <int BN>
-constexpr int kNarrowThreads = (kNarrowEpiWarps<BN> + 3) * 32;
+// Promotion warps of fp8_gemm_kernel: one per TMEM lane quadrant, from 33 tokens two and for 128 columns four, which share the
+// columns.  Four cost 0.2 to 0.4 us of start and barriers, which more than four K blocks a CTA pay (us, two and four a
+// quadrant: 96 tokens of 2560 x 9728 13.5 and 12.9, of 6144 x 2560 9.4 and 9.2, of 1536 x 2560, five blocks, 6.8 and 6.8, 65
+// 6.6 and 6.35; of 4096 x 2048, four blocks, 7.0 and 7.4).
+constexpr int narrow_warps(int bn, int blocks) { return bn >= 128 && blocks > 4 ? 16 : bn >= 64 ? 8 : 4; }
+constexpr int narrow_threads(int warps) { return (warps + 3) * 32; }
 
 template <int BN>
 struct GemmSmem {
@@ -139,14 +139,14 @@ __device__ __forceinline__ void store_row4(const GemmParams& p, int tok, int n0,
 
 // The end of the narrow kernel.  Every CTA of the cluster has parked its fp32 sums as [token][128 weight rows]; CTA
 // `rank` finishes its share of the live tokens.  A warp takes a token, a lane four weight rows (16-byte
-// distributed-shared-memory loads, the rows of several tokens from all CTAs in flight together) and adds the kSplit
+// distributed-shared-memory loads, the rows of several tokens from all CTAs in flight together; none for tokens past the
+// share: 33 tokens of 4096 x 2048 5.8 -> 5.4 us) and adds the kSplit
 // parts of K in part order, so that results do not depend on timing.
-template <int BN, Finish kFinish, int kSplit>
+template <int kWarps, int BN, Finish kFinish, int kSplit>
 __device__ __forceinline__ void finish_rows(const GemmParams& p, const QkvParams& qkv, const longlong2* place,
                                             uint32_t park, int rank, int tile, int tok0, int warp, int lane) {
   constexpr int kPeers = kFinish == Finish::kSilu ? 2 * kSplit : kSplit;  // gate parts have even ranks, up parts odd ones
   constexpr int kBatch = kPeers >= 8 ? 1 : kPeers >= 4 ? 2 : 4;
-  constexpr int kWarps = kNarrowEpiWarps<BN>;
   const int live = p.m - tok0 < BN ? p.m - tok0 : BN;
   const int slice = (live + kPeers - 1) / kPeers;
   const int lo = rank * slice, hi = lo + slice < live ? lo + slice : live;
@@ -155,7 +155,8 @@ __device__ __forceinline__ void finish_rows(const GemmParams& p, const QkvParams
     float4 part[kBatch][kPeers];
 #pragma unroll
     for (int u = 0; u < kBatch; ++u) {
-      const int j = j0 + u * kWarps < hi ? j0 + u * kWarps : j0;
+      const int j = j0 + u * kWarps;
+      if (j >= hi) break;
 #pragma unroll
       for (int peer = 0; peer < kPeers; ++peer)
         part[u][peer] = ld_cluster_f4(park + (uint32_t)((j * kTileR + lane * 4) * 4), (uint32_t)peer);
@@ -213,13 +214,13 @@ __device__ __forceinline__ void finish_rows(const GemmParams& p, const QkvParams
 // both frees its stage and hands its accumulator to the promotion.
 // grid = (tiles, split), cluster = (1, split, 1): CTA `rank` of a cluster takes the rank-th part of K.  Finish::kSilu: a
 // cluster has a CTA for the gate rows and one for the up rows of every part of K (ranks 2 part and 2 part + 1).
-template <int BN, Finish kFinish>
-__global__ void __launch_bounds__(kNarrowThreads<BN>, GemmSmem<BN>::kCtasPerSm)
+template <int BN, Finish kFinish, int E>
+__global__ void __launch_bounds__(narrow_threads(E), GemmSmem<BN>::kCtasPerSm)
     fp8_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                     const __grid_constant__ GemmParams p, const __grid_constant__ QkvParams qkv) {
   using S = GemmSmem<BN>;
   using SS = ScaleStage<BN>;
-  constexpr int E = kNarrowEpiWarps<BN>, kCols = BN * 4 / E;  // columns of a promotion warp
+  constexpr int kCols = BN * 4 / E;  // columns of a promotion warp
   constexpr int kStages = S::kStages;
   constexpr int kAcc = S::kAcc;
   constexpr uint32_t kTmemCols = kAcc * BN < 32 ? 32 : kAcc * BN;
@@ -418,13 +419,13 @@ __global__ void __launch_bounds__(kNarrowThreads<BN>, GemmSmem<BN>::kCtasPerSm)
   cluster_sync_all();
   if (warp < E) {
     if (split == 1)
-      finish_rows<BN, kFinish, 1>(p, qkv, place, park, rank, tn, tt * BN, warp, lane);
+      finish_rows<E, BN, kFinish, 1>(p, qkv, place, park, rank, tn, tt * BN, warp, lane);
     else if (split == 2)
-      finish_rows<BN, kFinish, 2>(p, qkv, place, park, rank, tn, tt * BN, warp, lane);
+      finish_rows<E, BN, kFinish, 2>(p, qkv, place, park, rank, tn, tt * BN, warp, lane);
     else if (split == 4)
-      finish_rows<BN, kFinish, 4>(p, qkv, place, park, rank, tn, tt * BN, warp, lane);
+      finish_rows<E, BN, kFinish, 4>(p, qkv, place, park, rank, tn, tt * BN, warp, lane);
     else if constexpr (!kPairs)
-      finish_rows<BN, kFinish, 8>(p, qkv, place, park, rank, tn, tt * BN, warp, lane);
+      finish_rows<E, BN, kFinish, 8>(p, qkv, place, park, rank, tn, tt * BN, warp, lane);
   }
   __syncwarp();
   if (gridDim.y > 1) cluster_sync_all();  // no CTA leaves while a peer may still read its rows
@@ -1060,26 +1061,22 @@ int choose_split(long long tiles, int kb_total, int bn, int ctas_per_sm, int max
   return best;
 }
 
-template <int BN, Finish kFinish>
+template <int BN, Finish kFinish, int E>
 int launch_narrow_tiles(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p, const QkvParams& qkv,
-                        int max_split, cudaStream_t stream) {
+                        int tiles, int split, cudaStream_t stream) {
   using S = GemmSmem<BN>;
   static bool configured[64] = {false};
   int dev = 0;
   MIE_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    MIE_CUDA(cudaFuncSetAttribute(fp8_gemm_kernel<BN, kFinish>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    MIE_CUDA(cudaFuncSetAttribute(fp8_gemm_kernel<BN, kFinish, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   S::kTotal));
     configured[dev] = true;
   }
   constexpr int kPair = kFinish == Finish::kSilu ? 2 : 1;
-  const long long tiles = (long long)((p.n + kTileR - 1) / kTileR) * ((p.m + BN - 1) / BN);
-  MIE_CHECK_ARG(tiles <= 0x7fffffff, "too many output tiles (%lld)", tiles);
-  const int kb = (p.k + kBlockK - 1) / kBlockK;
-  const int split = choose_split(tiles, kb, BN, S::kCtasPerSm, max_split, (S::kCtasPerSm == 2 ? 8 : 4) / kPair);
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3((unsigned)(tiles / kPair), (unsigned)(split * kPair), 1);
-  config.blockDim = dim3(kNarrowThreads<BN>, 1, 1);
+  config.blockDim = dim3(narrow_threads(E), 1, 1);
   config.dynamicSmemBytes = S::kTotal;
   config.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -1091,9 +1088,23 @@ int launch_narrow_tiles(const CUtensorMap& mw, const CUtensorMap& mx, const Gemm
   attr[0].val.clusterDim.z = 1;
   config.attrs = attr;
   config.numAttrs = chained_launch_enabled() ? 2 : 1;
-  MIE_CUDA(cudaLaunchKernelEx(&config, fp8_gemm_kernel<BN, kFinish>, mw, mx, p, qkv));
+  MIE_CUDA(cudaLaunchKernelEx(&config, fp8_gemm_kernel<BN, kFinish, E>, mw, mx, p, qkv));
   MIE_LAUNCH_CHECK("fp8_gemm_kernel");
   return MIE_OK;
+}
+
+template <int BN, Finish kFinish>
+int launch_narrow_columns(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p, const QkvParams& qkv,
+                          int max_split, cudaStream_t stream) {
+  constexpr int kPerSm = GemmSmem<BN>::kCtasPerSm, kPair = kFinish == Finish::kSilu ? 2 : 1;
+  const long long tiles = (long long)((p.n + kTileR - 1) / kTileR) * ((p.m + BN - 1) / BN);
+  MIE_CHECK_ARG(tiles <= 0x7fffffff, "too many output tiles (%lld)", tiles);
+  const int kb = (p.k + kBlockK - 1) / kBlockK;
+  const int split = choose_split(tiles, kb, BN, kPerSm, max_split, (kPerSm == 2 ? 8 : 4) / kPair);
+  constexpr int kFew = narrow_warps(BN, 1), kMany = narrow_warps(BN, 1 << 20);
+  if (narrow_warps(BN, (kb + split - 1) / split) == kFew)
+    return launch_narrow_tiles<BN, kFinish, kFew>(mw, mx, p, qkv, (int)tiles, split, stream);
+  return launch_narrow_tiles<BN, kFinish, kMany>(mw, mx, p, qkv, (int)tiles, split, stream);
 }
 
 // Column-tile width for the swapped orientation: smallest of 16/32/64/128 covering m.
@@ -1107,10 +1118,10 @@ int launch_narrow(const void* x8, long long ldx, const void* w8, long long ldw, 
   if (int rc = operand_map(w8, p.n, p.k, ldw, kTileR, &mw)) return rc;
   if (int rc = operand_map(x8, p.m, p.k, ldx, bn, &mx)) return rc;
   switch (bn) {
-    case 16: return launch_narrow_tiles<16, kFinish>(mw, mx, p, qkv, max_split, stream);
-    case 32: return launch_narrow_tiles<32, kFinish>(mw, mx, p, qkv, max_split, stream);
-    case 64: return launch_narrow_tiles<64, kFinish>(mw, mx, p, qkv, max_split, stream);
-    default: return launch_narrow_tiles<128, kFinish>(mw, mx, p, qkv, max_split, stream);
+    case 16: return launch_narrow_columns<16, kFinish>(mw, mx, p, qkv, max_split, stream);
+    case 32: return launch_narrow_columns<32, kFinish>(mw, mx, p, qkv, max_split, stream);
+    case 64: return launch_narrow_columns<64, kFinish>(mw, mx, p, qkv, max_split, stream);
+    default: return launch_narrow_columns<128, kFinish>(mw, mx, p, qkv, max_split, stream);
   }
 }
 

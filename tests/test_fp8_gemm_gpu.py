@@ -87,6 +87,22 @@ def test_tail_shapes_and_row_counts(m, n, k, device, status_clean):
         assert not out[1].any()  # an all-zero row stays exactly zero
 
 
+@pytest.mark.parametrize("m", [65, 81, 128])
+@pytest.mark.parametrize("k", [2048, 2064, 2560])
+def test_both_numbers_of_promotion_warps(m, k, device, status_clean):
+    """Four K blocks a CTA, and five: eight and sixteen warps; token shares of a CTA that the warps do not divide.  Bound: the
+    output's rounding to bf16, and fp32 sums of 20 blocks of 128 products."""
+
+    generator = torch.Generator().manual_seed(m + k)
+    w8 = (torch.randn(4096, k, generator=generator) * 32).clamp(-448, 448).to(torch.float8_e4m3fn)
+    w_scale = torch.rand(32, (k + 127) // 128, generator=generator) * 0.09 + 0.001
+    x = torch.randn(m, k, generator=generator).to(torch.bfloat16)
+    out = sm89_fp8.sm89_fp8_linear(x.to(device), w8.to(device), w_scale.to(device), block_size=[128, 128])
+    exact = _dequantised_product(*hot_path.quantize_activation(x), w8, w_scale)
+    error = (out.cpu().double() - exact).abs()
+    assert (error <= 2.0 ** -8 * exact.abs() + 2.0 ** -14 * exact.abs().amax()).all()
+
+
 def test_rows_are_independent_and_bias_dtype(device, status_clean):
     """A row's result does not depend on its neighbours (tests/test_sm89_fp8_exact.py:15-53)."""
 
