@@ -628,6 +628,9 @@ int mie_paged_attention_rows(const void* query, int64_t q_token_stride, int64_t 
  *
  * mie_sink_prefill_attention: packed chunks, query row i of request r at
  * position kv_lens[r] - q_len + i, as in mie_flash_prefill_attention.
+ * mie_sink_prefill_packed: the same with the number of packed tokens (0: not
+ * known), by which ragged chunks are spread over the GPU as they are and not
+ * as requests * max_query_len tokens.
  */
 int mie_sink_decode_supported(int32_t dim, int32_t value_dim, int32_t block_size, int32_t dtype);
 int mie_sink_decode_attention(const void* query, int64_t q_row_stride, int64_t q_head_stride, void* out,
@@ -640,6 +643,13 @@ int mie_sink_decode_attention(const void* query, int64_t q_row_stride, int64_t q
                               void* stream);
 int mie_sink_prefill_supported(int32_t q_heads, int32_t kv_heads, int32_t dim, int32_t value_dim,
                                int32_t block_size, int32_t dtype, float scale);
+int mie_sink_prefill_packed(const void* query, int64_t q_token_stride, int64_t q_head_stride, void* out,
+                            int64_t o_token_stride, int64_t o_head_stride, mie_view4_t key_blocks,
+                            mie_view4_t value_blocks, mie_index_t block_tables, mie_index_t cu_seqlens,
+                            mie_index_t kv_lens, int64_t total_tokens, int32_t requests, int32_t max_query_len,
+                            int32_t q_heads, int32_t kv_heads, int32_t dim, int32_t value_dim, int32_t block_size,
+                            int32_t num_blocks, int32_t table_width, int32_t dtype, float scale, int64_t window,
+                            const float* sinks, int32_t* status, void* stream);
 int mie_sink_prefill_attention(const void* query, int64_t q_token_stride, int64_t q_head_stride, void* out,
                                int64_t o_token_stride, int64_t o_head_stride, mie_view4_t key_blocks,
                                mie_view4_t value_blocks, mie_index_t block_tables, mie_index_t cu_seqlens,

@@ -171,6 +171,10 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
                                                   View4T, IndexT, IndexT, IndexT, c_int32, c_int32, c_int32, c_int32,
                                                   c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_float,
                                                   c_int64, c_void_p, c_void_p, c_void_p]),
+    "mie_sink_prefill_packed": (ctypes.c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, View4T, View4T,
+                                               IndexT, IndexT, IndexT, c_int64, c_int32, c_int32, c_int32, c_int32,
+                                               c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_float, c_int64,
+                                               c_void_p, c_void_p, c_void_p]),
     "mie_residual_norm": (ctypes.c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_float, c_void_p, c_void_p,
                                          c_int64, c_int32, c_int32, c_int32, c_float, c_void_p]),
     "mie_gelu": (ctypes.c_int, [c_void_p, c_int64, IndexT, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int32,

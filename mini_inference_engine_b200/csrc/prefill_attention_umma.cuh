@@ -30,6 +30,7 @@
 // the TMEM allocation.  Every wait is bounded and reports MIE_STATUS_WAIT_TIMEOUT.
 #pragma once
 
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
@@ -689,52 +690,67 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-// CTAs that share the K/V tiles of a pair of query tiles: as many as there are SMs for, when the pairs alone leave half of
-// them idle.  16 tokens over 3000: 38 us unsplit, 14 with six CTAs; 386 and 126 tokens over 1024: 31 us and 24; what it
-// costs is 3 to 5 us (the ranks' O through remote shared memory), which eight tiles in two halves pay.
-inline int prefill_split(long long pairs) {
-  int split = 1;
-  while (split < kMaxSplit && pairs * split * 2 <= sm_count()) split *= 2;
-  return split;
-}
-
+// CTAs that share the K/V tiles of a pair of query tiles: as many as leave all clusters on the GPU at once (of 148 SMs 74
+// clusters of two, 33 of four, 15 of eight; the 16 heads of a short prompt as clusters of eight take a second round: 64 tokens
+// with 192-dim keys 10.4 us, as clusters of four 9.5; one token over 4100 31.6 and 20.7).  16 tokens over 3000: 38 us unsplit,
+// 14 with six CTAs; 386 and 126 tokens over 1024: 31 us and 24; what it costs is 3 to 5 us (the ranks' O through remote shared
+// memory), which eight tiles in two halves pay.  75 to 148 pairs are not split, so that a pair of the longest rows takes
+// longer than two CTAs with a query tile each did (3000 tokens of 8 heads on one 39.7 -> 44.6 us); clusters of two of which
+// only the heaviest pairs use both are no way out: the SM that an idle rank leaves is not given to another cluster (20 ->
+// 40 us).
 template <typename T, int KH, int VH, bool kExt>
 int launch_prefill(const CUtensorMap& kmap, const CUtensorMap& vmap, const UmmaPrefillParams& p, long long tokens,
                    int max_query_len, cudaStream_t stream) {
   constexpr int kSmem = PrefillTile<KH, VH>::kSmemBytes;
-  static bool configured[64] = {false};
-  int dev = 0;
-  MIE_CUDA(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < 64 && !configured[dev]) {
-    MIE_CUDA(cudaFuncSetAttribute(prefill_umma_kernel<T, KH, VH, kExt>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    configured[dev] = true;
-  }
-  const int pair_tokens = kTiles * (kRows / p.group);
-  const int q_tiles = (max_query_len + pair_tokens - 1) / pair_tokens;
-  const int columns = p.kv_heads * (kExt ? p.v_passes : 1);
-  // Pairs with live rows (`tokens` of ragged requests): the last pair of a request is half empty on average, and each
-  // request has one.
-  const long long most = (long long)q_tiles * p.requests, mean = tokens / pair_tokens + (p.requests + 1) / 2;
-  const long long likely = mean < p.requests ? p.requests : mean < most ? mean : most;
-  const int split = prefill_split(likely * columns);
+  const auto kernel = prefill_umma_kernel<T, KH, VH, kExt>;
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3((unsigned)(q_tiles * split), (unsigned)p.requests, (unsigned)columns);
   config.blockDim = dim3(kThreads);
   config.dynamicSmemBytes = kSmem;
   config.stream = stream;
   cudaLaunchAttribute attr[2];
+  const auto in_clusters = [&](int size) {
+    cudaLaunchAttribute a;
+    a.id = cudaLaunchAttributeClusterDimension;
+    a.val.clusterDim.x = (unsigned)size;
+    a.val.clusterDim.y = a.val.clusterDim.z = 1;
+    return a;
+  };
+  static std::atomic<bool> configured[64];
+  static int fitting[64][4];  // clusters of 2, 4 and 8 that the device holds
+  int dev = 0;
+  MIE_CUDA(cudaGetDevice(&dev));
+  MIE_CHECK_ARG(dev >= 0 && dev < 64, "device %d", dev);
+  if (!configured[dev].load(std::memory_order_acquire)) {
+    MIE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    config.attrs = attr;
+    config.numAttrs = 1;
+    for (int i = 1; i < 4; ++i) {
+      attr[0] = in_clusters(1 << i);
+      config.gridDim = dim3(1u << i);
+      MIE_CUDA(cudaOccupancyMaxActiveClusters(&fitting[dev][i], kernel, &config));
+    }
+    configured[dev].store(true, std::memory_order_release);
+  }
+  const int pair_tokens = kTiles * (kRows / p.group);
+  const int q_tiles = (max_query_len + pair_tokens - 1) / pair_tokens;
+  const int columns = p.kv_heads * (kExt ? p.v_passes : 1);
+  // Pairs with live rows, as far as the host knows: as many as there can be when the requests are about equally long.  Of
+  // ragged ones the last pair is half empty on average, and each has one; that counts short requests for less than a pair,
+  // but theirs are over soon.
+  const long long most = (long long)q_tiles * p.requests, mean = tokens / pair_tokens + (p.requests + 1) / 2;
+  const bool equal = tokens * 16 >= (long long)max_query_len * p.requests * 15;
+  const long long likely = (equal || mean > most ? most : mean < p.requests ? p.requests : mean) * columns;
+  int split = 1;
+  for (int i = 1; i < 4 && likely <= fitting[dev][i]; ++i) split = 1 << i;
+  config.gridDim = dim3((unsigned)(q_tiles * split), (unsigned)p.requests, (unsigned)columns);
+  config.attrs = attr;
+  config.numAttrs = 0;
   if (chained_launch_enabled()) {
     attr[config.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[config.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
   }
-  if (split > 1) {
-    attr[config.numAttrs].id = cudaLaunchAttributeClusterDimension;
-    attr[config.numAttrs].val.clusterDim.x = (unsigned)split;
-    attr[config.numAttrs].val.clusterDim.y = attr[config.numAttrs].val.clusterDim.z = 1;
-    ++config.numAttrs;
-  }
-  config.attrs = attr;
-  MIE_CUDA(cudaLaunchKernelEx(&config, prefill_umma_kernel<T, KH, VH, kExt>, kmap, vmap, p, q_tiles, split));
+  if (split > 1) attr[config.numAttrs++] = in_clusters(split);
+  MIE_CUDA(cudaLaunchKernelEx(&config, kernel, kmap, vmap, p, q_tiles, split));
   MIE_LAUNCH_CHECK("prefill_umma_kernel");
   return MIE_OK;
 }

@@ -40,14 +40,14 @@ extern "C" int mie_sink_prefill_supported(int32_t q_heads, int32_t kv_heads, int
          block_size % kSub == 0 && scale > 0.f;
 }
 
-extern "C" int mie_sink_prefill_attention(const void* query, int64_t q_token_stride, int64_t q_head_stride, void* out,
-                                          int64_t o_token_stride, int64_t o_head_stride, mie_view4_t key_blocks,
-                                          mie_view4_t value_blocks, mie_index_t block_tables, mie_index_t cu_seqlens,
-                                          mie_index_t kv_lens, int32_t requests, int32_t max_query_len,
-                                          int32_t q_heads, int32_t kv_heads, int32_t dim, int32_t value_dim,
-                                          int32_t block_size, int32_t num_blocks, int32_t table_width, int32_t dtype,
-                                          float scale, int64_t window, const float* sinks, int32_t* status,
-                                          void* stream_) {
+extern "C" int mie_sink_prefill_packed(const void* query, int64_t q_token_stride, int64_t q_head_stride, void* out,
+                                       int64_t o_token_stride, int64_t o_head_stride, mie_view4_t key_blocks,
+                                       mie_view4_t value_blocks, mie_index_t block_tables, mie_index_t cu_seqlens,
+                                       mie_index_t kv_lens, int64_t total_tokens, int32_t requests,
+                                       int32_t max_query_len, int32_t q_heads, int32_t kv_heads, int32_t dim,
+                                       int32_t value_dim, int32_t block_size, int32_t num_blocks,
+                                       int32_t table_width, int32_t dtype, float scale, int64_t window,
+                                       const float* sinks, int32_t* status, void* stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
   MIE_CHECK_ARG(mie_sink_prefill_supported(q_heads, kv_heads, dim, value_dim, block_size, dtype, scale),
                 "sink prefill attention takes bf16, key sizes that are multiples of 8 up to 256, value sizes that are "
@@ -75,11 +75,25 @@ extern "C" int mie_sink_prefill_attention(const void* query, int64_t q_token_str
                       IndexView(block_tables), IndexView(cu_seqlens), IndexView(kv_lens), requests, q_heads, kv_heads,
                       group, block_size, num_blocks, table_width, scale * 1.4426950408889634f, status, dim, value_dim,
                       (value_dim + vh * 64 - 1) / (vh * 64), k_slab ? 1 : 0, v_slab ? 1 : 0, window, sinks};
-  const long long tokens = (long long)requests * max_query_len;  // at most
+  const long long tokens = total_tokens > 0 ? total_tokens : (long long)requests * max_query_len;  // at most
   switch (kh) {
     case 1: return launch_sink_prefill_v<1>(vh, kmap, vmap, p, tokens, max_query_len, stream);
     case 2: return launch_sink_prefill_v<2>(vh, kmap, vmap, p, tokens, max_query_len, stream);
     case 3: return launch_sink_prefill_v<3>(vh, kmap, vmap, p, tokens, max_query_len, stream);
     default: return launch_sink_prefill_v<4>(vh, kmap, vmap, p, tokens, max_query_len, stream);
   }
+}
+
+extern "C" int mie_sink_prefill_attention(const void* query, int64_t q_token_stride, int64_t q_head_stride, void* out,
+                                          int64_t o_token_stride, int64_t o_head_stride, mie_view4_t key_blocks,
+                                          mie_view4_t value_blocks, mie_index_t block_tables, mie_index_t cu_seqlens,
+                                          mie_index_t kv_lens, int32_t requests, int32_t max_query_len,
+                                          int32_t q_heads, int32_t kv_heads, int32_t dim, int32_t value_dim,
+                                          int32_t block_size, int32_t num_blocks, int32_t table_width, int32_t dtype,
+                                          float scale, int64_t window, const float* sinks, int32_t* status,
+                                          void* stream) {
+  return mie_sink_prefill_packed(query, q_token_stride, q_head_stride, out, o_token_stride, o_head_stride, key_blocks,
+                                 value_blocks, block_tables, cu_seqlens, kv_lens, 0, requests, max_query_len, q_heads,
+                                 kv_heads, dim, value_dim, block_size, num_blocks, table_width, dtype, scale, window,
+                                 sinks, status, stream);
 }

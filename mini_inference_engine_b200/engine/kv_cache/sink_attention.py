@@ -68,10 +68,10 @@ def sink_prefill_attention(query, out, key_blocks, value_blocks, block_tables, c
     requests = int(cu_seqlens.shape[0]) - 1
     if tokens == 0 or requests <= 0:
         return
-    _lib.check(_lib.load().mie_sink_prefill_attention(
+    _lib.check(_lib.load().mie_sink_prefill_packed(
         _lib.ptr(query), query.stride(0), query.stride(1), _lib.ptr(out), out.stride(0), out.stride(1),
         _lib.view4_arg(key_blocks), _lib.view4_arg(value_blocks), _lib.index_arg(block_tables),
-        _lib.index_arg(cu_seqlens), _lib.index_arg(kv_lens), requests, int(max_query_len), heads,
+        _lib.index_arg(cu_seqlens), _lib.index_arg(kv_lens), tokens, requests, int(max_query_len), heads,
         int(key_blocks.shape[1]), dim, int(value_blocks.shape[3]), int(key_blocks.shape[2]),
         int(key_blocks.shape[0]), int(block_tables.shape[1]), _lib.DTYPE_CODES[query.dtype], float(scale),
         int(window or 0), _lib.ptr(sinks), _lib.ptr(status), _lib.stream_arg(query.device)))

@@ -5,7 +5,7 @@ from __future__ import annotations
 import pytest
 import torch
 
-from mini_inference_engine_b200 import workloads
+from mini_inference_engine_b200 import _lib, workloads
 from test_prefill_attention_gpu import ATOL, _oracle, _run
 from test_sink_attention_gpu import Case
 
@@ -65,3 +65,21 @@ def test_what_is_no_number_reaches_the_result(sizes, device):
     want[5] = True
     want[..., 10] = True
     assert torch.equal(bad, want) and bool(case.out[5].isnan().all())
+
+
+@pytest.mark.parametrize("total", [None, 0, 530])
+def test_ragged_chunks_with_and_without_their_number_of_tokens(total, device):
+    """One long chunk among short ones: by the older entry point, and by the packed one that may know the tokens."""
+
+    case = Case([2500, 40, 700], [500, 20, 10], 8, 4, 128, 128, None, 16, torch.bfloat16, seed=14)
+    keys, values, tables = case.on(device)
+    cu = torch.tensor([0, 500, 520, 530], dtype=torch.int32, device=device)
+    lens = torch.tensor(case.lengths, dtype=torch.int32, device=device)
+    lib, name = _lib.load(), "mie_sink_prefill_attention" if total is None else "mie_sink_prefill_packed"
+    _lib.check(getattr(lib, name)(
+        _lib.ptr(case.q), case.q.stride(0), case.q.stride(1), _lib.ptr(case.out), case.out.stride(0), case.out.stride(1),
+        _lib.view4_arg(keys), _lib.view4_arg(values), _lib.index_arg(tables), _lib.index_arg(cu), _lib.index_arg(lens),
+        *(() if total is None else (total,)), 3, 500, 8, 4, 128, 128, 16, case.pages, int(tables.shape[1]),
+        _lib.DTYPE_CODES[torch.bfloat16], case.scale, 0, _lib.ptr(case.common["sinks"]), _lib.ptr(case.status),
+        _lib.stream_arg(device)))
+    case.check()
