@@ -1338,17 +1338,19 @@ extern "C" int mie_fp8_gemm_finish_pays(int32_t m, int32_t n, int32_t k, int32_t
 
 // Whether the wide kernel should finish the gated rows itself.  It saves a launch and the rows' way through memory, but the
 // tensor core has two K blocks to go on with while a tile is finished (about 3 us), and a tail of tiles is not cut.  Measured
-// (us, separate / finished), weights [gate | up] of 9728 columns each, K 2560: 96 tokens 17.4 / 16.1, 560 44.8 / 43.4, 1024
-// (cut tail) 71.7 / 69.0, 4096 252.8 / 241.1, but 8192 512 / 536 and 12032 733 / 766: over 24 rounds only with a long K
-// (12288, K 4096, 12032 tokens 1486 / 1421).  A cut tail matters in the first rounds (9728, 200 tokens 28.5 / 29.3) and with a
-// long K (12288, K 4096, 1024 tokens 120 / 126).
+// (us, separate / finished), weights [gate | up] of 9728 columns each, K 2560: 300 tokens 32.8 / 32.3, 1024 71.7 / 70.4, 4096
+// 257.5 / 242.2, 12032 829 / 812; of 12288, K 4096, 768 tokens 88.8 / 85.8, 12032 1545 / 1527.  What a cut tail is worth grows
+// with K and is set against the rounds' gain, about a fifth of a K block each: with K 2560 one round before it is too few (200
+// tokens 30.5 / 31.3) and two are enough (400 44.9 / 43.7), with K 3072 three are not (768 63.3 / 63.9) and six are (1536
+// 114.2 / 111.4), with K 4096 four are not (1024 95.7 / 96.7) and eight are (2048 180.4 / 174.2).
 static bool wide_silu_pays(int m, int cols, int k, int max_split) {
   const long long tiles = (long long)((m + kTileR - 1) / kTileR) * (cols / 128);
   const int kb = (k + kBlockK - 1) / kBlockK;
   if (cols % 128 != 0 || narrow_fits(m, 2 * cols) || tiles > 0x7fffffff) return false;
   const WidePlan plan = plan_wide(tiles, kb, max_split);
-  if (plan.main_split > 1 || (tiles > 24ll * sm_count() && kb < 32)) return false;
-  return plan.tail_split == 0 || (plan.main_tiles >= 2 * sm_count() && kb <= 24);
+  if (plan.main_split > 1) return false;
+  const int rounds = plan.main_tiles / sm_count();
+  return plan.tail_split == 0 || (kb <= 20 ? rounds >= 2 : 5 * rounds >= kb);
 }
 
 extern "C" int mie_fp8_gemm_silu_wide_pays(int32_t m, int32_t cols, int32_t k, int32_t max_split) {

@@ -183,3 +183,17 @@ def test_gated_rows_of_long_steps(m, cols, k, device, status_clean):
     _lib.check(lib.mie_silu_mul(_lib.ptr(both), _lib.ptr(both[:, cols:]), 2 * cols, None, _lib.ptr(want), cols,
                                 _lib.ptr(want_s), m + 2, m, cols, stream))
     assert torch.equal(got, want) and torch.equal(got_s, want_s)
+
+
+# Tokens, columns, K; whether the wide kernel finishes them, on a GPU of 148 SMs: no cut tail, many rounds; one round, two,
+# and three or more of longer sums in front of a cut tail; narrow steps; columns of no whole group.
+WIDE_RULE = [(300, 9728, 2560, 1), (12032, 9728, 2560, 1), (200, 9728, 2560, 0), (400, 9728, 2560, 1), (768, 9728, 3072, 0),
+             (1536, 9728, 3072, 1), (1024, 9728, 4096, 0), (2048, 9728, 4096, 1), (64, 9216, 2560, 0), (300, 9729, 2560, 0)]
+
+
+@pytest.mark.parametrize("m,cols,k,pays", WIDE_RULE)
+def test_rule_for_gated_rows_of_long_steps(m, cols, k, pays, device):
+    lib = _lib.load()
+    if int(lib.mie_sm_count()) != 148:
+        pytest.skip("measured on 148 SMs")
+    assert int(lib.mie_fp8_gemm_silu_wide_pays(m, cols, k, 0)) == pays
