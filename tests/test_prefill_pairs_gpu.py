@@ -5,6 +5,9 @@ from __future__ import annotations
 import pytest
 import torch
 
+from mini_inference_engine_b200 import workloads
+from oracle import hot_path
+from test_prefill_attention_gpu import ATOL, _run
 from test_sink_attention_gpu import Case
 
 pytestmark = pytest.mark.gpu
@@ -39,3 +42,23 @@ def test_wide_keys(sizes, window, device):
     for _ in range(3):
         case.prefill(device)
         case.check()
+
+
+# One query tile, shared by eight ranks; 79 pairs, not shared.
+@pytest.mark.parametrize("chunk,heads,kv_heads", [(20, 8, 2), (2500, 8, 1)])
+def test_more_than_64k_cached_tokens(chunk, heads, kv_heads, device, status_clean):
+    """The first and the last rows of the chunk; queries of three units, so that a few keys have most of the weight."""
+
+    case = workloads.prefill_case(seed=33, prefix_lengths=(66_000,), chunk_lengths=(chunk,), q_heads=heads,
+                                  kv_heads=kv_heads)
+    case.query.mul_(3.0)
+    _, out = _run(case, device)
+    keys, values = case.key_blocks.clone(), case.value_blocks.clone()
+    hot_path.write_packed_kv(case.new_keys, case.new_values, case.token_to_sequence, case.token_positions,
+                             case.block_tables, keys, values)
+    keys, values = (t[case.block_tables[0].long()].transpose(0, 1).flatten(1, 2).float() for t in (keys, values))
+    for row in {*range(10), *range(chunk - 10, chunk)}:
+        seen = 66_000 + row + 1
+        scores = case.query[row].float().view(kv_heads, -1, 128) @ keys[:, :seen].transpose(1, 2) * case.scale
+        want = (scores.softmax(-1) @ values[:, :seen]).reshape(heads, 128)
+        assert (out[row].float() - want).abs().max().item() <= ATOL

@@ -184,7 +184,7 @@ def test_pages_of_several_tiles(device):
 
 
 def test_long_context_past_the_shared_page_ids(device):
-    """A chunk at the end of 66k tokens: more pages than the prefill kernel keeps in shared memory, and a split
+    """A chunk at the end of 66k tokens, whose K/V tiles a cluster shares and looks up 32 boxes at a time, and a split
     decode of the same context."""
 
     length = 66_000
