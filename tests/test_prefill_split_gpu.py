@@ -83,3 +83,20 @@ def test_ragged_chunks_with_and_without_their_number_of_tokens(total, device):
         _lib.DTYPE_CODES[torch.bfloat16], case.scale, 0, _lib.ptr(case.common["sinks"]), _lib.ptr(case.status),
         _lib.stream_arg(device)))
     case.check()
+
+
+@pytest.mark.parametrize("heads,kv_heads,others", [(32, 8, 11), (8, 8, 11)])
+def test_alone_and_among_many(heads, kv_heads, others, device, status_clean):
+    """Alone a chunk is shared by six ranks, among eleven like it (96 pairs) by none: both within the bound, and their sums
+    in another order, which some of their bits show."""
+
+    sizes = dict(q_heads=heads, kv_heads=kv_heads)
+    alone = workloads.prefill_case(seed=15, prefix_lengths=(3000,), chunk_lengths=(16,), **sizes)
+    many = workloads.prefill_case(seed=15, prefix_lengths=(3000,) * (others + 1), chunk_lengths=(16,) * (others + 1), **sizes)
+    many.query[:16] = alone.query
+    many.new_keys[:, :, :16], many.new_values[:, :, :16] = alone.new_keys, alone.new_values
+    _, _, expected = _oracle(alone)
+    results = [_run(case, device)[1][:16].float() for case in (alone, many)]
+    for out in results:
+        assert (out - expected.float()).abs().max().item() <= ATOL
+    assert not torch.equal(*results)
