@@ -694,10 +694,9 @@ __global__ void __launch_bounds__(kThreads, 1)
 // clusters of two, 33 of four, 15 of eight; the 16 heads of a short prompt as clusters of eight take a second round: 64 tokens
 // with 192-dim keys 10.4 us, as clusters of four 9.5; one token over 4100 31.6 and 20.7).  16 tokens over 3000: 38 us unsplit,
 // 14 with six CTAs; 386 and 126 tokens over 1024: 31 us and 24; what it costs is 3 to 5 us (the ranks' O through remote shared
-// memory), which eight tiles in two halves pay.  75 to 148 pairs are not split, so that a pair of the longest rows takes
-// longer than two CTAs with a query tile each did (3000 tokens of 8 heads on one 39.7 -> 44.6 us); clusters of two of which
-// only the heaviest pairs use both are no way out: the SM that an idle rank leaves is not given to another cluster (20 ->
-// 40 us).
+// memory), which eight tiles in two halves pay.  75 to 148 pairs are only split where the wait of the last is no loss (below);
+// else a pair of the longest rows takes longer than two CTAs with a query tile each did.  Clusters of two of which only the
+// heaviest pairs use both are no way out: the SM that an idle rank leaves is not given to another cluster (20 -> 40 us).
 template <typename T, int KH, int VH, bool kExt>
 int launch_prefill(const CUtensorMap& kmap, const CUtensorMap& vmap, const UmmaPrefillParams& p, long long tokens,
                    int max_query_len, cudaStream_t stream) {
@@ -742,6 +741,16 @@ int launch_prefill(const CUtensorMap& kmap, const CUtensorMap& vmap, const UmmaP
   const long long likely = (equal || mean > most ? most : mean < p.requests ? p.requests : mean) * columns;
   int split = 1;
   for (int i = 1; i < 4 && likely <= fitting[dev][i]; ++i) split = 1 << i;
+  // Prompts with little room for a prefix: a pair has half of the last one's K/V tiles on average, and clusters of two that
+  // have to wait are over before the longest if they are the lighter pairs of the last (request, head), which come last, or of
+  // the last two of eight and more for a whole prompt of many tiles.  3000 tokens of 8 heads on one (94 pairs) 45.1 -> 32.0 us, of 8 heads on 8
+  // (96) 44.8 -> 41.5; left alone: two of 1500 on 8 (96) 27.2 -> 32.5, three of 3000 of 4 on one (141) 45.7 -> 51.2.
+  const long long room = (long long)p.table_width * p.block_size, waiting = likely - fitting[dev][1];
+  const int tiles = max_query_len / kKv;
+  const bool two = 8 * room <= 9ll * max_query_len && tiles >= 16 && 4 * q_tiles <= fitting[dev][1];
+  if (split == 1 && likely <= sm_count() && equal && tiles >= 12 && waiting <= (two ? 2 : 1) * q_tiles &&
+      2 * room <= 3ll * max_query_len && (p.window == 0 || p.window >= max_query_len))
+    split = 2;
   config.gridDim = dim3((unsigned)(q_tiles * split), (unsigned)p.requests, (unsigned)columns);
   config.attrs = attr;
   config.numAttrs = 0;

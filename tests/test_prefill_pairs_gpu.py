@@ -62,3 +62,15 @@ def test_more_than_64k_cached_tokens(chunk, heads, kv_heads, device, status_clea
         scores = case.query[row].float().view(kv_heads, -1, 128) @ keys[:, :seen].transpose(1, 2) * case.scale
         want = (scores.softmax(-1) @ values[:, :seen]).reshape(heads, 128)
         assert (out[row].float() - want).abs().max().item() <= ATOL
+
+
+# 76 to 97 pairs of whole prompts, more than there are clusters of two at once: shared with 19 K/V tiles, and with 12 of each of
+# two requests; not with 4 tiles, a table with room for a prefix or a window that ends in the prompt.
+@pytest.mark.parametrize("lengths,heads,kv_heads,window,spare", [
+    ((2500,), 8, 1, None, 0), ((1540, 1530), 8, 1, None, 0), ((600,) * 4, 8, 1, None, 0), ((2500,), 8, 1, None, 200),
+    ((2500,), 8, 1, 700, 0), ((2500,), 8, 1, 2600, 0)], ids=str)
+def test_whole_prompts_in_clusters_that_wait(lengths, heads, kv_heads, window, spare, device):
+    case = Case(lengths, lengths, heads, kv_heads, 64, 64, window, 16, torch.bfloat16, seed=34)
+    case.tables = torch.nn.functional.pad(case.tables, (0, spare), value=-1)
+    case.prefill(device)
+    case.check()
